@@ -74,23 +74,6 @@ __device__ __forceinline__ void pair_put(float4 *c, int v, int vn, float h, floa
 // ---------------------------------------------------------------------------
 // the reference Maxwellian of a solve (ugks_fused_block.ref, UGKS_REF_*)
 // ---------------------------------------------------------------------------
-enum { RM00, RM10, RM01, RM20, RM11, RM02, RM30, RM21, RM12, RM03, RB00, RB10, RB01, RNMOM };
-
-// Heat flux (calcQ, clKernel.c:480-543) relative to velocity U of a
-// distribution given by its raw moments M (the RM* / RB* sums over v of h u^a
-// v^b and of b u^a v^b), in the frame of the moments:
-//   q = 1/2 sum (c |c|^2 h + c b / K),  c = (u, v) - U.
-__device__ __forceinline__ V2 heat_flux_from_moments(const double *M, double K, V2 U) {
-  const double Ux = U.x, Uy = U.y;
-  const double cx3 = M[RM30] - 3.0 * Ux * M[RM20] + 3.0 * Ux * Ux * M[RM10] - Ux * Ux * Ux * M[RM00] + M[RM12] -
-                     2.0 * Uy * M[RM11] + Uy * Uy * M[RM10] - Ux * M[RM02] + 2.0 * Ux * Uy * M[RM01] -
-                     Ux * Uy * Uy * M[RM00];
-  const double cy3 = M[RM03] - 3.0 * Uy * M[RM02] + 3.0 * Uy * Uy * M[RM01] - Uy * Uy * Uy * M[RM00] + M[RM21] -
-                     2.0 * Ux * M[RM11] + Ux * Ux * M[RM01] - Uy * M[RM20] + 2.0 * Ux * Uy * M[RM10] -
-                     Uy * Ux * Ux * M[RM00];
-  return v2(0.5 * (cx3 + (M[RB10] - Ux * M[RB00]) / K), 0.5 * (cy3 + (M[RB01] - Uy * M[RB00]) / K));
-}
-
 struct RefMaxwellian {
   double lam0, P0, kb0;
   const double *mom;  // RNMOM raw moments, global frame
@@ -279,18 +262,7 @@ __global__ void __launch_bounds__(NT) wall_pass_delta(const ugks_fused_block *__
   const ugks_fused_block &blk = B[find_block<3>(B, nb, w)];
   const ugks_block_desc &d = blk.d;
   UGKS_CHECK_ITEM(3, blk, w, solves);
-  int lw = w - blk.wall_begin, mi, mj, dir;
-  if (lw < 2 * d.ni) {
-    dir = SOUTH;
-    mi = lw % d.ni;
-    mj = lw < d.ni ? 0 : d.nj;
-  } else {
-    lw -= 2 * d.ni;
-    dir = WEST;
-    mj = lw % d.nj;
-    mi = lw < d.nj ? 0 : d.ni;
-  }
-  const int fw = blk.face_begin + ((mi * (d.nj + 1) + mj) << 1) + dir;
+  const int fw = wall_to_face(blk, w);
   switch (d.flux_method) {
     case 0: face_item_delta<0, NT, true>(B, nb, solves, fw, 0); break;
     case 1: face_item_delta<1, NT, true>(B, nb, solves, fw, 0); break;

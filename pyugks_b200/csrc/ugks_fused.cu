@@ -41,59 +41,19 @@ constexpr int FT = 128;  // threads per face / cell / ghost CTA
 // the ghost copies, issued before the first store (a store may alias a later
 // load, so the compiler keeps them in program order)
 constexpr int GHOST_U = 4;
-// face kernels come in two shapes: narrow, FT threads per face at
-// FACE_MIN_BLOCKS CTAs per SM (fits while the per-face shared memory allows
-// that many), and wide, for larger velocity grids, where shared memory allows
-// only 2-3 faces per SM: 384 (FP64) or 256 (FP32) threads per face keep the
-// warps per SM up (config-3 batch: face pass 29.6 -> 23.7 ms FP64, 20.1 ->
-// 18.1 ms FP32, against 128 threads)
-#ifndef FACE_MIN_BLOCKS
-#define FACE_MIN_BLOCKS 6
-#endif
-#ifndef FACE_MIN_BLOCKS_F32
-#define FACE_MIN_BLOCKS_F32 5
-#endif
-#ifndef FACE_MIN_BLOCKS_WIDE
-#define FACE_MIN_BLOCKS_WIDE 2
-#endif
-#ifndef FACE_MIN_BLOCKS_WIDE_F32
-#define FACE_MIN_BLOCKS_WIDE_F32 2
-#endif
-#ifndef FACE_WIDE_THREADS
-#define FACE_WIDE_THREADS 384
-#endif
-#ifndef FACE_WIDE_THREADS_F32
-#define FACE_WIDE_THREADS_F32 256
-#endif
-// per storage type: the narrow and wide register budgets and the largest
-// velocity grid of the narrow one (that many face CTAs fit in shared memory:
-// FP64 6 x (32 B x 1100 + 3 KB), mixed 5 x (24 B x 1800 + 3 KB) <= 228 KB;
-// the mixed kernels' packed-pair arithmetic needs 96 registers to run
-// without spilling in its velocity loops)
-template <typename T> struct FaceBudget;
-template <> struct FaceBudget<double> {
-  static constexpr int narrow = FACE_MIN_BLOCKS, wide = FACE_MIN_BLOCKS_WIDE, narrow_max_nv = 1100,
-                       wide_threads = FACE_WIDE_THREADS;
-};
-template <> struct FaceBudget<float> {
-  static constexpr int narrow = FACE_MIN_BLOCKS_F32, wide = FACE_MIN_BLOCKS_WIDE_F32, narrow_max_nv = 1800,
-                       wide_threads = FACE_WIDE_THREADS_F32;
-};
+// mixed retry pass (wall faces, a CTA per face): narrow, FT threads per face,
+// or wide for velocity grids above RETRY_NARROW_NV nodes, whose shared memory
+// lets only two or three faces on an SM
+constexpr int RETRY_NARROW_MINB = 5, RETRY_NARROW_NV = 1800, RETRY_WIDE_NT = 256, RETRY_WIDE_MINB = 2;
 // Launch shapes a face-pass segment can run with (ugks_fused_sizes.seg_variant;
-// the tuner in pyugks_b200/tuner.py picks them by timing): variant 0 chooses
-// by velocity count (narrow up to FaceBudget::narrow_max_nv, wide above),
-// 1..4 force (threads per face CTA, CTAs per SM of the register budget):
-//   FP64  1 = 128 x 6 (narrow), 2 = 128 x 5, 3 = 256 x 3, 4 = 384 x 2 (wide)
-//   mixed 1 = 128 x 5 (narrow), 2 = 128 x 4, 3 = 256 x 3, 4 = 256 x 2 (wide)
-template <typename T, int V> struct FaceShape;
-template <> struct FaceShape<double, 1> { static constexpr int nt = 128, minb = 6; };
-template <> struct FaceShape<double, 2> { static constexpr int nt = 128, minb = 5; };
-template <> struct FaceShape<double, 3> { static constexpr int nt = 256, minb = 3; };
-template <> struct FaceShape<double, 4> { static constexpr int nt = 384, minb = 2; };
-template <> struct FaceShape<float, 1> { static constexpr int nt = 128, minb = 5; };
-template <> struct FaceShape<float, 2> { static constexpr int nt = 128, minb = 4; };
-template <> struct FaceShape<float, 3> { static constexpr int nt = 256, minb = 3; };
-template <> struct FaceShape<float, 4> { static constexpr int nt = 256, minb = 2; };
+// the tuner in pyugks_b200/tuner.py picks them by timing): variant 0 is the
+// default 1, 1..4 are (warps per CTA, CTAs per SM of the register budget).
+// FP64 face pass (a face per warp; measured at face_item_fp64):
+template <int V> struct FaceShape;
+template <> struct FaceShape<1> { static constexpr int wpc = 4, minb = 4; };
+template <> struct FaceShape<2> { static constexpr int wpc = 4, minb = 5; };
+template <> struct FaceShape<3> { static constexpr int wpc = 8, minb = 2; };
+template <> struct FaceShape<4> { static constexpr int wpc = 4, minb = 3; };
 // launch shapes of the mixed moments sweep (a face per warp): warps per CTA x
 // CTAs per SM
 template <int V> struct MomentsShape;
@@ -118,10 +78,6 @@ constexpr int FLUX_WPC = 4, FLUX_MINB = UGKS_FLUX_MINB;
 #define UGKS_FLUX_TMA_MINB 5
 #endif
 constexpr int FLUX_TMA_MINB = UGKS_FLUX_TMA_MINB;
-static_assert(FaceShape<double, 1>::minb == FACE_MIN_BLOCKS && FaceShape<double, 4>::nt == FACE_WIDE_THREADS &&
-                  FaceShape<float, 1>::minb == FACE_MIN_BLOCKS_F32 && FaceShape<float, 4>::minb == FACE_MIN_BLOCKS_WIDE_F32,
-              "variants 1 and 4 are the narrow and wide default shapes");
-
 // CTAs of 8 cell warps per SM: FP64 at 128 registers (at 80 the update loop
 // spills and the pass is 12% slower), mixed at 80 (3 CTAs: 0.215 against
 // 0.222 ms at 120 registers on the 2x2-block cavity)
@@ -148,10 +104,10 @@ constexpr size_t cell_ring_bytes() {
 
 // cp.async (sm_80+ asynchronous global -> shared copy of 8 or 16 bytes per
 // thread; a thread waits only for its own groups)
-template <int BYTES>
+template <int BYTES, bool CA = false>
 __device__ __forceinline__ void cp_async(void *dst, const void *src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (BYTES == 16)
+  if constexpr (BYTES == 16 && !CA)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
@@ -279,14 +235,23 @@ __device__ __forceinline__ void half_moments_rcp(double PI, double K, P4 prim, R
   Mxi[2] = (K * K + 2.0 * K) * (hl * hl);
 }
 
-// named barrier 1 between warp 0 (waits) and warp 1 (arrives): whole warps
-__device__ __forceinline__ void pair_wait() {
-  __syncwarp();
-  asm volatile("bar.sync 1, 64;" ::: "memory");
-}
-__device__ __forceinline__ void pair_arrive() {
-  __syncwarp();
-  asm volatile("bar.arrive 1, 64;" ::: "memory");
+// raw moments of a distribution up to third order: sums over the velocities
+// of h u^a v^b (RMab) and of b u^a v^b (RBab)
+enum { RM00, RM10, RM01, RM20, RM11, RM02, RM30, RM21, RM12, RM03, RB00, RB10, RB01, RNMOM };
+
+// Heat flux (calcQ, clKernel.c:480-543) relative to velocity U of a
+// distribution given by its raw moments M (the RM* / RB* sums over v of h u^a
+// v^b and of b u^a v^b), in the frame of the moments:
+//   q = 1/2 sum (c |c|^2 h + c b / K),  c = (u, v) - U.
+__device__ __forceinline__ V2 heat_flux_from_moments(const double *M, double K, V2 U) {
+  const double Ux = U.x, Uy = U.y;
+  const double cx3 = M[RM30] - 3.0 * Ux * M[RM20] + 3.0 * Ux * Ux * M[RM10] - Ux * Ux * Ux * M[RM00] + M[RM12] -
+                     2.0 * Uy * M[RM11] + Uy * Uy * M[RM10] - Ux * M[RM02] + 2.0 * Ux * Uy * M[RM01] -
+                     Ux * Uy * Uy * M[RM00];
+  const double cy3 = M[RM03] - 3.0 * Uy * M[RM02] + 3.0 * Uy * Uy * M[RM01] - Uy * Uy * Uy * M[RM00] + M[RM21] -
+                     2.0 * Ux * M[RM11] + Ux * Ux * M[RM01] - Uy * M[RM20] + 2.0 * Ux * Uy * M[RM10] -
+                     Uy * Ux * Ux * M[RM00];
+  return v2(0.5 * (cx3 + (M[RB10] - Ux * M[RB00]) / K), 0.5 * (cy3 + (M[RB01] - Uy * M[RB00]) / K));
 }
 
 // 1 / relaxTime
@@ -312,36 +277,41 @@ __device__ __forceinline__ void time_weights_rcp(double inv_tau, double dt, doub
   Mt[2] = 0.5 * (dt * dt) - tau * Mt[0];
 }
 
+// shared memory of a wall CTA: block-sum scratch, a broadcast
 template <int NT>
 struct FaceShared {
   double scratch[16 * (NT / 32)];
-  double bcast[48];
-  double nbr[2][5];  // left / right cell: rho, u, v (face frame), lambda, 1/|mid - centre|
-  double lr[2][19];  // per side: half-range Mu [7], slope a [4], <a u psi> [4], <a u^2 psi> [4]
-  double mt[5];      // time weights
+  double bcast[2];
 };
 
 // WENO5 (clFunctions.c:266-313) of one component, up to the final division:
-// slope * dx = num / den.  Written in the first differences D_k = S_{k+1} - S_k:
-//   12 beta_k = 13 (D_{k+1} - D_k)^2 + 3 r_k^2,  r = (3 D1 - D0, D1 + D2, D3 - 3 D2)
-//   f_k - S2  = (-D0/3 + 5 D1/6, D1/6 + D2/3, 2 D2/3 - D3/6)
+// slope * dx = num / den.  Written in the first and second differences
+// D_k = S_{k+1} - S_k, p_k = D_{k+1} - D_k:
+//   4 beta_k = 13/3 p_k^2 + r_k^2,  r = (2 D1 + p0, D1 + D2, p2 - 2 D2)
+//   6 (f_k - S2) = (2 r0 - D1, r1 + D2, D2 - r2)  (f_k: the candidates)
 // and the weights c_k / (eps + beta_k)^2 multiplied through by
-// prod_j (eps + beta_j)^2 / 0.1 (a common factor of num and den; eps scales
-// with beta).
-__device__ __forceinline__ void weno5_part(const double (&S)[5], double &num, double &den) {
+// prod_j (eps + beta_j)^2 (a common factor of num and den; eps scales with
+// beta); the 1/6 is left to the caller.  35 FP64 operations per component
+// against 44 with the candidates and smoothness terms spelled out.
+__device__ __forceinline__ void weno5_part(const double (&S)[5], double &num6, double &den) {
   const double D0 = S[1] - S[0], D1 = S[2] - S[1], D2 = S[3] - S[2], D3 = S[4] - S[3];
   const double p0 = D1 - D0, p1 = D2 - D1, p2 = D3 - D2;
-  const double r0 = fma(3.0, D1, -D0), r1 = D1 + D2, r2 = fma(-3.0, D2, D3);
-  const double e0 = 12e-16 + fma(13.0 * p0, p0, (3.0 * r0) * r0);
-  const double e1 = 12e-16 + fma(13.0 * p1, p1, (3.0 * r1) * r1);
-  const double e2 = 12e-16 + fma(13.0 * p2, p2, (3.0 * r2) * r2);
+  const double r0 = fma(2.0, D1, p0), r1 = D1 + D2, r2 = fma(-2.0, D2, p2);
+  constexpr double c = 13.0 / 3.0, eps = 4e-16;
+  const double e0 = fma(c * p0, p0, fma(r0, r0, eps));
+  const double e1 = fma(c * p1, p1, fma(r1, r1, eps));
+  const double e2 = fma(c * p2, p2, fma(r2, r2, eps));
   const double q0 = e0 * e0, q1 = e1 * e1, q2 = e2 * e2;
-  const double a0 = q1 * q2, a1 = 6.0 * (q0 * q2), a2 = 3.0 * (q0 * q1);
-  const double f0 = fma(-1.0 / 3.0, D0, (5.0 / 6.0) * D1);
-  const double f1 = fma(1.0 / 6.0, D1, (1.0 / 3.0) * D2);
-  const double f2 = fma(2.0 / 3.0, D2, (-1.0 / 6.0) * D3);
-  num = fma(a0, f0, fma(a1, f1, a2 * f2));
+  const double t0 = 3.0 * q0;
+  const double a0 = q1 * q2, a1 = (t0 + t0) * q2, a2 = t0 * q1;  // 1 : 6 : 3
+  num6 = fma(a0, fma(2.0, r0, -D1), fma(a1, r1 + D2, a2 * (D2 - r2)));
   den = (a0 + a1) + a2;
+}
+
+template <int L, typename VEC>
+__device__ __forceinline__ void load_stencil(const VEC *p, int st, VEC (&x)[L]) {
+#pragma unroll
+  for (int s = 0; s < L; ++s) x[s] = p[s * st];
 }
 
 // iFace (clUGKS.c:148-194) for one velocity: face value and slope of (h, b).
@@ -349,17 +319,15 @@ __device__ __forceinline__ void weno5_part(const double (&S)[5], double &num, do
 // The stencil runs upwind to downwind: cells MID+1 .. 1 before the face and
 // 0 .. L-MID-2 after it for u > 0, mirrored for u <= 0; `p` points at stencil
 // cell 0 and `st` is the signed cell stride in (h, b) pairs.
-template <typename T, int FM>
-__device__ __forceinline__ void reconstruct(const typename Store<T>::vec *p, int st, double inv_l,
-                                            double ds, double inv_ds, double &fh, double &fb,
-                                            double &sh, double &sb) {
+template <int FM>
+__device__ __forceinline__ void reconstruct(const double2 (&x)[FM == 1 ? 5 : 3], double inv_l, double ds,
+                                            double inv_ds, double &fh, double &fb, double &sh, double &sb) {
   constexpr int L = FM == 1 ? 5 : 3, MID = FM == 1 ? 2 : 1;
   double Sh[L], Sb[L];
 #pragma unroll
   for (int s = 0; s < L; ++s) {
-    const auto x = p[s * st];
-    Sh[s] = (double)x.x;
-    Sb[s] = (double)x.y;
+    Sh[s] = x[s].x;
+    Sb[s] = x[s].y;
   }
   if constexpr (FM == 0) {
     // vanLeer (clFunctions.c:255-261)
@@ -373,7 +341,7 @@ __device__ __forceinline__ void reconstruct(const typename Store<T>::vec *p, int
     double nh, dh, nb, db;
     weno5_part(Sh, nh, dh);
     weno5_part(Sb, nb, db);
-    const double r = nr_rcp(dh * db) * inv_ds;
+    const double r = nr_rcp(dh * db) * ((1.0 / 6.0) * inv_ds);
     sh = nh * (db * r);
     sb = nb * (dh * r);
   } else {
@@ -433,11 +401,6 @@ __device__ __forceinline__ void weno5_part_f(const float (&S)[5], float &num, fl
   const float f2 = fmaf(2.0f / 3.0f, D2, (-1.0f / 6.0f) * D3);
   num = fmaf(a0, f0, fmaf(a1, f1, a2 * f2));
   den = (a0 + a1) + a2;
-}
-template <int L, typename VEC>
-__device__ __forceinline__ void load_stencil(const VEC *p, int st, VEC (&x)[L]) {
-#pragma unroll
-  for (int s = 0; s < L; ++s) x[s] = p[s * st];
 }
 template <int FM>
 __device__ __forceinline__ void reconstruct_f(const float2 (&xs)[FM == 1 ? 5 : 3], float inv_l, float ds, float inv_ds,
@@ -681,10 +644,10 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
     const int kind = d.reflect[wall];
     double ratio = 1.0;
     if (refl > 0.0) {
-      // the reflected incoming distribution (wall_dist) of every velocity,
-      // staged in the slope buffer, which wall faces do not use
+      // the reflected incoming distribution (wall_dist) of every velocity
+      // (FP64: read in place, mixed: staged in shared memory)
       __syncthreads();
-      if (kind != UGKS_REFLECT_DIFFUSE)
+      if (!std::is_same<RIN, double2>::value && kind != UGKS_REFLECT_DIFFUSE)
         for (int v = threadIdx.x; v < Nv; v += NT) {
           const V2 x = ld2(blk.wall_dist, (size_t)ci * Nv + v);
           rin[v].x = x.x;
@@ -771,128 +734,21 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
   }
 }
 
-// Per-face coefficient block of an interior face, called by every thread of
-// the face CTA once W, prim and the neighbour cells (sh.nbr) are in place:
-// getPLR slopes (clUGKS.c:424-436) and initMacroFlux (446-518) split over
-// lanes 0 / 1 of warp 0 (one per side, the same instructions with one sign
-// flipped) while lane 0 of warp 1 computes the time weights and hands them
-// over through named barrier 1; the threads from warp 1 on run
-// meanwhile(t, nt) (item t of nt) in the meantime.  Leaves in sh.bcast:
-//   [0..4] / [5..9] distFlux coefficients of the upwind slope aL / aR,
-//   [10..14] those of the time slope aT ([10] includes Mt0),
-//   [15] Mt0, [16] Mt3 len, [17] Mt4 len,
-//   [18..21] len * g0, the analytic equilibrium part of the macro flux.
-template <int NT, typename Meanwhile>
-__device__ __forceinline__ void face_coefficients(const ugks_block_desc &d, FaceShared<NT> &sh, const P4 W,
-                                                  const P4 prim, const Rcp rc, const double len, const double dt,
-                                                  Meanwhile meanwhile) {
-  if (threadIdx.x < 32) {
-    const double kb = (0.5 * d.K) * rc.lam;
-    double Mv[MTUM], Mxi[3];
-    P4 a;
-    if (threadIdx.x < 2) {
-      const int side = threadIdx.x;
-      const double sg = side == 0 ? 1.0 : -1.0;
-      double Mh[MNUM];
-      half_moments_rcp(d.PI, d.K, prim, rc, sg, Mh, Mv, Mxi);
-      const double *o = sh.nbr[side];
-      // left: (W - W_L) / |mid - c_L|; right: (W_R - W) / |mid - c_R|
-      const double id = sg * o[4];
-      a = micro_slope_rcp(d.K, prim, rc,
-                          p4((W.s0 - o[0]) * id, (W.s1 - o[1]) * id, (W.s2 - o[2]) * id, (W.s3 - o[3]) * id));
-      const P4 t1 = moment_au(a, Mh, Mv, Mxi, 1, 0), t2 = moment_au(a, Mh, Mv, Mxi, 2, 0);
-      double *x = sh.lr[side];
-#pragma unroll
-      for (int k = 0; k < MNUM; ++k) x[k] = Mh[k];
-      x[7] = a.s0; x[8] = a.s1; x[9] = a.s2; x[10] = a.s3;
-      x[11] = t1.s0; x[12] = t1.s1; x[13] = t1.s2; x[14] = t1.s3;
-      x[15] = t2.s0; x[16] = t2.s1; x[17] = t2.s2; x[18] = t2.s3;
-    }
-    pair_wait();
-    double Mt[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) Mt[k] = sh.mt[k];
-    double *c = sh.bcast;
-    if (threadIdx.x < 2) {
-      // distFlux coefficients of the upwind slope (derivation at sweep 3)
-      const double xk = Mxi[2] - kb * kb;
-      double *ck = c + 5 * threadIdx.x;
-      ck[0] = Mt[1] * fma(0.5 * a.s3, kb, a.s0);
-      ck[1] = Mt[1] * a.s1;
-      ck[2] = Mt[1] * a.s2;
-      ck[3] = Mt[1] * (0.5 * a.s3);
-      ck[4] = Mt[1] * (0.5 * a.s3 * xk);
-    }
-    if (threadIdx.x == 0) {
-      const double *xl = sh.lr[0], *xr = sh.lr[1];
-      double Mu[MNUM];
-#pragma unroll
-      for (int k = 0; k < MNUM; ++k) Mu[k] = xl[k] + xr[k];
-      const P4 aT = micro_slope_rcp(d.K, prim, rc,
-                                    scale(-prim.s0, add(p4(xl[11], xl[12], xl[13], xl[14]),
-                                                        p4(xr[11], xr[12], xr[13], xr[14]))));
-      const P4 g0 = scale(prim.s0,
-                          add(add(scale(Mt[0], moment_uv(Mu, Mv, Mxi, 1, 0, 0)),
-                                  scale(Mt[1], add(p4(xl[15], xl[16], xl[17], xl[18]),
-                                                   p4(xr[15], xr[16], xr[17], xr[18])))),
-                              scale(Mt[2], moment_au(aT, Mu, Mv, Mxi, 1, 0))));
-      const double xk = Mxi[2] - kb * kb;
-      c[10] = Mt[2] * fma(0.5 * aT.s3, kb, aT.s0) + Mt[0];
-      c[11] = Mt[2] * aT.s1;
-      c[12] = Mt[2] * aT.s2;
-      c[13] = Mt[2] * (0.5 * aT.s3);
-      c[14] = Mt[2] * (0.5 * aT.s3 * xk);
-      c[15] = Mt[0];
-      c[16] = Mt[3] * len;
-      c[17] = Mt[4] * len;
-      c[18] = len * g0.s0; c[19] = len * g0.s1; c[20] = len * g0.s2; c[21] = len * g0.s3;
-    }
-  } else {
-    if (threadIdx.x < 64) {
-      if (threadIdx.x == 32) {
-        double Mt[5];
-        time_weights_rcp(inv_relax_time_rcp(d, prim, rc), dt, Mt);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) sh.mt[k] = Mt[k];
-      }
-      pair_arrive();
-    }
-    // warp 1, which computed the time weights, takes the last items
-    meanwhile((threadIdx.x + NT - 96) % (NT - 32), NT - 32);
-  }
-}
-
-// the two cells beside an interior face (the inputs of getAL / getAR and the
-// getPLR slopes, clUGKS.c:424-436) into sh.nbr, by two lanes of the last warp
-template <int NT>
-__device__ __forceinline__ void face_neighbours(const ugks_fused_block &blk, FaceShared<NT> &sh, const long gi,
-                                                const long gj, const int dir, const V2 n, const V2 mid) {
-  if (threadIdx.x >= NT - 32 && threadIdx.x < NT - 30) {
-    const ugks_block_desc &d = blk.d;
-    const int side = threadIdx.x - (NT - 32);  // 0: left (u > 0 upwind), 1: right
-    const size_t k = side == 0 ? gidx(d, gi - dir, gj - (1 - dir)) : gidx(d, gi, gj);
-    const P4 mc = ld4(blk.cell_mom, k);
-    const V2 uc = to_local(v2(mc.s1, mc.s2), n);
-    const V2 cc = ld2(blk.centre, k);
-    double *o = sh.nbr[side];
-    o[0] = mc.s0;
-    o[1] = uc.x;
-    o[2] = uc.y;
-    o[3] = mc.s3;
-    o[4] = nr_rcp(sqrt((mid.x - cc.x) * (mid.x - cc.x) + (mid.y - cc.y) * (mid.y - cc.y)));
-  }
-}
-
 // face work item -> (block, i, j, direction, wall face); false when the item
 // is skipped (inactive solve, retry pass of a solve without retry, another flux
-// method than FM >= 0, or the unused S face of the last column / W face of the last row).
-// S and W faces of one corner (i, j) are adjacent work items so that both
-// directions read f while it is in L2.
+// method than FM >= 0, or the unused S face of the last column / W face of the
+// last row).  S and W faces of one corner (i, j) are adjacent work items so that
+// both directions read f while it is in L2; with STRIPS a block's items are
+// ordered in strips of FACE_STRIP columns i, in each first the S faces with j
+// running fastest, then the W faces with i running fastest: consecutive items
+// (the warps of a CTA) are neighbours along their normal and share most of
+// their stencil rows in L1.
 struct FaceWork {
   int bi, dir, mi, mj, wall;
   long gi, gj;
 };
-template <int FM>
+constexpr int FACE_STRIP = 4;
+template <int FM, bool STRIPS = false>
 __device__ __forceinline__ bool face_work(const ugks_fused_block *__restrict__ B, int nb,
                                           const ugks_solve_state *__restrict__ solves, const int w, int retry_pass,
                                           FaceWork &fw) {
@@ -905,10 +761,20 @@ __device__ __forceinline__ bool face_work(const ugks_fused_block *__restrict__ B
   if (retry_pass && !sol.retry) return false;
   if (FM >= 0 && d.flux_method != FM) return false;  // FM < 0: any flux method
   int lf = w - blk.face_begin;
-  fw.dir = lf & 1;
-  lf >>= 1;
-  fw.mi = lf / (d.nj + 1);
-  fw.mj = lf % (d.nj + 1);
+  if (STRIPS) {
+    const int c = d.nj + 1, strip = 2 * FACE_STRIP * c, s = lf / strip;
+    const int wd = min(FACE_STRIP, d.ni + 1 - s * FACE_STRIP);
+    lf -= s * strip;
+    fw.dir = lf >= wd * c ? WEST : SOUTH;
+    if (fw.dir == WEST) lf -= wd * c;
+    fw.mi = s * FACE_STRIP + (fw.dir == SOUTH ? lf / c : lf % wd);
+    fw.mj = fw.dir == SOUTH ? lf % c : lf / wd;
+  } else {
+    fw.dir = lf & 1;
+    lf >>= 1;
+    fw.mi = lf / (d.nj + 1);
+    fw.mj = lf % (d.nj + 1);
+  }
   if (fw.dir == SOUTH ? (fw.mi >= d.ni) : (fw.mj >= d.nj)) return false;
   fw.gi = fw.mi + d.ghost;
   fw.gj = fw.mj + d.ghost;
@@ -923,136 +789,280 @@ __device__ __forceinline__ bool face_work(const ugks_fused_block *__restrict__ B
   return true;
 }
 
-// one FP64 face work item (all threads of the CTA take part)
-template <int FM, int NT>
-__device__ __forceinline__ void face_item_fp64(const ugks_fused_block *__restrict__ B, int nb,
-                                               ugks_solve_state *__restrict__ solves, const int w, int retry_pass) {
-  extern __shared__ double dyn[];
-  __shared__ FaceShared<NT> sh;
-  using St = Store<double>;
-  FaceWork fwk;
-  if (!face_work<FM>(B, nb, solves, w, retry_pass, fwk)) return;
-  const ugks_fused_block &blk = B[fwk.bi];
+// ---------------------------------------------------------------------------
+// FP64 interior faces: a face per warp, its lanes over the velocities
+// ---------------------------------------------------------------------------
+// Any velocity grid and any face normal; no barrier, no shared memory per
+// velocity: 16 faces are in flight on an SM whatever the velocity grid, each at
+// its own phase, and the serial middle part of one hides behind the sweeps of
+// the others.  On the 2x2-block cavity (Nv 1089, WENO5) 0.976 -> 0.730 ms, on a
+// 96x96 cavity with Nv 2401 (vanLeer) 1.154 -> 0.869 ms, against a CTA per face
+// that kept face values and slopes in shared memory over three velocity sweeps
+// (six, at Nv 2401 two, faces per SM, with barriers around its serial part).
+// Bound by the L1 / shared data pipe (73%: the stencil rows pass it once as
+// cp.async and once as loads) and FP64 issue (49%) at 16 warps per SM.  Measured
+// and not kept (0.730 ms here): no face values stored, the reconstruction run
+// again in sweep 2, 0.917; stencil rows by plain loads a trip ahead, 0.840;
+// rings of 3 or 4 stages, 0.750-0.790; 20 and 24 warps per SM at 96 and 80
+// registers, 0.775 and 1.016 (the rows in flight outgrow L2); two velocities
+// per lane side by side, 0.813; the three parts as launches of their own, 0.866;
+// a CTA per face with threads that hold their v node, 0.801.
+//
+//   sweep 1  reconstruction (iFace); the face values into the face's flux row
+//            (an L2 round trip of 16 bytes a velocity),
+//            nine raw moments that give the face state (getFaceCons) and heat
+//            flux (calcFaceQ);
+//   once     slopes (getPLR), initMacroFlux, time weights: the two sides of the
+//            face on even and odd lanes;
+//   sweep 2  macroFlux and distFlux over the stored values, the slope taken
+//            again as (face value - upwind cell) / distance.
+//
+// Face record (per warp, shared memory): polynomials a0 + ax x + ay y + a3 (x^2
+// + y^2) in the global velocity components, time weights, face state.  It
+// takes the place of the moments.
+enum {
+  FK_L = 0, FK_R = 6, FK_T = 12, FK_MT3 = 18, FK_MT4, FK_SX, FK_SY, FK_G0, FK_UX = FK_G0 + 4, FK_UY, FK_LAM, FK_KB,
+  FK_CHL, FK_NUM
+};
+constexpr int FACE_MOM = 9;    // h, xh, yh, xxh, xyh, yyh, b, x t, y t with t = (x^2 + y^2) h + b / K
+constexpr int FACE_TAB = 32;   // doubles of a record
+static_assert(FK_NUM <= FACE_TAB && FACE_MOM <= FACE_TAB, "face record layout");
+
+// what both sweeps of a face need
+template <int FM>
+struct FaceRows {
+  V2 n;
+  double dist0, idist0, il0, dist1, idist1, il1;
+  int step;
+  const double2 *fcell;  // cell (gi, gj), velocity 0
+  double2 *row;          // the face's flux row
+  static constexpr int L = FM == 1 ? 5 : 3, MID = FM == 1 ? 2 : 1;
+  __device__ __forceinline__ FaceRows(const ugks_fused_block &blk, const FaceWork &w) {
+    const ugks_block_desc &d = blk.d;
+    const size_t fk = faceidx(d, w.gi, w.gj, w.dir), base = fidx(d, w.gi, w.gj, 0);
+    n = ld2(blk.normal, fk);
+    const double *g = blk.face_geo + 6 * fk;
+    dist0 = g[0]; idist0 = g[1]; il0 = g[2]; dist1 = g[3]; idist1 = g[4]; il1 = g[5];
+    step = w.dir == SOUTH ? d.Nv : d.Nj * d.Nv;
+    fcell = reinterpret_cast<const double2 *>(blk.f) + base;
+    row = reinterpret_cast<double2 *>(w.dir == SOUTH ? blk.flux_S : blk.flux_W) + base;
+  }
+  __device__ __forceinline__ bool up(double2 e) const { return fma(e.x, n.x, e.y * n.y) > 0.0; }
+  // stencil cell 0 and the signed stride of velocity v
+  __device__ __forceinline__ const double2 *stencil(int v, bool u, int &st) const {
+    st = u ? step : -step;
+    return fcell + (v + (u ? -(MID + 1) * step : MID * step));
+  }
+  __device__ __forceinline__ void value(const double2 (&x)[L], bool u, double &h, double &b, double &sh,
+                                        double &sb) const {
+    reconstruct<FM>(x, u ? il1 : il0, u ? dist1 : dist0, u ? idist1 : idist0, h, b, sh, sb);
+  }
+};
+__device__ __forceinline__ void add_moments(double2 e, double Kinv, double h, double b, double (&m)[FACE_MOM]) {
+  const double xh = e.x * h, yh = e.y * h;
+  const double t = fma(fma(e.x, e.x, e.y * e.y), h, b * Kinv);
+  m[0] += h;
+  m[1] += xh;
+  m[2] += yh;
+  m[3] = fma(e.x, xh, m[3]);
+  m[4] = fma(e.y, xh, m[4]);
+  m[5] = fma(e.y, yh, m[5]);
+  m[6] += b;
+  m[7] = fma(e.x, t, m[7]);
+  m[8] = fma(e.y, t, m[8]);
+}
+
+// stages of cp.async in flight per lane: the stencil rows of FACE_RING
+// velocities in sweep 1, (face value, upwind cell) of as many as fit in the
+// same memory in sweep 2; a lane reads back only what it copied
+constexpr int FACE_RING = 2;
+template <int FM>
+constexpr int face_ring_elems() { return FACE_RING * FaceRows<FM>::L * 32; }
+
+// The per-face coefficients, by the face's warp: `rec` holds the moments and
+// receives the record.  Even lanes compute the side before the face, odd lanes
+// the side after it (the same instructions with one sign flipped).  Not
+// inlined: it runs once per face, and its registers (about 130) would weigh on
+// the sweeps, which run at 96.
+__device__ __noinline__ void face_coefficients(const ugks_fused_block &blk, double dt, const FaceWork fwk,
+                                               double *rec) {
   const ugks_block_desc &d = blk.d;
-  ugks_solve_state &sol = solves[blk.solve];
-  const double dt = sol.dt;
-  const int dir = fwk.dir, mi = fwk.mi, mj = fwk.mj, wall = fwk.wall;
-  const long gi = fwk.gi, gj = fwk.gj;
-  const int Nv = d.Nv;
-
-  // per velocity: (h, b) at the face and their slopes, kept for the later
-  // sweeps in shared memory
-  double2 *fhb = reinterpret_cast<double2 *>(dyn), *sgb = fhb + Nv;
-  const V2 n = ld2(blk.normal, faceidx(d, gi, gj, dir));
-  const V2 mid = ld2(blk.mid_side, faceidx(d, gi, gj, dir));
-  // velocity tables and the face-frame velocity (interfaceVelocity,
-  // clFunctions.c:191-209), with the table pointers held in registers
-  const double2 *__restrict__ qd = reinterpret_cast<const double2 *>(d.quad);
-  const double *__restrict__ wt = d.weight;
-  auto fvel = [&](int vv) {
-    const double2 e = qd[vv];
-    return v2(e.x * n.x + e.y * n.y, e.x * (-n.y) + e.y * n.x);
-  };
-  // stencil geometry for both upwind directions (iFace, clUGKS.c:148-176),
-  // precomputed by face_geometry: index 1 for u > 0 (upwind cell before the
-  // face), 0 otherwise
-  double g6[6];
-  {
-    const double *fg = blk.face_geo + 6 * faceidx(d, gi, gj, dir);
+  const int lane = threadIdx.x & 31, side = lane & 1;
+  double M[FACE_MOM];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) g6[k] = fg[k];
+  for (int k = 0; k < FACE_MOM; ++k) M[k] = rec[k];
+  __syncwarp();  // every lane has the moments before the record takes their place
+  const int dir = fwk.dir;
+  const long gi = fwk.gi, gj = fwk.gj;
+  const size_t fk = faceidx(d, gi, gj, dir);
+  const size_t ck = side == 0 ? gidx(d, gi - dir, gj - (1 - dir)) : gidx(d, gi, gj);
+  const P4 mc = ld4(blk.cell_mom, ck);
+  const V2 cc = ld2(blk.centre, ck), mid = ld2(blk.mid_side, fk), n = ld2(blk.normal, fk);
+  const double len = blk.side_length[fk], Kinv = nr_rcp(d.K);
+  const V2 Wm = to_local(v2(M[1], M[2]), n);
+  const P4 W = p4(M[0], Wm.x, Wm.y, 0.5 * (M[3] + M[5] + M[6]));
+  Rcp rc;
+  const P4 prim = to_primary_rcp(d, W, rc);  // getPLR (clUGKS.c:421-422)
+  const V2 Ug = to_global(v2(prim.s1, prim.s2), n);
+  const double kb = (0.5 * d.K) * rc.lam, sg = side == 0 ? 1.0 : -1.0;
+  double Mh[MNUM], Mv[MTUM], Mxi[3];
+  half_moments_rcp(d.PI, d.K, prim, rc, sg, Mh, Mv, Mxi);
+  // left: (W - W_L) / |mid - c_L|; right: (W_R - W) / |mid - c_R|
+  const V2 uc = to_local(v2(mc.s1, mc.s2), n);
+  const double id = sg * nr_rcp(sqrt((mid.x - cc.x) * (mid.x - cc.x) + (mid.y - cc.y) * (mid.y - cc.y)));
+  const P4 a = micro_slope_rcp(d.K, prim, rc,
+                               p4((W.s0 - mc.s0) * id, (W.s1 - uc.x) * id, (W.s2 - uc.y) * id, (W.s3 - mc.s3) * id));
+  // sums over both sides, by exchange with the neighbouring lane
+  auto both = [](double z) { return z + __shfl_xor_sync(0xffffffffu, z, 1); };
+  auto both4 = [&](P4 z) { return p4(both(z.s0), both(z.s1), both(z.s2), both(z.s3)); };
+  const P4 t1 = both4(moment_au(a, Mh, Mv, Mxi, 1, 0)), t2 = both4(moment_au(a, Mh, Mv, Mxi, 2, 0));
+  double Mu[MNUM];
+#pragma unroll
+  for (int k = 0; k < MNUM; ++k) Mu[k] = both(Mh[k]);
+  const P4 aT = micro_slope_rcp(d.K, prim, rc, scale(-prim.s0, t1));
+  double Mt[5];
+  time_weights_rcp(inv_relax_time_rcp(d, prim, rc), dt, Mt);
+  const P4 g0 = scale(prim.s0, add(add(scale(Mt[0], moment_uv(Mu, Mv, Mxi, 1, 0, 0)), scale(Mt[1], t2)),
+                                   scale(Mt[2], moment_au(aT, Mu, Mv, Mxi, 1, 0))));
+  // calcQ of the face values (calcFaceQ, clUGKS.c:522-585) from their raw
+  // moments about 0, global frame; times the Shakhov factor and Mt0
+  const double cu = fma(Ug.x, M[1], Ug.y * M[2]), U2 = fma(Ug.x, Ug.x, Ug.y * Ug.y);
+  const double T = fma(Kinv, M[6], M[3] + M[5]) - 2.0 * cu + U2 * M[0];
+  const double qx = M[7] - 2.0 * fma(Ug.x, M[3], Ug.y * M[4]) + U2 * M[1] - Ug.x * T;
+  const double qy = M[8] - 2.0 * fma(Ug.x, M[4], Ug.y * M[5]) + U2 * M[2] - Ug.y * T;
+  const double s0 = 0.4 * (1 - d.Pr) * (prim.s3 * prim.s3) * rc.rho * Mt[0];  // 0.8 ..., q = 1/2 sum
+  const double xk = Mxi[2] - kb * kb;
+  // a1 u + a2 v = x (a1 n.x - a2 n.y) + y (a1 n.y + a2 n.x)
+  auto put = [&](double *c, P4 z, double w, double w0) {
+    c[0] = fma(w, fma(0.5 * z.s3, kb, z.s0), w0);
+    c[1] = w * (z.s1 * n.x - z.s2 * n.y);
+    c[2] = w * (z.s1 * n.y + z.s2 * n.x);
+    c[3] = w * (0.5 * z.s3);
+    c[4] = w * (0.5 * z.s3 * xk);
+  };
+  if (lane < 2) put(rec + FK_L + 6 * side, a, Mt[1], 0.0);
+  if (lane == 2) put(rec + FK_T, aT, Mt[2], Mt[0]);
+  if (lane == 3) {
+    rec[FK_MT3] = Mt[3] * len;
+    rec[FK_MT4] = Mt[4] * len;
+    rec[FK_SX] = s0 * qx;
+    rec[FK_SY] = s0 * qy;
+    const V2 g = to_global(v2(g0.s1, g0.s2), n);
+    rec[FK_G0] = len * g0.s0;
+    rec[FK_G0 + 1] = len * g.x;
+    rec[FK_G0 + 2] = len * g.y;
+    rec[FK_G0 + 3] = len * g0.s3;
+    rec[FK_UX] = Ug.x;
+    rec[FK_UY] = Ug.y;
+    rec[FK_LAM] = prim.s3;
+    rec[FK_KB] = kb;
+    // Maxwellian prefactor rho lambda / pi (fM, clFunctions.c:49-58) times the
+    // face length: every per-velocity flux carries the length
+    rec[FK_CHL] = prim.s0 * prim.s3 * nr_rcp(d.PI) * len;
   }
-  const double dist0 = g6[0], idist0 = g6[1], il0 = g6[2], dist1 = g6[3], idist1 = g6[4], il1 = g6[5];
-  const int step = dir == SOUTH ? Nv : d.Nj * Nv;
-  const size_t base = fidx(d, gi, gj, 0);
-  constexpr int MID = FM == 1 ? 2 : 1;
-  const double2 *fcell = reinterpret_cast<const double2 *>(blk.f) + base;  // cell (gi, gj), velocity 0
-  const double2 *up1 = fcell - (MID + 1) * step, *up0 = fcell + MID * step;
+}
 
-  // ---- sweep 1: reconstruction (+ interior faces: the face moments W of
-  // getFaceCons; the 1/2 of the energy moment is applied after the sum)
-  double m[4] = {0.0, 0.0, 0.0, 0.0};
+// the Maxwellian factor of a velocity on a grid that is not a tensor product
+__device__ __noinline__ double plain_exp(double x) { return exp(x); }
+
+// Sweep 2.  With h0 = weight * fM (times the face length), kb = K / (2 lambda),
+// S = Mt0 s (c . Q) (the Shakhov factor of fS, clFunctions.c:64-77, times
+// Mt0), P4 = 2 lambda c^2 - 4, the upwind slope a (aL for u > 0, else aR),
+//   Ph = a0 + a1 u + a2 v + a3 (|u|^2 + kb) / 2, and Th likewise with aT,
+//   Rh = Mt3 fh - Mt4 u sh,   Rb = Mt3 fb - Mt4 u sb,
+//   Zh = u (S P4 h0 + Rh),    Zb = u (S (P4 + 2) kb h0 + Rb),
+//   B  = Mt0 + Mt1 u Ph + Mt2 Th,
+// distFlux's (clUGKS.c:683-772) two components are
+//   hx = Zh + u h0 B,
+//   hy = Zb + u h0 (kb B + Mt1 u a3 X / 2 + Mt2 aT3 X / 2),  X = Mxi2 - kb^2,
+// and macroFlux's (587-681) discrete part sums (Zh, x Zh, y Zh, (|u|^2 Zh + Zb) / 2)
+// in the global frame.
+template <int FM>
+__device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, const ugks_solve_state &sol, double *rec,
+                                               double2 *ring, const FaceWork &fwk) {
+  const ugks_block_desc &d = blk.d;
+  const int lane = threadIdx.x & 31, Nv = d.Nv, un = d.u_num, vn = d.v_num;
+  const FaceRows<FM> F(blk, fwk);
+  constexpr int L = FaceRows<FM>::L, D = FACE_RING, D2 = face_ring_elems<FM>() / 64;
+  const double2 *__restrict__ qd = reinterpret_cast<const double2 *>(d.quad);
+  ring += lane;
+  {
+    auto issue = [&](int v, int stage) {
+      if (v < Nv) {
+        int st;
+        const double2 *p = F.stencil(v, F.up(qd[v]), st);
+        double2 *r = ring + stage * (L * 32);
+#pragma unroll
+        for (int s = 0; s < L; ++s) cp_async<16, true>(r + 32 * s, p + s * st);
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < D; ++s) issue(lane + 32 * s, s);
+    double m[FACE_MOM] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const double Kinv = nr_rcp(d.K);
+    int stage = 0;
 #pragma unroll 1
-  for (int v = threadIdx.x; v < Nv; v += NT) {
-    const V2 uv = fvel(v);
-    const bool up = uv.x > 0.0;
-    double ffh, ffb, sx, sy;
-    reconstruct<double, FM>((up ? up1 : up0) + v, up ? step : -step, up ? il1 : il0, up ? dist1 : dist0,
-                            up ? idist1 : idist0, ffh, ffb, sx, sy);
-    fhb[v] = make_double2(ffh, ffb);
-    sgb[v] = make_double2(sx, sy);
-    if (wall < 0) {
-      const double uu = fma(uv.x, uv.x, uv.y * uv.y);
-      m[0] += ffh;
-      m[1] = fma(uv.x, ffh, m[1]);
-      m[2] = fma(uv.y, ffh, m[2]);
-      m[3] += fma(uu, ffh, ffb);
+    for (int v = lane; v < Nv; v += 32) {
+      const double2 e = qd[v];
+      cp_async_wait<D - 1>();
+      double2 xs[L];
+      const double2 *r = ring + stage * (L * 32);
+#pragma unroll
+      for (int s = 0; s < L; ++s) xs[s] = r[32 * s];
+      double h, b, sh, sb;
+      F.value(xs, F.up(e), h, b, sh, sb);
+      F.row[v] = make_double2(h, b);
+      issue(v + 32 * D, stage);
+      stage = stage + 1 == D ? 0 : stage + 1;
+      add_moments(e, Kinv, h, b, m);
     }
+    cp_async_wait<0>();
+    const double t = warp_spread_sum<FACE_MOM>(m);
+    constexpr int S = spread_shift<FACE_MOM>();
+    if ((lane & ((1 << S) - 1)) == 0 && (lane >> S) < FACE_MOM) rec[lane >> S] = t;
   }
-  // loaded by the last warp, which has the fewest velocities in sweep 1
-  if (wall < 0) face_neighbours<NT>(blk, sh, gi, gj, dir, n, mid);
-  const double len = blk.side_length[faceidx(d, gi, gj, dir)];
-
-  if (wall < 0) {
-    // ---------------- interior face ----------------
-    block_sum_spread<4>(m, sh.scratch);
-    const P4 W = p4(m[0], m[1], m[2], 0.5 * m[3]);
-    Rcp rc;
-    const P4 prim = to_primary_rcp(d, W, rc);  // getPLR (clUGKS.c:421-422), every thread
-    const int un = d.u_num, vn = d.v_num;
-    const bool sep = un > 0 && un * vn == Nv && un + vn <= 512;
-    double *Eu = reinterpret_cast<double *>(sgb + Nv), *Ev = Eu + (sep ? un : 0);
-    const V2 Ug = to_global(v2(prim.s1, prim.s2), n);  // face mean velocity, global frame
-    // Maxwellian prefactor rho lambda / pi (fM, clFunctions.c:49-58), times the
-    // face length: every per-velocity flux below carries the length
-    const double chl = (prim.s0 * (prim.s3 / d.PI)) * len;
-    double q[2] = {0.0, 0.0};
-    face_coefficients<NT>(d, sh, W, prim, rc, len, dt, [&](int t, int nt) {
-      // face heat flux (calcFaceQ, clUGKS.c:522-585) and the axis factors of
-      // the face Maxwellian
-      const double Kinv = 1.0 / d.K;
-      for (int v = t; v < Nv; v += nt) {
-        const V2 uv = fvel(v);
-        const double cx = uv.x - prim.s1, cy = uv.y - prim.s2, c2 = cx * cx + cy * cy;
-        const double2 fv = fhb[v];
-        const double tq = c2 * fv.x + fv.y * Kinv;
-        q[0] += 0.5 * (cx * tq);
-        q[1] += 0.5 * (cy * tq);
-      }
-      if (sep) {
-        axis_exp(Eu, d.quad, un, vn, 0, Ug.x, prim.s3, t, nt, chl);
-        axis_exp(Ev, d.quad, vn, 1, 1, Ug.y, prim.s3, t, nt);
-      }
-    });
-    block_sum_spread<2>(q, sh.scratch);
-    // ---- sweep 3: macroFlux (587-681) and distFlux (683-772).
-    // With h0 = weight * fM (times the face length), kb = K / (2 lambda),
-    // S = Mt0 s (c . Q) (the Shakhov factor of fS, clFunctions.c:64-77, times
-    // Mt0), P4 = 2 lambda c^2 - 4, the upwind slope a (aL for u > 0, else aR),
-    //   Ph = a0 + a1 u + a2 v + a3 (|u|^2 + kb) / 2, and Th likewise with aT,
-    //   Rh = Mt3 fh - Mt4 u sh,   Rb = Mt3 fb - Mt4 u sb,
-    //   Zh = u (S P4 h0 + Rh),    Zb = u (S (P4 + 2) kb h0 + Rb),
-    //   B  = Mt0 + Mt1 u Ph + Mt2 Th,
-    // distFlux's two components are
-    //   hx = Zh + u h0 B,
-    //   hy = Zb + u h0 (kb B + Mt1 u a3 X / 2 + Mt2 aT3 X / 2),  X = Mxi2 - kb^2,
-    // and macroFlux's discrete part sums (Zh, u Zh, v Zh, (|u|^2 Zh + Zb) / 2).
-    const double *c = sh.bcast;
-    const V2 Q = v2(q[0], q[1]);
-    const double lam = prim.s3, Ux = prim.s1, Uy = prim.s2, lam2 = 2.0 * lam;
-    const double kb = (0.5 * d.K) * rc.lam;
-    const double s0 = 0.8 * (1 - d.Pr) * (lam * lam) * rc.rho;
-    const double Mt0 = c[15], Mt3 = c[16], Mt4 = c[17];
-    const double sx = (Mt0 * s0) * Q.x, sy = (Mt0 * s0) * Q.y;
-    const double T0 = c[10], T1 = c[11], T2 = c[12], T3 = c[13], CT = c[14];
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    void *flux = dir == SOUTH ? blk.flux_S : blk.flux_W;
-    const int qs = sep ? NT / vn : 0, rs = sep ? NT % vn : 0;
-    int iu = sep ? threadIdx.x / vn : 0, jv = sep ? threadIdx.x % vn : 0;
-    for (int v = threadIdx.x; v < Nv; v += NT) {
-      const V2 uv = fvel(v);
-      const double u = uv.x, vt = uv.y, uu = fma(u, u, vt * vt);
-      const double cx = u - Ux, cy = vt - Uy, c2 = fma(cx, cx, cy * cy);
+  __threadfence_block();  // this lane's row[] before its copies of it
+  __syncwarp();
+  auto issue = [&](int v, int stage) {
+    if (v < Nv) {
+      const bool u = F.up(qd[v]);
+      double2 *r = ring + stage * 64;
+      cp_async<16>(r, F.row + v);
+      cp_async<16>(r + 32, F.fcell + v - (u ? F.step : 0));
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < D2; ++s) issue(lane + 32 * s, s);  // under the coefficients
+  face_coefficients(blk, sol.dt, fwk, rec);
+  __syncwarp();
+  const bool sep = un > 0 && un * vn == Nv && un + vn <= 512;
+  double *Eu = rec + FACE_TAB, *Ev = Eu + un;
+  const double lam = rec[FK_LAM], Ux = rec[FK_UX], Uy = rec[FK_UY], kb = rec[FK_KB];
+  if (sep) {
+    // axis factors of the face Maxwellian, the prefactor on the u axis
+    const double chl = rec[FK_CHL];
+    for (int k = lane; k < un + vn; k += 32) {
+      const double z = k < un ? qd[(size_t)k * vn].x - Ux : qd[k - un].y - Uy;
+      Eu[k] = (k < un ? chl : 1.0) * exp(-lam * (z * z));
+    }
+    __syncwarp();
+  }
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  {
+    const double lam2 = 2.0 * lam, sx = rec[FK_SX], sy = rec[FK_SY], Mt3 = rec[FK_MT3], Mt4 = rec[FK_MT4];
+    const double T0 = rec[FK_T], T1 = rec[FK_T + 1], T2 = rec[FK_T + 2], T3 = rec[FK_T + 3], CT = rec[FK_T + 4];
+    const double *__restrict__ wt = d.weight;
+    const int qs = sep ? 32 / vn : 0, rs = sep ? 32 % vn : 0;
+    int iu = sep ? lane / vn : 0, jv = sep ? lane % vn : 0;
+    int stage = 0;
+#pragma unroll 1
+    for (int v = lane; v < Nv; v += 32) {
+      const double2 e = qd[v];
+      const double wv = wt[v];
+      const double u = fma(e.x, F.n.x, e.y * F.n.y), uu = fma(e.x, e.x, e.y * e.y);
+      const double cx = e.x - Ux, cy = e.y - Uy, c2 = fma(cx, cx, cy * cy);
       double E;
       if (sep) {
         E = Eu[iu] * Ev[jv];
@@ -1060,43 +1070,136 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block *__restric
         iu += qs;
         if (jv >= vn) { jv -= vn; ++iu; }
       } else {
-        E = chl * exp(-lam * c2);
+        E = rec[FK_CHL] * plain_exp(-lam * c2);
       }
-      const double h0 = wt[v] * E;
+      const double h0 = wv * E;
       const double Sp = fma(cx, sx, cy * sy);
       const double S4 = Sp * fma(lam2, c2, -4.0), S2 = fma(2.0, Sp, S4);
-      const double *A = c + (u > 0.0 ? 0 : 5);
-      const double MP = fma(A[3], uu, fma(A[2], vt, fma(A[1], u, A[0])));
-      const double Bk = fma(u, MP, fma(T3, uu, fma(T2, vt, fma(T1, u, T0))));
-      const double2 fd = fhb[v], fs = sgb[v];
-      const double mu = Mt4 * u;
-      const double Rh = fma(-mu, fs.x, Mt3 * fd.x), Rb = fma(-mu, fs.y, Mt3 * fd.y);
+      const double *A = rec + (u > 0.0 ? FK_L : FK_R);
+      const double MP = fma(A[3], uu, fma(A[2], e.y, fma(A[1], e.x, A[0])));
+      const double Bk = fma(u, MP, fma(T3, uu, fma(T2, e.y, fma(T1, e.x, T0))));
+      cp_async_wait<D2 - 1>();
+      const double2 fd = ring[stage * 64], fc = ring[stage * 64 + 32];
+      issue(v + 32 * D2, stage);
+      stage = stage + 1 == D2 ? 0 : stage + 1;
+      const double mu = (Mt4 * u) * (u > 0.0 ? F.idist1 : F.idist0);
+      const double Rh = fma(-mu, fd.x - fc.x, Mt3 * fd.x), Rb = fma(-mu, fd.y - fc.y, Mt3 * fd.y);
       const double Zh = u * fma(S4, h0, Rh), Zb = u * fma(S2, h0 * kb, Rb);
       const double uh = u * h0;
       const double hx = fma(uh, Bk, Zh);
       const double hy = fma(uh, fma(kb, Bk, fma(A[4], u, CT)), Zb);
       acc[0] += Zh;
-      acc[1] = fma(u, Zh, acc[1]);
-      acc[2] = fma(vt, Zh, acc[2]);
-      acc[3] = fma(uu, Zh, acc[3]);
-      acc[4] += Zb;
-      St::store(flux, base + v, v2(hx, hy));
+      acc[1] = fma(e.x, Zh, acc[1]);
+      acc[2] = fma(e.y, Zh, acc[2]);
+      acc[3] = fma(uu, Zh, acc[3]) + Zb;
+      // streamed: read next by the cell pass, a gigabyte of other traffic later
+      __stcs(F.row + v, make_double2(hx, hy));
     }
-    block_sum_spread_to0<5>(acc, sh.scratch);
-    if (threadIdx.x == 0) {
-      P4 out = p4(acc[0] + c[18], acc[1] + c[19], acc[2] + c[20], 0.5 * (acc[3] + acc[4]) + c[21]);
-      const V2 g = to_global(v2(out.s1, out.s2), n);
-      out.s1 = g.x;
-      out.s2 = g.y;
-      st4(dir == SOUTH ? blk.flux_macro_S : blk.flux_macro_W, gidx(d, gi, gj), out);
-    }
+    cp_async_wait<0>();
+  }
+  acc[3] *= 0.5;
+  const double t = warp_spread_sum<4>(acc);
+  constexpr int S = spread_shift<4>();
+  if ((lane & ((1 << S) - 1)) == 0) {
+    const int k = lane >> S;
+    (fwk.dir == SOUTH ? blk.flux_macro_S : blk.flux_macro_W)[4 * gidx(d, fwk.gi, fwk.gj) + k] = t + rec[FK_G0 + k];
+  }
+  __syncwarp();  // the record is free again
+}
+
+// A wall face in FP64 (all NT threads of the CTA take part): the face values
+// are reconstructed into the face's flux row, which the wall procedure works
+// on in place (each thread reads back only what it wrote); the reflected
+// incoming distribution it gathers from is read where P1 put it, wall_dist.
+template <int FM, int NT>
+__device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_solve_state &sol, FaceShared<NT> &sh,
+                                            const FaceWork fwk) {
+  const ugks_block_desc &d = blk.d;
+  const int dir = fwk.dir, Nv = d.Nv;
+  const long gi = fwk.gi, gj = fwk.gj;
+  const size_t fk = faceidx(d, gi, gj, dir), base = fidx(d, gi, gj, 0);
+  const V2 n = ld2(blk.normal, fk);
+  const double *fg = blk.face_geo + 6 * fk;
+  const int step = dir == SOUTH ? Nv : d.Nj * Nv;
+  constexpr int L = FM == 1 ? 5 : 3, MID = FM == 1 ? 2 : 1;
+  const double2 *fcell = reinterpret_cast<const double2 *>(blk.f) + base;
+  const double2 *up1 = fcell - (MID + 1) * step, *up0 = fcell + MID * step;
+  const double2 *qd = reinterpret_cast<const double2 *>(d.quad);
+  double2 *row = reinterpret_cast<double2 *>(dir == SOUTH ? blk.flux_S : blk.flux_W) + base;
+  for (int v = threadIdx.x; v < Nv; v += NT) {
+    const double2 e = qd[v];
+    const bool up = fma(e.x, n.x, e.y * n.y) > 0.0;
+    const double *g = fg + (up ? 3 : 0);
+    double2 xs[L];
+    load_stencil((up ? up1 : up0) + v, up ? step : -step, xs);
+    double h, b, sx, sy;
+    reconstruct<FM>(xs, g[2], g[0], g[1], h, b, sx, sy);
+    row[v] = make_double2(h, b);
+  }
+  const long ci = dir == SOUTH ? fwk.mi : fwk.mj;
+  wall_face<NT>(blk, sol, sh, reinterpret_cast<double *>(row),
+                reinterpret_cast<double2 *>(blk.wall_dist) + (size_t)ci * Nv, fwk.wall, dir, gi, gj, fwk.mi, fwk.mj, n,
+                blk.side_length[fk], sol.dt, [&](int v, double hx, double hy) { row[v] = make_double2(hx, hy); });
+}
+
+// wall work item (2 (ni + nj) per block: the S faces of rows 0 and nj, then
+// the W faces of columns 0 and ni) -> the face work item of that face
+__device__ __forceinline__ int wall_to_face(const ugks_fused_block &blk, int w) {
+  const ugks_block_desc &d = blk.d;
+  int lw = w - blk.wall_begin, mi, mj, dir;
+  if (lw < 2 * d.ni) {
+    dir = SOUTH;
+    mi = lw % d.ni;
+    mj = lw < d.ni ? 0 : d.nj;
+  } else {
+    lw -= 2 * d.ni;
+    dir = WEST;
+    mj = lw % d.nj;
+    mi = lw < d.nj ? 0 : d.ni;
+  }
+  return blk.face_begin + ((mi * (d.nj + 1) + mj) << 1) + dir;
+}
+
+// a wall work item of any flux method (all threads of the CTA)
+template <int NT>
+__device__ __forceinline__ void wall_work_fp64(const ugks_fused_block *__restrict__ B, int nb,
+                                               ugks_solve_state *__restrict__ solves, const int w, int retry_pass) {
+  __shared__ FaceShared<NT> sh;
+  const ugks_fused_block &blk = B[find_block<3>(B, nb, w)];
+  UGKS_CHECK_ITEM(3, blk, w, solves);
+  FaceWork fwk;
+  if (!face_work<-1>(B, nb, solves, wall_to_face(blk, w), retry_pass, fwk) || fwk.wall < 0) return;
+  ugks_solve_state &sol = solves[blk.solve];
+  switch (blk.d.flux_method) {
+    case 0: wall_item_fp64<0, NT>(blk, sol, sh, fwk); break;
+    case 1: wall_item_fp64<1, NT>(blk, sol, sh, fwk); break;
+    case 3: wall_item_fp64<3, NT>(blk, sol, sh, fwk); break;
+    default: break;
+  }
+}
+
+// FP64 face pass: the first n_wall CTAs take a wall work item each (they are
+// the longest, so they start first), the others WPC interior faces, one per warp
+template <int FM, int WPC>
+__device__ __forceinline__ double2 *face_ring(double *dyn, int wstride, int warp) {
+  return reinterpret_cast<double2 *>(dyn + WPC * wstride) + warp * face_ring_elems<FM>();
+}
+template <int FM, int WPC, int MINB>
+__global__ void __launch_bounds__(WPC * 32, MINB) face_pass_fp64(const ugks_fused_block *__restrict__ B, int nb,
+                                                                 ugks_solve_state *__restrict__ solves, int n_wall,
+                                                                 int first, int count, int wstride) {
+  extern __shared__ double dyn[];
+  if ((int)blockIdx.x < n_wall) {
+    wall_work_fp64<WPC * 32>(B, nb, solves, (int)blockIdx.x, 0);
     return;
   }
-
-  // ---------------- wall face ----------------
-  wall_face<NT>(blk, sol, sh, reinterpret_cast<double *>(fhb), sgb, wall, dir, gi, gj, mi, mj, n, len, dt,
-                [&](int v, double hx, double hy) { St::store(dir == SOUTH ? blk.flux_S : blk.flux_W, base + v,
-                                                               v2(hx, hy)); });
+  const int warp = threadIdx.x >> 5;
+  const int item = ((int)blockIdx.x - n_wall) * WPC + warp;
+  if (item >= count) return;
+  FaceWork fwk;
+  if (!face_work<FM, true>(B, nb, solves, first + item, 0, fwk) || fwk.wall >= 0) return;
+  const ugks_fused_block &blk = B[fwk.bi];
+  face_item_fp64<FM>(blk, solves[blk.solve], dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
 }
 
 // the mixed path's face work item (ugks_delta.cuh, included further down):
@@ -1106,38 +1209,53 @@ template <int FM, int NT, bool WALLS>
 __device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                 ugks_solve_state *__restrict__ solves, const int w, int retry_pass);
 
-// one face work item: FP64 storage, or the mixed path's FP32 deviations
-template <typename T, int FM, int NT, bool RETRY>
-__device__ __forceinline__ void face_item(const ugks_fused_block *__restrict__ B, int nb,
-                                          ugks_solve_state *__restrict__ solves, const int w) {
-  if constexpr (std::is_same<T, float>::value) face_item_delta<FM, NT, RETRY>(B, nb, solves, w, RETRY ? 1 : 0);
-  else face_item_fp64<FM, NT>(B, nb, solves, w, RETRY ? 1 : 0);
-}
-
-// main face pass: one CTA per face work item of the blocks of one flux method
-template <typename T, int FM, int MINB, int NT>
-__global__ void __launch_bounds__(NT, MINB) face_pass(const ugks_fused_block *__restrict__ B, int nb,
-                                                                 ugks_solve_state *__restrict__ solves,
-                                                                 int first) {
-  face_item<T, FM, NT, false>(B, nb, solves, first + (int)blockIdx.x);
-}
-
 // the flux pass redone after a dt change (ugks_sim.py:432-441): RETRY_CTAS
 // CTAs per solve; a solve whose retry flag is clear costs one early exit each
 constexpr int RETRY_CTAS = 148;
-template <typename T, int FM, int MINB, int NT>
-__global__ void __launch_bounds__(NT, MINB) face_retry(const ugks_fused_block *__restrict__ B, int nb,
-                                                                  ugks_solve_state *__restrict__ solves,
-                                                                  int ns) {
-  const int s = blockIdx.x / RETRY_CTAS, r = blockIdx.x % RETRY_CTAS;
-  if (s >= ns) return;
+// the solve of a retry CTA of flux method FM, or false
+template <int FM>
+__device__ __forceinline__ bool retry_solve(const ugks_fused_block *__restrict__ B,
+                                            const ugks_solve_state *__restrict__ solves, int ns, int &b0, int &bl) {
+  const int s = blockIdx.x / RETRY_CTAS;
+  if (s >= ns) return false;
   const ugks_solve_state &x = solves[s];
-  if (!x.active || !x.retry || x.nblocks <= 0) return;
-  const ugks_fused_block &b0 = B[x.first_block], &bl = B[x.first_block + x.nblocks - 1];
-  if (b0.d.flux_method != FM) return;
-  const int end = bl.face_begin + 2 * (bl.d.ni + 1) * (bl.d.nj + 1);
-  for (int w = b0.face_begin + r; w < end; w += RETRY_CTAS) {
-    face_item<T, FM, NT, true>(B, nb, solves, w);
+  if (!x.active || !x.retry || x.nblocks <= 0) return false;
+  b0 = x.first_block;
+  bl = x.first_block + x.nblocks - 1;
+  return B[b0].d.flux_method == FM;
+}
+template <int FM, int WPC, int MINB>
+__global__ void __launch_bounds__(WPC * 32, MINB) face_retry_fp64(const ugks_fused_block *__restrict__ B, int nb,
+                                                                  ugks_solve_state *__restrict__ solves, int ns,
+                                                                  int wstride) {
+  extern __shared__ double dyn[];
+  int b0, bl;
+  if (!retry_solve<FM>(B, solves, ns, b0, bl)) return;
+  const int r = blockIdx.x % RETRY_CTAS, warp = threadIdx.x >> 5;
+  const ugks_block_desc &e = B[bl].d;
+  const int wall_end = B[bl].wall_begin + 2 * (e.ni + e.nj);
+  for (int w = B[b0].wall_begin + r; w < wall_end; w += RETRY_CTAS) {
+    wall_work_fp64<WPC * 32>(B, nb, solves, w, 1);
+    __syncthreads();  // the next item reuses the shared tables
+  }
+  const int end = B[bl].face_begin + 2 * (e.ni + 1) * (e.nj + 1);
+  for (int w = B[b0].face_begin + r * WPC + warp; w < end; w += RETRY_CTAS * WPC) {
+    FaceWork fwk;
+    if (!face_work<FM>(B, nb, solves, w, 1, fwk) || fwk.wall >= 0) continue;
+    const ugks_fused_block &blk = B[fwk.bi];
+    face_item_fp64<FM>(blk, solves[blk.solve], dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
+  }
+}
+// mixed: only the wall faces have anything to redo (the interior faces take the
+// dt after the first check)
+template <int FM, int MINB, int NT>
+__global__ void __launch_bounds__(NT, MINB) face_retry(const ugks_fused_block *__restrict__ B, int nb,
+                                                       ugks_solve_state *__restrict__ solves, int ns) {
+  int b0, bl;
+  if (!retry_solve<FM>(B, solves, ns, b0, bl)) return;
+  const int end = B[bl].face_begin + 2 * (B[bl].d.ni + 1) * (B[bl].d.nj + 1);
+  for (int w = B[b0].face_begin + blockIdx.x % RETRY_CTAS; w < end; w += RETRY_CTAS) {
+    face_item_delta<FM, NT, true>(B, nb, solves, w, 1);
     __syncthreads();  // the next item reuses the shared tables
   }
 }
@@ -1718,45 +1836,40 @@ int restart_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, u
   return launch_status();
 }
 
-template <typename T, int FM, int MINB, int NT>
-cudaError_t set_face_attributes() {
-  cudaError_t e = cudaFuncSetAttribute(face_pass<T, FM, MINB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       200 * 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(face_retry<T, FM, MINB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(face_pass<T, FM, MINB, NT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-  return e;
+template <typename K>
+cudaError_t allow_smem(K kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
-
-template <typename T, int V>
+template <int V>
 cudaError_t set_face_shape() {
-  constexpr int NT = FaceShape<T, V>::nt, MINB = FaceShape<T, V>::minb;
-  if constexpr (std::is_same<T, float>::value) {
-    return cudaSuccess;  // mixed: no face_pass (set_wall_attributes covers its retry pass)
-  } else {
-    cudaError_t e = set_face_attributes<T, 0, MINB, NT>();
-    if (e == cudaSuccess) e = set_face_attributes<T, 1, MINB, NT>();
-    if (e == cudaSuccess) e = set_face_attributes<T, 3, MINB, NT>();
-    return e;
+  constexpr int W = FaceShape<V>::wpc, M = FaceShape<V>::minb;
+  cudaError_t r[6] = {allow_smem(face_pass_fp64<0, W, M>), allow_smem(face_pass_fp64<1, W, M>),
+                      allow_smem(face_pass_fp64<3, W, M>), cudaSuccess, cudaSuccess, cudaSuccess};
+  if constexpr (V == 1) {
+    r[3] = allow_smem(face_retry_fp64<0, W, M>);
+    r[4] = allow_smem(face_retry_fp64<1, W, M>);
+    r[5] = allow_smem(face_retry_fp64<3, W, M>);
   }
+  for (cudaError_t e : r)
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
 }
 template <typename T>
 cudaError_t set_wall_attributes() {
+  if constexpr (std::is_same<T, double>::value) {
+    cudaError_t r[4] = {set_face_shape<1>(), set_face_shape<2>(), set_face_shape<3>(), set_face_shape<4>()};
+    for (cudaError_t e : r)
+      if (e != cudaSuccess) return e;
+  }
   if constexpr (std::is_same<T, float>::value) {
     // the wall launch and the retry pass's wall faces (both budgets)
-    cudaError_t e =
-        cudaFuncSetAttribute(wall_pass_delta<WALL_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    constexpr int NN = FT, NW = FaceBudget<float>::wide_threads;
-    constexpr int MN = FaceBudget<float>::narrow, MW = FaceBudget<float>::wide;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(face_retry<float, 0, MN, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(face_retry<float, 1, MN, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(face_retry<float, 3, MN, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(face_retry<float, 0, MW, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(face_retry<float, 1, MW, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(face_retry<float, 3, MW, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return e;
+    constexpr int NN = FT, NW = RETRY_WIDE_NT, MN = RETRY_NARROW_MINB, MW = RETRY_WIDE_MINB;
+    cudaError_t r[7] = {allow_smem(wall_pass_delta<WALL_NT>), allow_smem(face_retry<0, MN, NN>),
+                        allow_smem(face_retry<1, MN, NN>), allow_smem(face_retry<3, MN, NN>),
+                        allow_smem(face_retry<0, MW, NW>), allow_smem(face_retry<1, MW, NW>),
+                        allow_smem(face_retry<3, MW, NW>)};
+    for (cudaError_t e : r)
+      if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -1818,9 +1931,8 @@ cudaError_t set_step_attributes() {
   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> guard(lock);
   if (done[dev]) return cudaSuccess;
-  cudaError_t r[8] = {
-      set_face_shape<T, 1>(), set_face_shape<T, 2>(), set_face_shape<T, 3>(), set_face_shape<T, 4>(),
-      set_cell_attributes<T, 2>(), set_cell_attributes<T, 3>(), set_wall_attributes<T>(), set_flux_attributes<T>()};
+  cudaError_t r[4] = {set_cell_attributes<T, 2>(), set_cell_attributes<T, 3>(), set_wall_attributes<T>(),
+                      set_flux_attributes<T>()};
   for (cudaError_t x : r)
     if (x != cudaSuccess) return x;
   if (std::is_same<T, float>::value) {
@@ -1831,35 +1943,70 @@ cudaError_t set_step_attributes() {
   return cudaSuccess;
 }
 
-// shared memory of a face CTA: FP64, (h, b) and slopes per velocity + axis
-// tables; mixed, the wall procedure's FP64 face values (retry pass; the
-// mixed main pass sizes its warp sweeps itself)
+// the largest velocity grid a step accepts, as bytes against 200 KB: per
+// velocity a face's values and slopes (FP64) or a wall face's values (mixed)
 template <typename T>
-inline size_t face_smem(int max_nv, int max_axes, bool retry = false) {
-  if (std::is_same<T, float>::value) return retry ? delta_wall_smem(max_nv) : 0;
+inline size_t face_limit_bytes(int max_nv, int max_axes) {
+  if (std::is_same<T, float>::value) return delta_wall_smem(max_nv);
   return 4 * sizeof(double) * (size_t)max_nv + sizeof(double) * (size_t)max_axes;
 }
 
-// the main face pass of one segment (one flux method, one register budget)
-template <typename T, int MINB, int NT>
-void launch_segment(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int first,
-                    int count, size_t smem, cudaStream_t st) {
+// doubles of shared memory per FP64 face warp beside its ring: the face record
+// and the axis factors
+inline int face_stride(int max_axes) { return FACE_TAB + ((max_axes + 1) & ~1); }
+template <int FM, int WPC>
+size_t face_smem(int wstride) {
+  return (size_t)WPC * (wstride * sizeof(double) + face_ring_elems<FM>() * sizeof(double2));
+}
+
+// the FP64 face pass of one segment (one flux method) in launch shape v; the
+// first segment's launch takes the wall faces of the whole table with it
+template <int WPC, int MINB>
+void launch_faces_shape(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall, int first,
+                        int count, int axes, cudaStream_t st) {
+  const int ws = face_stride(axes);
+  const unsigned g = (unsigned)(n_wall + (count + WPC - 1) / WPC), t = WPC * 32;
   switch (method) {
-    case 0: face_pass<T, 0, MINB, NT><<<count, NT, smem, st>>>(B, nb, solves, first); break;
-    case 1: face_pass<T, 1, MINB, NT><<<count, NT, smem, st>>>(B, nb, solves, first); break;
-    case 3: face_pass<T, 3, MINB, NT><<<count, NT, smem, st>>>(B, nb, solves, first); break;
+    case 0: face_pass_fp64<0, WPC, MINB><<<g, t, face_smem<0, WPC>(ws), st>>>(B, nb, solves, n_wall, first, count, ws); break;
+    case 1: face_pass_fp64<1, WPC, MINB><<<g, t, face_smem<1, WPC>(ws), st>>>(B, nb, solves, n_wall, first, count, ws); break;
+    case 3: face_pass_fp64<3, WPC, MINB><<<g, t, face_smem<3, WPC>(ws), st>>>(B, nb, solves, n_wall, first, count, ws); break;
     default: break;
+  }
+}
+inline void launch_faces(int v, const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall,
+                         int first, int count, int axes, cudaStream_t st) {
+  switch (v) {
+    case 2: launch_faces_shape<FaceShape<2>::wpc, FaceShape<2>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
+    case 3: launch_faces_shape<FaceShape<3>::wpc, FaceShape<3>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
+    case 4: launch_faces_shape<FaceShape<4>::wpc, FaceShape<4>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
+    default: launch_faces_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
   }
 }
 
 // the retry pass of every flux method (per solve; rare)
-template <typename T, int MINB, int NT>
-void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves,
-                  int ns, size_t smem, cudaStream_t st) {
+template <typename T>
+void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves, int ns,
+                  cudaStream_t st) {
   const unsigned rg = (unsigned)ns * RETRY_CTAS;
-  if (z->face_count[0]) face_retry<T, 0, MINB, NT><<<rg, NT, smem, st>>>(B, nb, solves, ns);
-  if (z->face_count[1]) face_retry<T, 1, MINB, NT><<<rg, NT, smem, st>>>(B, nb, solves, ns);
-  if (z->face_count[3]) face_retry<T, 3, MINB, NT><<<rg, NT, smem, st>>>(B, nb, solves, ns);
+  if constexpr (std::is_same<T, float>::value) {
+    const size_t sm = delta_wall_smem(z->max_nv);
+    constexpr int NN = FT, NW = RETRY_WIDE_NT, MN = RETRY_NARROW_MINB, MW = RETRY_WIDE_MINB;
+    if (z->max_nv <= RETRY_NARROW_NV) {
+      if (z->face_count[0]) face_retry<0, MN, NN><<<rg, NN, sm, st>>>(B, nb, solves, ns);
+      if (z->face_count[1]) face_retry<1, MN, NN><<<rg, NN, sm, st>>>(B, nb, solves, ns);
+      if (z->face_count[3]) face_retry<3, MN, NN><<<rg, NN, sm, st>>>(B, nb, solves, ns);
+    } else {
+      if (z->face_count[0]) face_retry<0, MW, NW><<<rg, NW, sm, st>>>(B, nb, solves, ns);
+      if (z->face_count[1]) face_retry<1, MW, NW><<<rg, NW, sm, st>>>(B, nb, solves, ns);
+      if (z->face_count[3]) face_retry<3, MW, NW><<<rg, NW, sm, st>>>(B, nb, solves, ns);
+    }
+  } else {
+    constexpr int WPC = FaceShape<1>::wpc, MINB = FaceShape<1>::minb, NT = WPC * 32;
+    const int ws = face_stride(z->max_axes);
+    if (z->face_count[0]) face_retry_fp64<0, WPC, MINB><<<rg, NT, face_smem<0, WPC>(ws), st>>>(B, nb, solves, ns, ws);
+    if (z->face_count[1]) face_retry_fp64<1, WPC, MINB><<<rg, NT, face_smem<1, WPC>(ws), st>>>(B, nb, solves, ns, ws);
+    if (z->face_count[3]) face_retry_fp64<3, WPC, MINB><<<rg, NT, face_smem<3, WPC>(ws), st>>>(B, nb, solves, ns, ws);
+  }
 }
 
 // the mixed moments sweep of one segment, in launch shape v (ugks_fused_sizes.seg_variant)
@@ -1899,16 +2046,14 @@ template <typename T>
 int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves,
               int ns, void *stream, void *const *events = nullptr) {
   cudaStream_t st = S(stream);
-  // face pass: (h, b) and slopes per velocity + the two axis factor tables;
   // cell pass: the axis factor tables of the old and new macro state
-  const size_t smem = face_smem<T>(z->max_nv, z->max_axes, true);
   constexpr bool mixed = std::is_same<T, float>::value;
   // doubles of shared memory per cell warp
   const int cstride = mixed ? delta_cell_stride(z->max_axes) : 2 * z->max_axes + CELL_COEF;
   const size_t csmem = (size_t)CW * cstride * sizeof(double) + (mixed ? 0 : (size_t)CW * cell_ring_bytes<T>());
   const cudaError_t attr = set_step_attributes<T>();
   if (attr != cudaSuccess) return -(int)attr;
-  if (smem > 200 * 1024 || csmem > 200 * 1024) return -(int)cudaErrorInvalidValue;
+  if (face_limit_bytes<T>(z->max_nv, z->max_axes) > 200 * 1024 || csmem > 200 * 1024) return -(int)cudaErrorInvalidValue;
   const unsigned sg = (unsigned)((ns + 127) / 128);
   auto mark = [&](int k) {
     if (events && events[k]) cudaEventRecord(reinterpret_cast<cudaEvent_t>(events[k]), st);
@@ -1932,36 +2077,29 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     wall_pass_delta<WALL_NT><<<(unsigned)z->n_wall, WALL_NT, delta_wall_smem(z->max_nv), ws->s>>>(B, nb, solves);
     cudaEventRecord(ws->join, ws->s);
   }
+  int walls = z->n_wall;
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) {
     if (z->seg_count[k] <= 0) continue;
-    const size_t sm = face_smem<T>(z->seg_max_nv[k], z->seg_max_axes[k]);
     int v = z->seg_variant[k];
     const int m = z->seg_method[k], b0 = z->seg_begin[k], n = z->seg_count[k];
+    if (v <= 0 || v > 4) v = 1;
     if constexpr (mixed) {
-      if (v <= 0 || v > 4) v = 1;
       launch_moments(v, B, nb, solves, m, b0, n, z->seg_max_axes[k], st);
     } else {
-      if (v <= 0 || v > 4) v = z->seg_max_nv[k] <= FaceBudget<T>::narrow_max_nv ? 1 : 4;
-      switch (v) {
-        case 1: launch_segment<T, FaceShape<T, 1>::minb, FaceShape<T, 1>::nt>(B, nb, solves, m, b0, n, sm, st); break;
-        case 2: launch_segment<T, FaceShape<T, 2>::minb, FaceShape<T, 2>::nt>(B, nb, solves, m, b0, n, sm, st); break;
-        case 3: launch_segment<T, FaceShape<T, 3>::minb, FaceShape<T, 3>::nt>(B, nb, solves, m, b0, n, sm, st); break;
-        default: launch_segment<T, FaceShape<T, 4>::minb, FaceShape<T, 4>::nt>(B, nb, solves, m, b0, n, sm, st); break;
-      }
+      launch_faces(v, B, nb, solves, m, walls, b0, n, z->seg_max_axes[k], st);
+      walls = 0;
     }
   }
   if (ws) {
     cudaStreamWaitEvent(st, ws->join, 0);
     ws_guard.unlock();
   }
-  const bool narrow = z->max_nv <= FaceBudget<T>::narrow_max_nv;
   // mixed: the interior faces' coefficient and flux launches follow the first
   // dt check (they use its dt), and the events bracket all of the face pass
   if (!mixed) mark(1);
   dt_check<<<sg, 128, 0, st>>>(solves, ns, 0);
   if (!mixed) mark(2);
-  if (narrow) launch_retry<T, FaceBudget<T>::narrow, FT>(B, nb, z, solves, ns, smem, st);
-  else launch_retry<T, FaceBudget<T>::wide, FaceBudget<T>::wide_threads>(B, nb, z, solves, ns, smem, st);
+  launch_retry<T>(B, nb, z, solves, ns, st);
   if (mixed && z->n_faces) {
     face_coef_delta<<<(unsigned)((z->n_faces + 127) / 128), 128, 0, st>>>(B, nb, solves, z->n_faces);
     if (UGKS_FLUX_TMA) {
