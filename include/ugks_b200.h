@@ -435,9 +435,10 @@ int ugks_step_mixed(const ugks_fused_block *blocks_dev, int nblocks, const ugks_
                     ugks_solve_state *solves_dev, int nsolves, UGKS_STREAM);
 
 /* The same step with cudaEventRecord of events[0..7] (cudaEvent_t) on the
-   stream around the phases: [0] start, [1] after the face pass, [2] after the
-   dt check, [3] after the retry face pass, [4] after the second dt check,
-   [5] after the cell pass, [6] after the dt update, [7] after the ghost pass.
+   stream around the phases: [0] start, [1] and [2] after the face
+   pass, [3] and [4] after the retry face pass (mixed: its coefficient and flux
+   launches are part of the face pass, [1]..[4] follow them), [5] and [6] after
+   the cell pass, [7] after the ghost pass, which ends the step (dt update).
    mixed != 0 selects FP32 storage.  A null entry records nothing (each
    record costs the stream a few microseconds).  Used to time each kernel
    live. */

@@ -202,7 +202,7 @@ __device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restri
   const ugks_fused_block &blk = B[fwk.bi];
   const ugks_block_desc &d = blk.d;
   ugks_solve_state &sol = solves[blk.solve];
-  const double dt = sol.dt;
+  const double dt = retry_pass ? step_dt(sol).flux : sol.dt;
   const int dir = fwk.dir, mi = fwk.mi, mj = fwk.mj, wall = fwk.wall;
   const long gi = fwk.gi, gj = fwk.gj;
   const int Nv = d.Nv, NP = npairs(d), vn = d.v_num;
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *_
   if (!face_work<-1>(B, nb, solves, w, 0, fwk) || fwk.wall >= 0) return;
   const ugks_fused_block &blk = B[fwk.bi];
   const ugks_block_desc &d = blk.d;
-  const double dt = solves[blk.solve].dt;
+  const double dt = step_dt(solves[blk.solve]).flux;
   const int dir = fwk.dir;
   const long gi = fwk.gi, gj = fwk.gj;
   const RefMaxwellian ref = ref_of(blk);
@@ -913,70 +913,38 @@ __device__ __forceinline__ float sr_pick(float hi, float lo, uint32_t u16) {
 inline int delta_cell_stride(int max_axes) { return 2 * (max_axes + 1) + CELL_COEF; }
 
 template <int MINB>
-__global__ void __launch_bounds__(CW * 32, MINB) cell_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
+__global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                                    ugks_solve_state *__restrict__ solves,
                                                                    int n_cells, int wstride) {
   extern __shared__ double dyn[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int w = blockIdx.x * CW + warp;
-  if (w >= n_cells) return;
-  const int bi = find_block<1>(B, nb, w);
+  CellWork cw;
+  const bool on = cell_work(B, nb, solves, (int)blockIdx.x * CW + warp, n_cells, cw);
+  const int bi = on ? cw.bi : 0;
   const ugks_fused_block &blk = B[bi];
   const ugks_block_desc &d = blk.d;
-  UGKS_CHECK_ITEM(1, blk, w, solves);
-  ugks_solve_state &sol = solves[blk.solve];
-  if (!sol.active) return;
+  const ugks_solve_state &sol = solves[blk.solve];
   const RefMaxwellian ref = ref_of(blk);
-  const int lc = w - blk.cell_begin;
-  const long mi = lc / d.nj, mj = lc % d.nj;
-  const long gi = mi + d.ghost, gj = mj + d.ghost;
+  const long gi = cw.gi, gj = cw.gj;
   const int NP = npairs(d), un = d.u_num, vn = d.v_num;
+  const size_t cm = on ? midx(d, cw.mi, cw.mj) : 0;
   float4 *TU = reinterpret_cast<float4 *>(dyn + (size_t)warp * wstride), *TV = TU + (un + 1);
-  double *bc = dyn + (size_t)warp * wstride + (wstride - CELL_COEF);
-  const double dt = sol.dt;
-  const P4 old = ld4(blk.macro, midx(d, mi, mj));
-  // calcQ of f^n with the macro of f^n (accumulated by the previous cell pass)
-  const V2 Q = ld2(blk.Q_next, midx(d, mi, mj));
+  const double *bc = dyn + (size_t)warp * wstride + (wstride - CELL_COEF);
+  P4 old = p4(1.0, 0.0, 0.0, 1.0);
+  V2 Q = v2(0.0, 0.0);
+  if (on) {
+    old = ld4(blk.macro, cm);
+    // calcQ of f^n with the macro of f^n (accumulated by the previous cell pass)
+    Q = ld2(blk.Q_next, cm);
+  }
   const double *R = ref.mom;
-  if (lane == 0) {
-    // updateMacro
-    const P4 wc = to_conserved(d, old);
-    const double iA = 1.0 / blk.area[gidx(d, gi, gj)];
-    const P4 s0 = ld4(blk.flux_macro_S, gidx(d, gi, gj)), s1 = ld4(blk.flux_macro_S, gidx(d, gi, gj + 1));
-    const P4 w0 = ld4(blk.flux_macro_W, gidx(d, gi, gj)), w1 = ld4(blk.flux_macro_W, gidx(d, gi + 1, gj));
-    const P4 nw = p4(wc.s0 + (s0.s0 - s1.s0 + w0.s0 - w1.s0) * iA, wc.s1 + (s0.s1 - s1.s1 + w0.s1 - w1.s1) * iA,
-                     wc.s2 + (s0.s2 - s1.s2 + w0.s2 - w1.s2) * iA, wc.s3 + (s0.s3 - s1.s3 + w0.s3 - w1.s3) * iA);
-    Rcp rn, ro;
-    const P4 prim = to_primary_rcp(d, nw, rn);
-    ro.rho = nr_rcp(old.s0);
-    ro.lam = nr_rcp(old.s3);
-    st4(blk.macro, midx(d, mi, mj), prim);
-    st4(blk.prim_old, midx(d, mi, mj), old);
-    st2(blk.Q, midx(d, mi, mj), Q);
-    // UGKS_update (clUGKS.c:1189-1257):
-    //   df' = a1 df + a2 sum(dflux) + a4 (fEQ(old) - M) + a3 (fEQ(new) - M),
-    //   a1 = (1 - dt/2 /tau_old) / D, a2 = 1 / (A D), a3 = dt/2 / (tau D),
-    //   a4 = dt/2 / (tau_old D), D = 1 + dt/2 / tau (a1 + a3 + a4 = 1)
-    const double itau_old = inv_relax_time_rcp(d, old, ro), itau = inv_relax_time_rcp(d, prim, rn);
-    const double hdt = 0.5 * dt, iden = nr_rcp(1.0 + hdt * itau);
-    const double P0pi = ref.P0 * d.PI;
-    bc[0] = prim.s1;
-    bc[1] = prim.s2;
-    bc[2] = prim.s3;
-    bc[3] = (1.0 - hdt * itau_old) * iden;                            // a1
-    bc[4] = iden * iA;                                                // a2
-    bc[5] = hdt * itau * iden;                                        // a3
-    bc[6] = hdt * itau_old * iden;                                    // a4
-    bc[7] = log((prim.s0 * prim.s3) / P0pi);                          // ln(P / P0) new
-    bc[8] = log((old.s0 * old.s3) / P0pi);                            // ln(P / P0) old
-    bc[9] = (0.5 * d.K) * rn.lam;                                     // K / (2 lambda) new
-    bc[10] = 0.8 * (1 - d.Pr) * (prim.s3 * prim.s3) * rn.rho;         // Shakhov factor new
-    const double fq = cfl_freq(blk, prim, mi, mj);
-    atomicMax(&sol.max_freq, (unsigned long long)__double_as_longlong(fq));
-  } else {
+  __syncthreads();  // every warp has its cell's old state before it is updated
+  cta_cell_coefficients<true>(B, nb, solves, n_cells, dyn, wstride);
+  __syncwarp();
+  if (on) {
     // the old state's tables, axis factors and velocities
     const double lnPo = log((old.s0 * old.s3) / (ref.P0 * d.PI));
-    for (int k = lane - 1; k <= un + vn; k += 31) {
+    for (int k = lane; k <= un + vn; k += 32) {
       if (k < un) {
         const double x = d.quad[2 * (size_t)k * vn];
         TU[k] = make_float4((float)axis_expm1(x, old.s1, old.s3, ref.lam0, lnPo), 0.0f, (float)ref.Au[k], (float)x);
@@ -989,20 +957,21 @@ __global__ void __launch_bounds__(CW * 32, MINB) cell_pass_delta(const ugks_fuse
       }
     }
   }
-  __syncwarp();
-  const double nU = bc[0], nV = bc[1], nl = bc[2], lnPn = bc[7];
+  __syncthreads();
+  if (!on) return;
+  const double nU = bc[CC_U], nV = bc[CC_V], nl = bc[CC_LAM], lnPn = bc[CC_LNP];
   for (int k = lane; k < un + vn; k += 32) {
     if (k < un) TU[k].y = (float)axis_expm1(d.quad[2 * (size_t)k * vn], nU, nl, ref.lam0, lnPn);
     else TV[k - un].y = (float)axis_expm1(d.quad[2 * (size_t)(k - un) + 1], nV, nl, ref.lam0);
   }
   __syncwarp();
-  const double a3 = bc[5], a4 = bc[6], kn = bc[9], sn = bc[10];
+  const double a3 = bc[CC_A3], a4 = bc[CC_A4], kn = bc[CC_KN], sn = bc[CC_SN];
   const double ko = (0.5 * d.K) * nr_rcp(old.s3);
   const double so = 0.8 * (1 - d.Pr) * (old.s3 * old.s3) * nr_rcp(old.s0);
-  const float2 fa1 = bc2((float)bc[3]), fa2 = bc2((float)bc[4]), fa3 = bc2((float)a3), fa4 = bc2((float)a4);
+  const float2 fa1 = bc2((float)bc[CC_A1]), fa2 = bc2((float)bc[CC_A2]), fa3 = bc2((float)a3), fa4 = bc2((float)a4);
 #if UGKS_SR_STORE
-  const float a1h = (float)bc[3];
-  const float2 fa1h = bc2(a1h), fna1h = bc2(-a1h), fna1l = bc2(-(float)(bc[3] - (double)a1h));
+  const float a1h = (float)bc[CC_A1];
+  const float2 fa1h = bc2(a1h), fna1h = bc2(-a1h), fna1l = bc2(-(float)(bc[CC_A1] - (double)a1h));
   const uint32_t srseed =
       sr_hash((uint32_t)sol.steps * 0x9e3779b9u + (uint32_t)(bi - sol.first_block) * 0x85ebca6bu);
 #endif
@@ -1093,11 +1062,11 @@ __global__ void __launch_bounds__(CW * 32, MINB) cell_pass_delta(const ugks_fuse
   for (int k = 0; k < 6; ++k) dm[k] = mom[k];
   warp_sum<6>(dm);
   if (lane == 0) {
-    if (isnan(dm[0]) || isnan(dm[3])) atomicExch(&sol.status, 1);
+    if (isnan(dm[0]) || isnan(dm[3])) atomicExch(&solves[blk.solve].status, 1);
     st4(blk.cell_mom, gidx(d, gi, gj),
         p4(R[RM00] + dm[0], R[RM10] + dm[1], R[RM01] + dm[2], 0.5 * ((R[RM20] + R[RM02] + R[RB00]) + dm[3])));
     const V2 qr = heat_flux_from_moments(R, d.K, v2(nU, nV));
-    st2(blk.Q_next, midx(d, mi, mj), v2(qr.x + 0.5 * dm[4], qr.y + 0.5 * dm[5]));
+    st2(blk.Q_next, cm, v2(qr.x + 0.5 * dm[4], qr.y + 0.5 * dm[5]));
   }
 }
 
@@ -1108,8 +1077,9 @@ __global__ void __launch_bounds__(CW * 32, MINB) cell_pass_delta(const ugks_fuse
 // ghosts are fEQ - M in FP64, rounded once
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(FT) ghost_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
-                                                       const ugks_solve_state *__restrict__ solves) {
+                                                       ugks_solve_state *solves, int finish) {
   __shared__ double scratch[4 * (FT / 32)];
+  finish_steps(solves, finish);
   const int w = blockIdx.x;
   const int bi = find_block<2>(B, nb, w);
   const ugks_fused_block &blk = B[bi];
@@ -1228,7 +1198,7 @@ __global__ void __launch_bounds__(FT) ghost_pass_delta(const ugks_fused_block *_
     swap_cell_index(NI, NJ, G, face, iB, jB, that, NIB, NJB);
     if (iB < 0 || iB >= NIB || jB < 0 || jB >= NJB || ob.d.Nv != Nv || ob.ref != blk.ref) {
       // connection that does not map onto the neighbour: flag, do not read
-      if (threadIdx.x == 0) atomicExch(const_cast<int32_t *>(&solves[blk.solve].status), 6);
+      if (threadIdx.x == 0) atomicExch(&solves[blk.solve].status, 6);
       return;
     }
     const float4 *src = reinterpret_cast<const float4 *>(ob.f) + ((size_t)iB * NJB + jB) * (size_t)NP;

@@ -1,23 +1,18 @@
-// ugks_fused.cu -- the whole UGKS time step in five launches, for every block
+// ugks_fused.cu -- the whole UGKS time step in four launches, for every block
 // of every solve of a device-resident block table.
 //
 // Per step (UGKSim.one_step, ugks_sim.py:407-501):
-//   face pass   one CTA per face of either direction: reconstruction (iFace),
+//   face pass   a face per warp, in either direction: reconstruction (iFace),
 //               face moments (getFaceCons/getAL/getAR), slopes (getPLR),
-//               initMacroFlux, calcFaceQ, macroFlux and distFlux fused, or the
-//               wall procedure for wall faces (accommodatingWallDist |
-//               adsorbingWall_P1 + adsorbingWallD_P2, then wallFlux and
-//               wallMassEnergyFluxes).  The per-velocity interface
-//               distribution and slope stay in shared memory between the
-//               three velocity sweeps a face needs (moments -> heat flux ->
-//               flux), so f is read once per face from HBM/L2.
-//   dt check    updateTimeStep inside the dt loop (ugks_sim.py:430-441):
-//               device-side, sets the retry flag of a solve whose dt changed.
-//   face pass   again, only for solves whose retry flag is set.
-//   cell pass   one CTA per cell: calcQ, updateMacro and UGKS_update fused,
-//               plus the cell's CFL frequency (clFindDT) and residual terms.
-//   dt update   calcTimeStep + updateTimeStep + time advance, device-side.
-//   ghost pass  one CTA per ghost cell of every block face (updateBC).
+//               initMacroFlux, calcFaceQ, macroFlux and distFlux fused; wall
+//               faces a CTA each: accommodatingWallDist | adsorbingWall_P1 + P2,
+//               then wallFlux and wallMassEnergyFluxes.
+//   face pass   again, only for solves whose dt changed (updateTimeStep inside
+//               the dt loop, ugks_sim.py:430-441).
+//   cell pass   a cell per warp: calcQ, updateMacro and UGKS_update fused, plus
+//               the cell's CFL frequency (clFindDT).
+//   ghost pass  one CTA per ghost cell of every block face (updateBC), and the
+//               end of the step: calcTimeStep, updateTimeStep, time advance.
 // Nothing reads the host in between, so a step can be captured in a graph.
 #include <cuda_runtime.h>
 #include <float.h>
@@ -78,29 +73,15 @@ constexpr int FLUX_WPC = 4, FLUX_MINB = UGKS_FLUX_MINB;
 #define UGKS_FLUX_TMA_MINB 5
 #endif
 constexpr int FLUX_TMA_MINB = UGKS_FLUX_TMA_MINB;
-// CTAs of 8 cell warps per SM: FP64 at 128 registers (at 80 the update loop
-// spills and the pass is 12% slower), mixed at 80 (3 CTAs: 0.215 against
-// 0.222 ms at 120 registers on the 2x2-block cavity)
-#ifndef CELL_MIN_BLOCKS
-#define CELL_MIN_BLOCKS 2
-#endif
-#ifndef CELL_MIN_BLOCKS_F32
-#define CELL_MIN_BLOCKS_F32 3
-#endif
-// ...and the depth of the per-warp ring of asynchronous copies that stream
-// the f and flux rows of the cell update into shared memory
-// (FP64 only: with 8-byte FP32 elements the ring was 18% slower than plain loads)
-#ifndef CELL_RING_F64
-#define CELL_RING_F64 3
-#endif
-template <typename T> struct CellBudget { static constexpr int minb = CELL_MIN_BLOCKS, ring = CELL_RING_F64; };
-template <> struct CellBudget<float> { static constexpr int minb = CELL_MIN_BLOCKS_F32, ring = 0; };
+// cell pass: CELL_MINB x 8 cell warps per SM by default, 16 at 128 registers (24
+// at 80 spill: FP64 1.06 -> 1.22 ms a step on the 2x2-block cavity, mixed 0.720
+// -> 0.730), and the depth of the per-warp ring of asynchronous copies that
+// stream the f and flux rows of the FP64 update into shared memory (with the
+// 16-byte pairs of the mixed storage the ring was 18% slower than plain loads)
+constexpr int CELL_MINB = 2, CELL_RING_F64 = 3;
 // shared memory of the cell-update ring: per warp, ring stages x 5 rows
 // (f, S face j, S face j+1, W face i, W face i+1) x 32 lanes
-template <typename T>
-constexpr size_t cell_ring_bytes() {
-  return (size_t)CellBudget<T>::ring * 5 * 32 * sizeof(typename Store<T>::vec);
-}
+constexpr size_t cell_ring_bytes() { return (size_t)CELL_RING_F64 * 5 * 32 * sizeof(double2); }
 
 // cp.async (sm_80+ asynchronous global -> shared copy of 8 or 16 bytes per
 // thread; a thread waits only for its own groups)
@@ -173,6 +154,24 @@ __device__ __forceinline__ double limited_dt(double dt_old, double dt_new, doubl
     return dt_new;
   }
   return dt_old;
+}
+
+// The time steps of one fused step (the dt loop of one_step, ugks_sim.py:430-446):
+// the first flux pass runs at `first`; when the limiter changes dt the pass is
+// redone at `flux` and dt is limited once more for the cell update.  A pure
+// function of the solve record, which only finish_step writes, so that every
+// kernel of the step evaluates it for itself.
+struct StepDt {
+  double first, flux, cell;
+  bool retry;
+};
+__device__ __forceinline__ StepDt step_dt(const ugks_solve_state &x) {
+  StepDt t;
+  t.first = x.dt;
+  t.flux = limited_dt(x.dt, x.max_dt, x.delta_dt);
+  t.retry = t.flux != x.dt;
+  t.cell = t.retry ? limited_dt(t.flux, x.max_dt, x.delta_dt) : t.flux;
+  return t;
 }
 
 // ---------------------------------------------------------------------------
@@ -758,7 +757,7 @@ __device__ __forceinline__ bool face_work(const ugks_fused_block *__restrict__ B
   UGKS_CHECK_ITEM(0, blk, w, solves, false);
   const ugks_solve_state &sol = solves[blk.solve];
   if (!sol.active) return false;
-  if (retry_pass && !sol.retry) return false;
+  if (retry_pass && !step_dt(sol).retry) return false;
   if (FM >= 0 && d.flux_method != FM) return false;  // FM < 0: any flux method
   int lf = w - blk.face_begin;
   if (STRIPS) {
@@ -978,7 +977,7 @@ __device__ __noinline__ double plain_exp(double x) { return exp(x); }
 // and macroFlux's (587-681) discrete part sums (Zh, x Zh, y Zh, (|u|^2 Zh + Zb) / 2)
 // in the global frame.
 template <int FM>
-__device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, const ugks_solve_state &sol, double *rec,
+__device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, const double dt, double *rec,
                                                double2 *ring, const FaceWork &fwk) {
   const ugks_block_desc &d = blk.d;
   const int lane = threadIdx.x & 31, Nv = d.Nv, un = d.u_num, vn = d.v_num;
@@ -1035,7 +1034,7 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, cons
   };
 #pragma unroll
   for (int s = 0; s < D2; ++s) issue(lane + 32 * s, s);  // under the coefficients
-  face_coefficients(blk, sol.dt, fwk, rec);
+  face_coefficients(blk, dt, fwk, rec);
   __syncwarp();
   const bool sep = un > 0 && un * vn == Nv && un + vn <= 512;
   double *Eu = rec + FACE_TAB, *Ev = Eu + un;
@@ -1112,8 +1111,8 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, cons
 // on in place (each thread reads back only what it wrote); the reflected
 // incoming distribution it gathers from is read where P1 put it, wall_dist.
 template <int FM, int NT>
-__device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_solve_state &sol, FaceShared<NT> &sh,
-                                            const FaceWork fwk) {
+__device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_solve_state &sol, const double dt,
+                                            FaceShared<NT> &sh, const FaceWork fwk) {
   const ugks_block_desc &d = blk.d;
   const int dir = fwk.dir, Nv = d.Nv;
   const long gi = fwk.gi, gj = fwk.gj;
@@ -1139,7 +1138,7 @@ __device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_so
   const long ci = dir == SOUTH ? fwk.mi : fwk.mj;
   wall_face<NT>(blk, sol, sh, reinterpret_cast<double *>(row),
                 reinterpret_cast<double2 *>(blk.wall_dist) + (size_t)ci * Nv, fwk.wall, dir, gi, gj, fwk.mi, fwk.mj, n,
-                blk.side_length[fk], sol.dt, [&](int v, double hx, double hy) { row[v] = make_double2(hx, hy); });
+                blk.side_length[fk], dt, [&](int v, double hx, double hy) { row[v] = make_double2(hx, hy); });
 }
 
 // wall work item (2 (ni + nj) per block: the S faces of rows 0 and nj, then
@@ -1170,10 +1169,11 @@ __device__ __forceinline__ void wall_work_fp64(const ugks_fused_block *__restric
   FaceWork fwk;
   if (!face_work<-1>(B, nb, solves, wall_to_face(blk, w), retry_pass, fwk) || fwk.wall < 0) return;
   ugks_solve_state &sol = solves[blk.solve];
+  const double dt = retry_pass ? step_dt(sol).flux : sol.dt;
   switch (blk.d.flux_method) {
-    case 0: wall_item_fp64<0, NT>(blk, sol, sh, fwk); break;
-    case 1: wall_item_fp64<1, NT>(blk, sol, sh, fwk); break;
-    case 3: wall_item_fp64<3, NT>(blk, sol, sh, fwk); break;
+    case 0: wall_item_fp64<0, NT>(blk, sol, dt, sh, fwk); break;
+    case 1: wall_item_fp64<1, NT>(blk, sol, dt, sh, fwk); break;
+    case 3: wall_item_fp64<3, NT>(blk, sol, dt, sh, fwk); break;
     default: break;
   }
 }
@@ -1199,7 +1199,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_pass_fp64(const ugks_fuse
   FaceWork fwk;
   if (!face_work<FM, true>(B, nb, solves, first + item, 0, fwk) || fwk.wall >= 0) return;
   const ugks_fused_block &blk = B[fwk.bi];
-  face_item_fp64<FM>(blk, solves[blk.solve], dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
+  face_item_fp64<FM>(blk, solves[blk.solve].dt, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
 }
 
 // the mixed path's face work item (ugks_delta.cuh, included further down):
@@ -1219,7 +1219,7 @@ __device__ __forceinline__ bool retry_solve(const ugks_fused_block *__restrict__
   const int s = blockIdx.x / RETRY_CTAS;
   if (s >= ns) return false;
   const ugks_solve_state &x = solves[s];
-  if (!x.active || !x.retry || x.nblocks <= 0) return false;
+  if (!x.active || x.nblocks <= 0 || !step_dt(x).retry) return false;
   b0 = x.first_block;
   bl = x.first_block + x.nblocks - 1;
   return B[b0].d.flux_method == FM;
@@ -1243,7 +1243,8 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_retry_fp64(const ugks_fus
     FaceWork fwk;
     if (!face_work<FM>(B, nb, solves, w, 1, fwk) || fwk.wall >= 0) continue;
     const ugks_fused_block &blk = B[fwk.bi];
-    face_item_fp64<FM>(blk, solves[blk.solve], dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
+    face_item_fp64<FM>(blk, step_dt(solves[blk.solve]).flux, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp),
+                       fwk);
   }
 }
 // mixed: only the wall faces have anything to redo (the interior faces take the
@@ -1269,12 +1270,19 @@ __device__ __forceinline__ double cfl_freq(const ugks_fused_block &blk, P4 m, lo
   return cfl_frequency(blk.d, blk.xy, blk.area, m, mi, mj, blk.d.Kn_eff);
 }
 
-// one warp per cell, CW cells per CTA: no block-wide barrier, so the serial
-// per-cell coefficients of one cell (lane 0) stall only that cell's warp
-constexpr int CW = 8;
+// One warp per cell, CW cells per CTA.  The serial per-cell part (updateMacro,
+// two relaxation times, the CFL frequency: some 1500 instructions) of the CTA's
+// cells runs on CW lanes of its first warp, one cell each, while the others
+// build the old states' tables and the first rows are on their way; every warp
+// running it for its own cell on one lane cost 2x2-block FP64 0.320 ms against
+// 0.301, a 24x24 cavity 18.4 us against 16.8.  The moments of f^{n+1} are summed
+// in the update loop (a second sweep over f: 0.314 ms).  Bound by memory latency:
+// 1.2 GB at 4 TB/s with 16 warps per SM.
+constexpr int CW = 4;
 // per-warp shared memory: the axis tables of the old and new state
 // (2 (u_num + v_num) doubles) and CELL_COEF coefficient slots
-constexpr int CELL_COEF = 16;
+constexpr int CELL_COEF = 14;
+enum { CC_U, CC_V, CC_LAM, CC_A1, CC_A2, CC_A3, CC_A4, CC_P, CC_KN, CC_SN, CC_LNP };
 
 template <int N>
 __device__ __forceinline__ void warp_sum(double (&x)[N]) {
@@ -1285,130 +1293,162 @@ __device__ __forceinline__ void warp_sum(double (&x)[N]) {
   }
 }
 
-template <typename T, int MINB = CellBudget<T>::minb>
-__global__ void __launch_bounds__(CW * 32, MINB) cell_pass(const ugks_fused_block *__restrict__ B, int nb,
-                                                        ugks_solve_state *__restrict__ solves, int n_cells,
-                                                        int wstride) {
-  extern __shared__ double dyn[];
-  using St = Store<T>;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int w = blockIdx.x * CW + warp;
-  if (w >= n_cells) return;
-  const int bi = find_block<1>(B, nb, w);
-  const ugks_fused_block &blk = B[bi];
-  const ugks_block_desc &d = blk.d;
-  UGKS_CHECK_ITEM(1, blk, w, solves);
-  ugks_solve_state &sol = solves[blk.solve];
-  if (!sol.active) return;
+// a cell warp's cell: false when the warp has none (past the end, or a solve
+// that is switched off)
+struct CellWork {
+  int bi;
+  long mi, mj, gi, gj;
+};
+__device__ __forceinline__ bool cell_work(const ugks_fused_block *__restrict__ B, int nb,
+                                          const ugks_solve_state *__restrict__ solves, int w, int n_cells, CellWork &c) {
+  if (w >= n_cells) return false;
+  c.bi = find_block<1>(B, nb, w);
+  const ugks_fused_block &blk = B[c.bi];
+  UGKS_CHECK_ITEM(1, blk, w, solves, false);
+  if (!solves[blk.solve].active) return false;
   const int lc = w - blk.cell_begin;
-  const long mi = lc / d.nj, mj = lc % d.nj;
-  const long gi = mi + d.ghost, gj = mj + d.ghost;
-  const int Nv = d.Nv, un = d.u_num, vn = d.v_num;
-  const bool sep = un > 0 && un * vn == Nv && un + vn <= 512;
-  double *Eou = dyn + (size_t)warp * wstride, *Eov = Eou + un, *Enu = Eov + vn, *Env = Enu + un;
-  double *bc = dyn + (size_t)warp * wstride + (wstride - CELL_COEF);
-  const size_t base = fidx(d, gi, gj, 0);
-  const size_t sj = (size_t)Nv, si = (size_t)d.Nj * Nv;
-  const double dt = sol.dt;
-  const P4 old = ld4(blk.macro, midx(d, mi, mj));
+  c.mi = lc / blk.d.nj;
+  c.mj = lc % blk.d.nj;
+  c.gi = c.mi + blk.d.ghost;
+  c.gj = c.mj + blk.d.ghost;
+  return true;
+}
+
+// updateMacro, the relaxation weights of UGKS_update and the CFL frequency of
+// one cell (a thread), its coefficients into bc:
+//   a1 = (1 - dt/2 /tau_old) / D, a2 = 1 / (A D), a3 = dt/2 / (tau D),
+//   a4 = dt/2 / (tau_old D), D = 1 + dt/2 / tau  (a1 + a3 + a4 = 1)
+__device__ __forceinline__ double cell_coefficients(const ugks_fused_block &blk, const ugks_solve_state &sol,
+                                                    const CellWork &c, double *bc, double P0pi) {
+  const ugks_block_desc &d = blk.d;
+  const size_t m = midx(d, c.mi, c.mj);
+  const P4 old = ld4(blk.macro, m);
+  const P4 s0 = ld4(blk.flux_macro_S, gidx(d, c.gi, c.gj)), s1 = ld4(blk.flux_macro_S, gidx(d, c.gi, c.gj + 1));
+  const P4 w0 = ld4(blk.flux_macro_W, gidx(d, c.gi, c.gj)), w1 = ld4(blk.flux_macro_W, gidx(d, c.gi + 1, c.gj));
+  const double iA = 1.0 / blk.area[gidx(d, c.gi, c.gj)], dt = step_dt(sol).cell;
   // calcQ of f^n with the macro of f^n: accumulated by the previous cell pass
   // (or the initialisation) in Q_next
-  const V2 Q = ld2(blk.Q_next, midx(d, mi, mj));
-  if (lane == 0) {
-    // updateMacro
-    const P4 wc = to_conserved(d, old);
-    const double iA = 1.0 / blk.area[gidx(d, gi, gj)];
-    const P4 s0 = ld4(blk.flux_macro_S, gidx(d, gi, gj)), s1 = ld4(blk.flux_macro_S, gidx(d, gi, gj + 1));
-    const P4 w0 = ld4(blk.flux_macro_W, gidx(d, gi, gj)), w1 = ld4(blk.flux_macro_W, gidx(d, gi + 1, gj));
-    const P4 nw = p4(wc.s0 + (s0.s0 - s1.s0 + w0.s0 - w1.s0) * iA, wc.s1 + (s0.s1 - s1.s1 + w0.s1 - w1.s1) * iA,
-                     wc.s2 + (s0.s2 - s1.s2 + w0.s2 - w1.s2) * iA, wc.s3 + (s0.s3 - s1.s3 + w0.s3 - w1.s3) * iA);
-    Rcp rn, ro;
-    const P4 prim = to_primary_rcp(d, nw, rn);
-    ro.rho = nr_rcp(old.s0);
-    ro.lam = nr_rcp(old.s3);
-    st4(blk.macro, midx(d, mi, mj), prim);
-    st4(blk.prim_old, midx(d, mi, mj), old);
-    st2(blk.Q, midx(d, mi, mj), Q);
-    // UGKS_update (clUGKS.c:1189-1257) per velocity, regrouped:
-    //   f' = f a1 + (sum of face fluxes) a2 + fEQ(new) a3 + fEQ(old) a4,
-    //   a1 = (1 - dt/2 /tau_old) / D, a2 = 1 / (A D), a3 = dt/2 / (tau D),
-    //   a4 = dt/2 / (tau_old D), D = 1 + dt/2 / tau;
-    // a3 and a4 go into the Maxwellian prefactors rho lambda / pi of fEQ
-    const double itau_old = inv_relax_time_rcp(d, old, ro), itau = inv_relax_time_rcp(d, prim, rn);
-    const double hdt = 0.5 * dt, iden = nr_rcp(1.0 + hdt * itau);
-    const double ipi = nr_rcp(d.PI);
-    bc[0] = prim.s1;
-    bc[1] = prim.s2;
-    bc[2] = prim.s3;
-    bc[3] = (1.0 - hdt * itau_old) * iden;                         // a1
-    bc[4] = iden * iA;                                             // a2
-    bc[5] = prim.s0 * (prim.s3 * ipi) * (hdt * itau * iden);       // new prefactor x a3
-    bc[6] = old.s0 * (old.s3 * ipi) * (hdt * itau_old * iden);     // old prefactor x a4
-    bc[7] = (0.5 * d.K) * rn.lam;                                  // K / (2 lambda) new
-    bc[8] = 0.8 * (1 - d.Pr) * (prim.s3 * prim.s3) * rn.rho;       // Shakhov factor new
-    const double fq = cfl_freq(blk, prim, mi, mj);
-    atomicMax(&sol.max_freq, (unsigned long long)__double_as_longlong(fq));
-  } else if (sep) {
-    axis_exp(Eou, d.quad, un, vn, 0, old.s1, old.s3, lane - 1, 31);
-    axis_exp(Eov, d.quad, vn, 1, 1, old.s2, old.s3, lane - 1, 31);
-  }
-  __syncwarp();
-  const double nU = bc[0], nV = bc[1], nl = bc[2];
-  if (sep) {
-    axis_exp(Enu, d.quad, un, vn, 0, nU, nl, lane, 32);
-    axis_exp(Env, d.quad, vn, 1, 1, nV, nl, lane, 32);
-    __syncwarp();
-  }
-  const double a1 = bc[3], a2 = bc[4], cn = bc[5], co = bc[6], kn = bc[7], sn = bc[8];
-  const double ko = (0.5 * d.K) * nr_rcp(old.s3);
-  const double so = 0.8 * (1 - d.Pr) * (old.s3 * old.s3) * nr_rcp(old.s0);
-  const int qs = sep ? 32 / vn : 0, rs = sep ? 32 % vn : 0;
-  int iu = sep ? lane / vn : 0, jv = sep ? lane % vn : 0;
-  bool nan = false;
-  // FP64: the five rows this lane reads run D velocities (of this lane)
-  // ahead through a ring of cp.async stages; a stage is refilled only after
-  // the store that consumed its values, whose operands are the stage's loads
-  constexpr int D = CellBudget<T>::ring;
-  using E = typename St::vec;
+  st2(blk.Q, m, ld2(blk.Q_next, m));
+  const P4 wc = to_conserved(d, old);
+  const P4 nw = p4(wc.s0 + (s0.s0 - s1.s0 + w0.s0 - w1.s0) * iA, wc.s1 + (s0.s1 - s1.s1 + w0.s1 - w1.s1) * iA,
+                   wc.s2 + (s0.s2 - s1.s2 + w0.s2 - w1.s2) * iA, wc.s3 + (s0.s3 - s1.s3 + w0.s3 - w1.s3) * iA);
+  Rcp rn, ro;
+  const P4 prim = to_primary_rcp(d, nw, rn);
+  ro.rho = nr_rcp(old.s0);
+  ro.lam = nr_rcp(old.s3);
+  st4(blk.macro, m, prim);
+  st4(blk.prim_old, m, old);
+  const double itau_old = inv_relax_time_rcp(d, old, ro), itau = inv_relax_time_rcp(d, prim, rn);
+  const double hdt = 0.5 * dt, iden = nr_rcp(1.0 + hdt * itau);
+  bc[CC_U] = prim.s1;
+  bc[CC_V] = prim.s2;
+  bc[CC_LAM] = prim.s3;
+  bc[CC_A1] = (1.0 - hdt * itau_old) * iden;
+  bc[CC_A2] = iden * iA;
+  bc[CC_A3] = hdt * itau * iden;
+  bc[CC_A4] = hdt * itau_old * iden;
+  bc[CC_P] = prim.s0 * prim.s3;                                  // pi times the prefactor of fM
+  bc[CC_KN] = (0.5 * d.K) * rn.lam;                              // K / (2 lambda)
+  bc[CC_SN] = 0.8 * (1 - d.Pr) * (prim.s3 * prim.s3) * rn.rho;   // Shakhov factor
+  if (P0pi > 0.0) bc[CC_LNP] = log((prim.s0 * prim.s3) / P0pi);  // mixed: ln(P / P0)
+  return cfl_freq(blk, prim, c.mi, c.mj);
+}
+// the same for the CTA's cells, one per lane of its first warp
+template <bool MIXED>
+__device__ __forceinline__ void cta_cell_coefficients(const ugks_fused_block *__restrict__ B, int nb,
+                                                      ugks_solve_state *__restrict__ solves, int n_cells, double *dyn,
+                                                      int wstride) {
+  if (threadIdx.x >= CW) return;
+  CellWork c;
+  if (!cell_work(B, nb, solves, (int)blockIdx.x * CW + (int)threadIdx.x, n_cells, c)) return;
+  const ugks_fused_block &blk = B[c.bi];
+  const double P0pi = MIXED ? blk.ref[UGKS_REF_P0] * blk.d.PI : 0.0;
+  const double fq = cell_coefficients(blk, solves[blk.solve], c,
+                                      dyn + (size_t)threadIdx.x * wstride + (wstride - CELL_COEF), P0pi);
+  atomicMax(&solves[blk.solve].max_freq, (unsigned long long)__double_as_longlong(fq));
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_fp64(const ugks_fused_block *__restrict__ B, int nb,
+                                                                ugks_solve_state *__restrict__ solves, int n_cells,
+                                                                int wstride) {
+  extern __shared__ double dyn[];
+  using St = Store<double>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  CellWork cw;
+  const bool on = cell_work(B, nb, solves, (int)blockIdx.x * CW + warp, n_cells, cw);
+  const ugks_fused_block &blk = B[on ? cw.bi : 0];
+  const ugks_block_desc &d = blk.d;
+  const int Nv = on ? d.Nv : 0, un = d.u_num, vn = d.v_num;
+  const bool sep = un > 0 && un * vn == d.Nv && un + vn <= 512;
+  double *Eou = dyn + (size_t)warp * wstride, *Eov = Eou + un, *Enu = Eov + vn, *Env = Enu + un;
+  const double *bc = dyn + (size_t)warp * wstride + (wstride - CELL_COEF);
+  const size_t base = on ? fidx(d, cw.gi, cw.gj, 0) : 0;
+  const size_t sj = (size_t)d.Nv, si = (size_t)d.Nj * d.Nv, m = on ? midx(d, cw.mi, cw.mj) : 0;
+  // the five rows this lane reads run D velocities (of this lane) ahead
+  // through a ring of cp.async stages; a stage is refilled only after the
+  // store that consumed its values, whose operands are the stage's loads
+  constexpr int D = CELL_RING_F64;
+  using E = double2;
   E *ring = reinterpret_cast<E *>(dyn + (size_t)CW * wstride) + (size_t)warp * (D * 5 * 32) + lane;
   const E *gf = reinterpret_cast<const E *>(blk.f), *gS = reinterpret_cast<const E *>(blk.flux_S),
           *gW = reinterpret_cast<const E *>(blk.flux_W);
   auto issue = [&](int vv, int stage) {
-    if (D == 0) return;
     if (vv < Nv) {
       const size_t k = base + vv;
       E *r = ring + stage * (5 * 32);
-      cp_async<sizeof(E)>(r, gf + k);
-      cp_async<sizeof(E)>(r + 32, gS + k);
-      cp_async<sizeof(E)>(r + 64, gS + k + sj);
-      cp_async<sizeof(E)>(r + 96, gW + k);
-      cp_async<sizeof(E)>(r + 128, gW + k + si);
+      cp_async<16>(r, gf + k);
+      cp_async<16>(r + 32, gS + k);
+      cp_async<16>(r + 64, gS + k + sj);
+      cp_async<16>(r + 96, gW + k);
+      cp_async<16>(r + 128, gW + k + si);
     }
     cp_async_commit();
   };
 #pragma unroll
   for (int s = 0; s < D; ++s) issue(lane + 32 * s, s);
+  P4 old = p4(1.0, 0.0, 0.0, 1.0);
+  V2 Q = v2(0.0, 0.0);
+  if (on) {
+    old = ld4(blk.macro, m);
+    Q = ld2(blk.Q_next, m);
+  }
+  __syncthreads();  // every warp has its cell's old state before it is updated
+  cta_cell_coefficients<false>(B, nb, solves, n_cells, dyn, wstride);
+  __syncwarp();
+  if (on && sep) {
+    axis_exp(Eou, d.quad, un, vn, 0, old.s1, old.s3, lane, 32);
+    axis_exp(Eov, d.quad, vn, 1, 1, old.s2, old.s3, lane, 32);
+  }
+  __syncthreads();
+  if (!on) return;
+  const double nU = bc[CC_U], nV = bc[CC_V], nl = bc[CC_LAM], ipi = nr_rcp(d.PI);
+  const double a1 = bc[CC_A1], a2 = bc[CC_A2], kn = bc[CC_KN], sn = bc[CC_SN];
+  const double cn = bc[CC_P] * ipi * bc[CC_A3], co = old.s0 * (old.s3 * ipi) * bc[CC_A4];
+  if (sep) {
+    axis_exp(Enu, d.quad, un, vn, 0, nU, nl, lane, 32);
+    axis_exp(Env, d.quad, vn, 1, 1, nV, nl, lane, 32);
+    __syncwarp();
+  }
+  const double ko = (0.5 * d.K) * nr_rcp(old.s3);
+  const double so = 0.8 * (1 - d.Pr) * (old.s3 * old.s3) * nr_rcp(old.s0);
+  const int qs = sep ? 32 / vn : 0, rs = sep ? 32 % vn : 0;
+  int iu = sep ? lane / vn : 0, jv = sep ? lane % vn : 0;
+  bool nan = false;
   int stage = 0;
+  const double Kinv = nr_rcp(d.K);
+  // moments of f^{n+1} for the next face pass, and calcQ (clKernel.c:480-543)
+  // of f^{n+1} with the new macro for the next cell pass
+  double mom[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  // UGKS_update (clUGKS.c:1189-1257) per velocity, regrouped:
+  //   f' = f a1 + (sum of face fluxes) a2 + fEQ(new) a3 + fEQ(old) a4,
+  // a3 and a4 in the Maxwellian prefactors rho lambda / pi of fEQ
 #pragma unroll 1
   for (int v = lane; v < Nv; v += 32) {
     const size_t k = base + v;
-    V2 f, s0, s1, w0, w1;
-    if constexpr (D > 0) {
-      cp_async_wait<D - 1>();
-      const E *r = ring + stage * (5 * 32);
-      const E fe = r[0], s0e = r[32], s1e = r[64], w0e = r[96], w1e = r[128];
-      f = v2(fe.x, fe.y);
-      s0 = v2(s0e.x, s0e.y);
-      s1 = v2(s1e.x, s1e.y);
-      w0 = v2(w0e.x, w0e.y);
-      w1 = v2(w1e.x, w1e.y);
-    } else {
-      f = St::load(blk.f, k);
-      s0 = St::load(blk.flux_S, k);
-      s1 = St::load(blk.flux_S, k + sj);
-      w0 = St::load(blk.flux_W, k);
-      w1 = St::load(blk.flux_W, k + si);
-    }
+    cp_async_wait<D - 1>();
+    const E *r = ring + stage * (5 * 32);
+    const E f = r[0], s0 = r[32], s1 = r[64], w0 = r[96], w1 = r[128];
     const V2 e = quad_at(d, v);
     const double wv = d.weight[v];
     const double ox = e.x - old.s1, oy = e.y - old.s2, o2 = fma(ox, ox, oy * oy);
@@ -1421,8 +1461,8 @@ __global__ void __launch_bounds__(CW * 32, MINB) cell_pass(const ugks_fused_bloc
       iu += qs;
       if (jv >= vn) { jv -= vn; ++iu; }
     } else {
-      Eo = exp(-old.s3 * o2);
-      En = exp(-nl * n2);
+      Eo = plain_exp(-old.s3 * o2);
+      En = plain_exp(-nl * n2);
     }
     // fEQ (clFunctions.c:79-86) at the old and the new macro state, scaled
     const double ho = wv * co * Eo, hn = wv * cn * En;
@@ -1434,37 +1474,49 @@ __global__ void __launch_bounds__(CW * 32, MINB) cell_pass(const ugks_fused_bloc
     const V2 out = v2(fma(f.x, a1, fma(flh, a2, eh)), fma(f.y, a1, fma(flb, a2, eb)));
     nan |= isnan(out.x) || isnan(out.y);
     St::store(blk.f, k, out);
-    if constexpr (D > 0) {
-      issue(v + 32 * D, stage);
-      stage = stage + 1 == D ? 0 : stage + 1;
-    }
-  }
-  if constexpr (D > 0) cp_async_wait<0>();
-  if (nan) atomicExch(&sol.status, 1);
-  // moments of f^{n+1} for the next face pass, and calcQ (clKernel.c:480-543)
-  // of f^{n+1} with the new macro for the next cell pass: a second sweep over
-  // the values this lane just stored (L2-resident), which keeps the update
-  // loop's registers free
-  const double Kinv = nr_rcp(d.K);
-  double mom[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int v = lane; v < Nv; v += 32) {
-    const V2 o = St::load(blk.f, base + v);
-    const V2 e = quad_at(d, v);
-    const double nx = e.x - nU, ny = e.y - nV, n2 = fma(nx, nx, ny * ny);
-    mom[0] += o.x;
-    mom[1] = fma(e.x, o.x, mom[1]);
-    mom[2] = fma(e.y, o.x, mom[2]);
-    mom[3] += fma(fma(e.x, e.x, e.y * e.y), o.x, o.y);
-    const double t = fma(n2, o.x, o.y * Kinv);
+    issue(v + 32 * D, stage);
+    stage = stage + 1 == D ? 0 : stage + 1;
+    mom[0] += out.x;
+    mom[1] = fma(e.x, out.x, mom[1]);
+    mom[2] = fma(e.y, out.x, mom[2]);
+    mom[3] += fma(fma(e.x, e.x, e.y * e.y), out.x, out.y);
+    const double t = fma(n2, out.x, out.y * Kinv);
     mom[4] = fma(nx, t, mom[4]);
     mom[5] = fma(ny, t, mom[5]);
   }
-  warp_sum<6>(mom);
-  if (lane == 0) {
-    st4(blk.cell_mom, gidx(d, gi, gj), p4(mom[0], mom[1], mom[2], 0.5 * mom[3]));
-    st2(blk.Q_next, midx(d, mi, mj), v2(0.5 * mom[4], 0.5 * mom[5]));
+  cp_async_wait<0>();
+  if (nan) atomicExch(&solves[blk.solve].status, 1);
+  const double t = warp_spread_sum<6>(mom);
+  constexpr int S = spread_shift<6>();
+  if ((lane & ((1 << S) - 1)) == 0 && (lane >> S) < 6) {
+    const int k = lane >> S;
+    if (k < 4) blk.cell_mom[4 * gidx(d, cw.gi, cw.gj) + k] = k == 3 ? 0.5 * t : t;
+    else blk.Q_next[2 * m + (k - 4)] = 0.5 * t;
   }
 }
+
+// ---------------------------------------------------------------------------
+// dt control (ugks_sim.py:285-311, 430-446, 458-460, 491): after the cell pass
+// the dt of the step, calcTimeStep + updateTimeStep, time += dt
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void finish_step(ugks_solve_state &x) {
+  if (!x.active) return;
+  const StepDt t = step_dt(x);
+  if (t.retry) x.retries += 1;
+  const double fq = __longlong_as_double((long long)x.max_freq);
+  x.max_dt = x.CFL / fq;
+  x.dt = limited_dt(t.cell, x.max_dt, x.delta_dt);
+  x.time += x.dt;
+  x.steps += 1;
+  x.max_freq = 0ull;
+  x.retry = 0;
+}
+// every solve, by the threads of a whole launch (the ghost pass, which needs
+// none of what this writes)
+__device__ __forceinline__ void finish_steps(ugks_solve_state *solves, int ns) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) finish_step(solves[s]);
+}
+__global__ void dt_update(ugks_solve_state *solves, int ns) { finish_steps(solves, ns); }
 
 // ---------------------------------------------------------------------------
 // ghost pass (UGKSBlock.updateBC, ugks_block.py:621-665): one CTA per ghost
@@ -1472,8 +1524,9 @@ __global__ void __launch_bounds__(CW * 32, MINB) cell_pass(const ugks_fused_bloc
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(FT) ghost_pass(const ugks_fused_block *__restrict__ B, int nb,
-                                                 const ugks_solve_state *__restrict__ solves) {
+                                                 ugks_solve_state *solves, int finish) {
   __shared__ double scratch[4 * (FT / 32)];
+  finish_steps(solves, finish);
   using St = Store<T>;
   const int w = blockIdx.x;
   const int bi = find_block<2>(B, nb, w);
@@ -1554,7 +1607,7 @@ __global__ void __launch_bounds__(FT) ghost_pass(const ugks_fused_block *__restr
     swap_cell_index(NI, NJ, G, face, iB, jB, that, NIB, NJB);
     if (iB < 0 || iB >= NIB || jB < 0 || jB >= NJB || ob.d.Nv != Nv) {
       // connection that does not map onto the neighbour: flag, do not read
-      if (threadIdx.x == 0) atomicExch(const_cast<int32_t *>(&solves[blk.solve].status), 6);
+      if (threadIdx.x == 0) atomicExch(&solves[blk.solve].status, 6);
       return;
     }
     const size_t src = ((size_t)iB * NJB + jB) * (size_t)Nv;
@@ -1631,40 +1684,6 @@ __global__ void __launch_bounds__(FT) ghost_pass(const ugks_fused_block *__restr
   }
   block_sum<4>(mom, scratch);
   if (threadIdx.x == 0) st4(blk.cell_mom, gidx(d, gi, gj), p4(mom[0], mom[1], mom[2], 0.5 * mom[3]));
-}
-
-// ---------------------------------------------------------------------------
-// dt control (ugks_sim.py:285-311, 430-446, 458-460, 491)
-// ---------------------------------------------------------------------------
-// after a flux pass: updateTimeStep inside the dt loop; phase 0 sets retry
-__global__ void dt_check(ugks_solve_state *solves, int ns, int phase) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns) return;
-  ugks_solve_state &x = solves[s];
-  if (!x.active) return;
-  if (phase == 0) {
-    const double dt = limited_dt(x.dt, x.max_dt, x.delta_dt);
-    x.retry = dt != x.dt;
-    x.dt = dt;
-  } else if (x.retry) {
-    x.dt = limited_dt(x.dt, x.max_dt, x.delta_dt);
-    x.retries += 1;
-  }
-}
-
-// after the cell pass: calcTimeStep + updateTimeStep, time += dt, residual
-__global__ void dt_update(ugks_solve_state *solves, int ns) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns) return;
-  ugks_solve_state &x = solves[s];
-  if (!x.active) return;
-  const double fq = __longlong_as_double((long long)x.max_freq);
-  x.max_dt = x.CFL / fq;
-  x.dt = limited_dt(x.dt, x.max_dt, x.delta_dt);
-  x.time += x.dt;
-  x.steps += 1;
-  x.max_freq = 0ull;
-  x.retry = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1797,13 +1816,17 @@ __global__ void dt_init(ugks_solve_state *solves, int ns) {
 // the mixed-precision (FP32 deviation) kernels
 #include "ugks_delta.cuh"
 
-// the ghost update of every block of the table
+// the ghost update of every block of the table, and with finish = the number of
+// solves the end of their step
 template <typename T>
 void launch_ghosts(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves,
-                   cudaStream_t st) {
-  if (!z->n_ghost) return;
-  if (std::is_same<T, float>::value) ghost_pass_delta<<<z->n_ghost, FT, 0, st>>>(B, nb, solves);
-  else ghost_pass<double><<<z->n_ghost, FT, 0, st>>>(B, nb, solves);
+                   int finish, cudaStream_t st) {
+  if (!z->n_ghost) {
+    if (finish) dt_update<<<(finish + 127) / 128, 128, 0, st>>>(solves, finish);
+    return;
+  }
+  if (std::is_same<T, float>::value) ghost_pass_delta<<<z->n_ghost, FT, 0, st>>>(B, nb, solves, finish);
+  else ghost_pass<double><<<z->n_ghost, FT, 0, st>>>(B, nb, solves, finish);
 }
 
 template <typename T>
@@ -1817,7 +1840,7 @@ int init_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     else init_cells<double><<<z->n_cells, FT, 0, st>>>(B, nb, solves);
   }
   dt_init<<<(ns + 127) / 128, 128, 0, st>>>(solves, ns);
-  launch_ghosts<T>(B, nb, z, solves, st);
+  launch_ghosts<T>(B, nb, z, solves, 0, st);
   return launch_status();
 }
 
@@ -1832,7 +1855,7 @@ int restart_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, u
     else restart_cells<double><<<z->n_cells, FT, 0, st>>>(B, nb, solves);
   }
   dt_init<<<(ns + 127) / 128, 128, 0, st>>>(solves, ns);
-  launch_ghosts<T>(B, nb, z, solves, st);
+  launch_ghosts<T>(B, nb, z, solves, 0, st);
   return launch_status();
 }
 
@@ -1889,7 +1912,7 @@ template <typename T, int MINB>
 cudaError_t set_cell_attributes() {
   if (std::is_same<T, float>::value)
     return cudaFuncSetAttribute(cell_pass_delta<MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  return cudaFuncSetAttribute(cell_pass<double, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  return cudaFuncSetAttribute(cell_pass_fp64<MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 // Kernel attributes (the dynamic shared memory above 48 KB that the face and
@@ -2050,11 +2073,10 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   constexpr bool mixed = std::is_same<T, float>::value;
   // doubles of shared memory per cell warp
   const int cstride = mixed ? delta_cell_stride(z->max_axes) : 2 * z->max_axes + CELL_COEF;
-  const size_t csmem = (size_t)CW * cstride * sizeof(double) + (mixed ? 0 : (size_t)CW * cell_ring_bytes<T>());
+  const size_t csmem = (size_t)CW * cstride * sizeof(double) + (mixed ? 0 : (size_t)CW * cell_ring_bytes());
   const cudaError_t attr = set_step_attributes<T>();
   if (attr != cudaSuccess) return -(int)attr;
   if (face_limit_bytes<T>(z->max_nv, z->max_axes) > 200 * 1024 || csmem > 200 * 1024) return -(int)cudaErrorInvalidValue;
-  const unsigned sg = (unsigned)((ns + 127) / 128);
   auto mark = [&](int k) {
     if (events && events[k]) cudaEventRecord(reinterpret_cast<cudaEvent_t>(events[k]), st);
   };
@@ -2094,11 +2116,12 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     cudaStreamWaitEvent(st, ws->join, 0);
     ws_guard.unlock();
   }
-  // mixed: the interior faces' coefficient and flux launches follow the first
-  // dt check (they use its dt), and the events bracket all of the face pass
-  if (!mixed) mark(1);
-  dt_check<<<sg, 128, 0, st>>>(solves, ns, 0);
-  if (!mixed) mark(2);
+  // mixed: the interior faces' coefficient and flux launches take the dt of the
+  // final flux pass, and the events bracket all of the face pass
+  if (!mixed) {
+    mark(1);
+    mark(2);
+  }
   launch_retry<T>(B, nb, z, solves, ns, st);
   if (mixed && z->n_faces) {
     face_coef_delta<<<(unsigned)((z->n_faces + 127) / 128), 128, 0, st>>>(B, nb, solves, z->n_faces);
@@ -2118,27 +2141,25 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   }
   mark(3);
   phase.reset();
-  dt_check<<<sg, 128, 0, st>>>(solves, ns, 1);
   mark(4);
   phase.emplace("ugks cell pass");
   if (z->n_cells) {
-    // cell_variant: 0 the default register budget, 2 or 3 CTAs of 8 warps per SM
+    // cell_variant: 0 the default register budget, 2 or 3 times 8 warps per SM
     const unsigned cg = (unsigned)((z->n_cells + CW - 1) / CW);
-    const int cv = z->cell_variant == 2 || z->cell_variant == 3 ? z->cell_variant : CellBudget<T>::minb;
+    const int cv = z->cell_variant == 2 || z->cell_variant == 3 ? z->cell_variant : CELL_MINB;
     if (mixed) {
       if (cv == 3) cell_pass_delta<3><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
       else cell_pass_delta<2><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
     } else {
-      if (cv == 3) cell_pass<double, 3><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
-      else cell_pass<double, 2><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
+      if (cv == 3) cell_pass_fp64<3><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
+      else cell_pass_fp64<2><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
     }
   }
   mark(5);
   phase.reset();
-  dt_update<<<sg, 128, 0, st>>>(solves, ns);
   mark(6);
   phase.emplace("ugks ghost pass");
-  launch_ghosts<T>(B, nb, z, solves, st);
+  launch_ghosts<T>(B, nb, z, solves, ns, st);
   mark(7);
   return launch_status();
 }
@@ -2242,10 +2263,8 @@ int ugks_step_launches(const ugks_fused_sizes *z, int mixed) {
   if (mixed && z->n_wall) n += 1;   // and its wall launch
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) n += z->seg_count[k] > 0 ? 1 : 0;
   for (int m = 0; m < 4; ++m) n += z->face_count[m] > 0 ? 1 : 0;  // retry passes
-  n += 2;                                                          // dt checks
   n += z->n_cells ? 1 : 0;
-  n += 1;                                                          // dt update
-  n += z->n_ghost ? 1 : 0;
+  n += 1;                                                          // ghost pass (or the dt update alone)
   return n;
 }
 

@@ -5,7 +5,7 @@ more solves (a solve = one pyUGKS simulation, possibly multi-block) and
 advances them with the fused entry points of libugks_b200.so:
 
 * ``ugks_step_fp64`` / ``ugks_step_mixed``: one ``UGKSim.one_step`` of every
-  active solve in five kernel launches plus two tiny dt launches, with dt
+  active solve in four kernel launches (mixed: eight), with dt
   control, the reference's single flux retry, and the ghost update done on
   the device (no host synchronisation inside a step);
 * ``ugks_residual``: the reference residual on demand.
@@ -320,9 +320,8 @@ class FusedSolver:
     def launches_per_step(self) -> int:
         """Kernel launches of one ugks_step_* call (ugks_step_launches): one
         face pass per (limiter, Nv) segment, one retry pass per limiter
-        present, two dt checks, the cell pass, the dt update and the ghost
-        pass; mixed precision adds the face pass's coefficient and flux
-        launches."""
+        present, the cell pass and the ghost pass; mixed precision adds the
+        face pass's wall, coefficient and flux launches."""
         return self.lib.ugks_step_launches(C.byref(self.sizes), 0 if self.precision == "fp64" else 1)
 
     def step(self, n: int = 1):
