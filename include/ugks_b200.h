@@ -325,9 +325,8 @@ typedef struct ugks_fused_block {
   const double *ref;           /* *_mixed only: the solve's reference Maxwellian
                                   (UGKS_REF_* layout above), the same array for
                                   every block of the solve; unused by *_fp64 */
-  void *aux_S;                 /* *_mixed only: scratch of the face pass, shaped like
-                                  flux_S: the slopes of the SOUTH-face deviations */
-  void *aux_W;                 /* *_mixed only: the same for the WEST faces */
+  void *aux_S;                 /* unused (earlier versions: slopes of the mixed face  */
+  void *aux_W;                 /* pass); may be NULL                                  */
   double *face_rec;            /* *_mixed only: [Ni][Nj][2] x UGKS_FACE_REC scratch */
 } ugks_fused_block;
 

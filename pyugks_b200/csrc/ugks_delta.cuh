@@ -112,26 +112,23 @@ __device__ __forceinline__ float2 rel_excess(float2 a, float2 b) { return fma2(a
 // ---------------------------------------------------------------------------
 // WENO5 (clFunctions.c:266-313) in the difference form of weno5_part with the
 // smoothness terms normalised by their sum (the FP32 range), two velocities
-// at once; returns the slope times dx as num / den
+// at once; returns six times the slope times dx as num / den
 __device__ __forceinline__ void weno5_pair(const float2 (&S)[5], float2 &num, float2 &den) {
   const float2 D0 = sub2(S[1], S[0]), D1 = sub2(S[2], S[1]), D2 = sub2(S[3], S[2]), D3 = sub2(S[4], S[3]);
   const float2 p0 = sub2(D1, D0), p1 = sub2(D2, D1), p2 = sub2(D3, D2);
-  // r0 = 3 D1 - D0 = p0 + 2 D1, r1 = D1 + D2, r2 = D3 - 3 D2 = p2 - 2 D2
   const float2 r0 = fma2(D1, bc2(2.0f), p0), r1 = add2(D1, D2), r2 = fma2(D2, bc2(-2.0f), p2);
-  const float2 eps = bc2(12e-16f), c13 = bc2(13.0f), c3 = bc2(3.0f);
-  float2 e0 = fma2(mul2(c13, p0), p0, fma2(mul2(c3, r0), r0, eps));
-  float2 e1 = fma2(mul2(c13, p1), p1, fma2(mul2(c3, r1), r1, eps));
-  float2 e2 = fma2(mul2(c13, p2), p2, fma2(mul2(c3, r2), r2, eps));
+  const float2 eps = bc2(4e-16f), c = bc2(13.0f / 3.0f);
+  float2 e0 = fma2(mul2(c, p0), p0, fma2(r0, r0, eps));
+  float2 e1 = fma2(mul2(c, p1), p1, fma2(r1, r1, eps));
+  float2 e2 = fma2(mul2(c, p2), p2, fma2(r2, r2, eps));
   const float2 sc = rcp2(add2(add2(e0, e1), e2));
   e0 = mul2(e0, sc);
   e1 = mul2(e1, sc);
   e2 = mul2(e2, sc);
   const float2 q0 = mul2(e0, e0), q1 = mul2(e1, e1), q2 = mul2(e2, e2);
-  const float2 a0 = mul2(q1, q2), a1 = mul2(mul2(bc2(6.0f), q0), q2), a2 = mul2(mul2(c3, q0), q1);
-  const float2 f0 = fma2(bc2(-1.0f / 3.0f), D0, mul2(bc2(5.0f / 6.0f), D1));
-  const float2 f1 = fma2(bc2(1.0f / 6.0f), D1, mul2(bc2(1.0f / 3.0f), D2));
-  const float2 f2 = fma2(bc2(2.0f / 3.0f), D2, mul2(bc2(-1.0f / 6.0f), D3));
-  num = fma2(a0, f0, fma2(a1, f1, mul2(a2, f2)));
+  const float2 t0 = mul2(q0, bc2(3.0f));
+  const float2 a0 = mul2(q1, q2), a1 = mul2(add2(t0, t0), q2), a2 = mul2(t0, q1);  // 1 : 6 : 3
+  num = fma2(a0, fma2(r0, bc2(2.0f), make_float2(-D1.x, -D1.y)), fma2(a1, add2(r1, D2), mul2(a2, sub2(D2, r2))));
   den = add2(add2(a0, a1), a2);
 }
 
@@ -142,7 +139,7 @@ __device__ __forceinline__ float2 slope_pair(const float2 (&S)[FM == 1 ? 5 : 3],
   if constexpr (FM == 1) {
     float2 nm, dn;
     weno5_pair(S, nm, dn);
-    return mul2(mul2(nm, rcp2(dn)), ids);
+    return mul2(mul2(nm, rcp2(dn)), mul2(ids, bc2(1.0f / 6.0f)));
   } else if constexpr (FM == 0) {
     // vanLeer (clFunctions.c:255-261) on (S1 - S0) / l and (S2 - S1) / l
     const float2 s1 = mul2(sub2(S[1], S[0]), il), s2 = mul2(sub2(S[2], S[1]), il);
@@ -165,11 +162,11 @@ __device__ __forceinline__ float2 slope_pair(const float2 (&S)[FM == 1 ? 5 : 3],
 // two lanes of every face CTA while the rest of the CTA waits.  Here it runs
 // one face per thread, between two sweeps that take one face per warp:
 //   1. face_moments_warp: the reconstruction of every velocity pair, stored
-//      as the face deviation in the face's flux row and the slopes in its aux
-//      row, and the 13 raw moments of the deviation into the face record;
+//      as the face deviation in the face's flux row, and nine raw moments of
+//      the deviation into the face record;
 //   2. face_coef_delta (a thread per face): the face state and every per-face
 //      coefficient of the flux into the face record;
-//   3. face_flux_warp: the deviation flux of every velocity pair over the
+//   3. face_flux_tma: the deviation flux of every velocity pair over the
 //      stored face deviations, written over them, and the macro flux.
 // Wall faces run their whole procedure in a launch of their own
 // (wall_pass_delta, a CTA per face).  Interior faces take the dt after the
@@ -178,7 +175,7 @@ __device__ __forceinline__ float2 slope_pair(const float2 (&S)[FM == 1 ? 5 : 3],
 // two passes, for the side effects of adsorbing walls.
 
 // layout of a face record (ugks_fused_block.face_rec, UGKS_FACE_REC doubles
-// per face): [0, 13) the raw moments of the face deviation (face frame);
+// per face): [0, 9) the raw moments of the face deviation (global frame);
 // [16, 38) the coefficients of face_coefficients (c[0..21]); then
 constexpr int FR_MOM = 0, FR_C = 16, FR_UX = 38, FR_UY = 39, FR_LAM = 40, FR_KB = 41, FR_SX = 42, FR_SY = 43,
               FR_LNP = 44, FR_UGX = 45, FR_UGY = 46;
@@ -272,27 +269,6 @@ __global__ void __launch_bounds__(NT) wall_pass_delta(const ugks_fused_block *__
 }
 constexpr int WALL_NT = 128;
 
-// raw moments up to third order (RM* / RB*) of a distribution, from the
-// global frame (x, y) into a face frame u = nx x + ny y, t = nx y - ny x: the
-// moment tensors rotate as the velocities do
-__device__ __forceinline__ void rotate_moments(double (&m)[RNMOM], V2 n) {
-  const double a = n.x, c = n.y, aa = a * a, cc = c * c, ac = a * c;
-  const double m10 = m[RM10], m01 = m[RM01], m20 = m[RM20], m11 = m[RM11], m02 = m[RM02];
-  const double m30 = m[RM30], m21 = m[RM21], m12 = m[RM12], m03 = m[RM03], b10 = m[RB10], b01 = m[RB01];
-  m[RM10] = a * m10 + c * m01;
-  m[RM01] = a * m01 - c * m10;
-  m[RM20] = aa * m20 + 2.0 * ac * m11 + cc * m02;
-  m[RM11] = ac * (m02 - m20) + (aa - cc) * m11;
-  m[RM02] = cc * m20 - 2.0 * ac * m11 + aa * m02;
-  // u^3, u^2 t, u t^2, t^3 expanded in x^3, x^2 y, x y^2, y^3
-  m[RM30] = a * aa * m30 + 3.0 * aa * c * m21 + 3.0 * a * cc * m12 + c * cc * m03;
-  m[RM21] = -aa * c * m30 + a * (aa - 2.0 * cc) * m21 + c * (2.0 * aa - cc) * m12 + a * cc * m03;
-  m[RM12] = a * cc * m30 + c * (cc - 2.0 * aa) * m21 + a * (aa - 2.0 * cc) * m12 + aa * c * m03;
-  m[RM03] = -c * cc * m30 + 3.0 * a * cc * m21 - 3.0 * aa * c * m12 + a * aa * m03;
-  m[RB10] = a * b10 + c * b01;
-  m[RB01] = a * b01 - c * b10;
-}
-
 // 2. coefficients: the per-face block of face_coefficients, one face per
 // thread (the same chain as the lanes of a face CTA run there)
 __global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *__restrict__ B, int nb,
@@ -311,25 +287,22 @@ __global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *_
   double *rec = blk.face_rec + (size_t)UGKS_FACE_REC * fk;
   const V2 n = ld2(blk.normal, fk), mid = ld2(blk.mid_side, fk);
   const double len = blk.side_length[fk];
-  double dm[RNMOM];
+  double dm[FACE_MOM];
 #pragma unroll
-  for (int k = 0; k < RNMOM; ++k) dm[k] = rec[FR_MOM + k];
-  rotate_moments(dm, n);
-  // face state: the reference's moments in the face frame plus the deviation's
+  for (int k = 0; k < FACE_MOM; ++k) dm[k] = rec[FR_MOM + k];
+  // face state: the reference's moments plus the deviation's, face frame
   const double *R = ref.mom;
-  const V2 rU = to_local(v2(R[RM10], R[RM01]), n);
-  const P4 W = p4(R[RM00] + dm[RM00], rU.x + dm[RM10], rU.y + dm[RM01],
-                  0.5 * ((R[RM20] + R[RM02] + R[RB00]) + (dm[RM20] + dm[RM02] + dm[RB00])));
+  const V2 Wm = to_local(v2(R[RM10] + dm[1], R[RM01] + dm[2]), n);
+  const P4 W = p4(R[RM00] + dm[0], Wm.x, Wm.y, 0.5 * ((R[RM20] + R[RM02] + R[RB00]) + (dm[3] + dm[5] + dm[6])));
   Rcp rc;
   const P4 prim = to_primary_rcp(d, W, rc);
   const V2 Ug = to_global(v2(prim.s1, prim.s2), n);
-  // face heat flux (calcFaceQ, clUGKS.c:522-585): M's part from its global
-  // moments rotated into the face frame, the deviation's from its raw moments
-  V2 Q = to_local(heat_flux_from_moments(R, d.K, Ug), n);
+  // face heat flux (calcFaceQ, clUGKS.c:522-585): M's part and the deviation's,
+  // in the global frame, from their raw moments
+  V2 Q = heat_flux_from_moments(R, d.K, Ug);
   {
-    const V2 qd_ = heat_flux_from_moments(dm, d.K, v2(prim.s1, prim.s2));
-    Q.x += qd_.x;
-    Q.y += qd_.y;
+    const V2 qd_ = face_heat_flux(dm, nr_rcp(d.K), Ug);
+    Q = to_local(v2(Q.x + qd_.x, Q.y + qd_.y), n);
   }
   // the two cells beside the face (getAL / getAR inputs, getPLR slopes)
   double nbr[2][5];
@@ -407,8 +380,16 @@ __global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *_
 // in at most max_axes + 2 doubles), flux (the face record, then the axis
 // tables)
 inline int delta_moments_stride(int max_axes) { return ((max_axes + 2) + 1) & ~1; }
-inline int delta_flux_stride(int max_axes) { return 48 + (((12 * (max_axes + 2) + 7) / 8 + 1) & ~1); }
 
+constexpr int DELTA_RING = 2;
+template <int FM>
+constexpr size_t delta_ring_bytes() { return (size_t)DELTA_RING * ((FM == 1 ? 5 : 3) + 1) * 32 * sizeof(float4); }
+
+// Bound by the packed-FP32 pipe (69%) and the L1 / shared data pipe (66%) at 16
+// warps per SM.  Against plain loads of the stencil rows with the slopes stored
+// beside the values (latency-bound, 707 MB to DRAM): 280 -> 234 us on the 2x2-block
+// cavity with 422 MB; the flux sweep, which takes the slopes again from the
+// values and the cells, 171 -> 189 us.
 template <int FM, int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB) face_moments_warp(const ugks_fused_block *__restrict__ B, int nb,
                                                                     ugks_solve_state *__restrict__ solves,
@@ -418,7 +399,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_moments_warp(const ugks_f
   const int item = (int)blockIdx.x * WPC + warp;
   if (item >= count) return;
   FaceWork fwk;
-  if (!face_work<FM>(B, nb, solves, first + item, 0, fwk) || fwk.wall >= 0) return;
+  if (!face_work<FM, true>(B, nb, solves, first + item, 0, fwk) || fwk.wall >= 0) return;
   const ugks_fused_block &blk = B[fwk.bi];
   const ugks_block_desc &d = blk.d;
   const int dir = fwk.dir;
@@ -439,88 +420,114 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_moments_warp(const ugks_f
   }
   __syncwarp();
   const int pstep = (dir == SOUTH ? 1 : d.Nj) * NP;  // pairs between neighbouring cells along the normal
-  const float4 *fcell = reinterpret_cast<const float4 *>(blk.f) + pidx(d, gi, gj, 0);
-  const float4 *up1 = fcell - (MID + 1) * pstep, *up0 = fcell + MID * pstep;
+  const float4 *far = reinterpret_cast<const float4 *>(blk.f) + pidx(d, gi, gj, 0) - (MID + 1) * pstep;  // slot 0
   float4 *frow = reinterpret_cast<float4 *>(dir == SOUTH ? blk.flux_S : blk.flux_W) + pidx(d, gi, gj, 0);
-  float4 *arow = reinterpret_cast<float4 *>(dir == SOUTH ? blk.aux_S : blk.aux_W) + pidx(d, gi, gj, 0);
-  const float2 nx2 = bc2((float)n.x), ny2 = bc2((float)n.y), mny2 = bc2(-(float)n.y);
-  // raw moments of the face deviation in the global frame (the coefficient
-  // pass rotates the sums into the face frame): products and each lane's sums
-  // in packed FP32, the two velocities of a pair in the two halves, about 17
-  // terms per half at Nv 1089; the halves and the lanes are combined in FP64
-  float2 acc[RNMOM];
+  const float2 nx2 = bc2((float)n.x), ny2 = bc2((float)n.y);
+  // raw moments (FACE_MOM, as face_item_fp64's) of the face deviation in the
+  // global frame: products and each lane's sums in packed FP32, the two
+  // velocities of a pair in the two halves, about 17 terms per half at Nv 1089;
+  // the halves and the lanes are combined in FP64
+  float2 acc[FACE_MOM];
 #pragma unroll
-  for (int k = 0; k < RNMOM; ++k) acc[k] = make_float2(0.0f, 0.0f);
+  for (int k = 0; k < FACE_MOM; ++k) acc[k] = make_float2(0.0f, 0.0f);
+  const float2 Kinv = bc2((float)(1.0 / d.K));
   // pair p = a v_num + jv: velocities (2a, jv) and (2a + 1, jv)
   const int qs = 32 / vn, rs = 32 % vn;
-  int ia = lane / vn, jv = lane % vn;
-  // reconstruction, stored face values and slopes, and moments of pair p
-  // from its stencil rows
-  auto pair_work = [&](int p, const float2 (&Sh)[L], const float2 (&Sb)[L], float2 qx, float2 qy, bool ua, bool ub) {
-    const float2 il = make_float2(ua ? il1 : il0, ub ? il1 : il0);
-    const float2 ds = make_float2(ua ? dist1 : dist0, ub ? dist1 : dist0);
-    const float2 ids = make_float2(ua ? idist1 : idist0, ub ? idist1 : idist0);
-    const float2 sh2 = slope_pair<FM>(Sh, il, ids), sb2 = slope_pair<FM>(Sb, il, ids);
-    const float2 fh = fma2(sh2, ds, Sh[MID]), fb = fma2(sb2, ds, Sb[MID]);
-    frow[p] = cat2(fh, fb);
-    arow[p] = cat2(sh2, sb2);
-    // raw moments (global frame); the padding velocity has df = 0
-    const float2 xh = mul2(qx, fh), yh = mul2(qy, fh), xx = mul2(qx, qx), yy = mul2(qy, qy);
-    acc[RM00] = add2(acc[RM00], fh);
-    acc[RM10] = add2(acc[RM10], xh);
-    acc[RM01] = add2(acc[RM01], yh);
-    acc[RM20] = fma2(qx, xh, acc[RM20]);
-    acc[RM11] = fma2(qy, xh, acc[RM11]);
-    acc[RM02] = fma2(qy, yh, acc[RM02]);
-    acc[RM30] = fma2(xx, xh, acc[RM30]);
-    acc[RM21] = fma2(xx, yh, acc[RM21]);
-    acc[RM12] = fma2(yy, xh, acc[RM12]);
-    acc[RM03] = fma2(yy, yh, acc[RM03]);
-    acc[RB00] = add2(acc[RB00], fb);
-    acc[RB10] = fma2(qx, fb, acc[RB10]);
-    acc[RB01] = fma2(qy, fb, acc[RB01]);
+  auto advance = [&](int &ia, int &jv) {
+    jv += rs;
+    ia += qs;
+    if (jv >= vn) { jv -= vn; ++ia; }
   };
+  auto normal_velocity = [&](int ia, int jv) {
+    return fma2(*reinterpret_cast<const float2 *>(QXf + 2 * ia), nx2, mul2(bc2(QYf[jv]), ny2));
+  };
+  // the stencil rows run DELTA_RING pairs of this lane ahead through cp.async
+  // stages: slots 0 .. L hold the cells from MID + 1 before the face to MID
+  // after it; a pair upwinded from one side copies the L it needs, one whose
+  // velocities disagree all of them; a lane reads back only what it copied
+  constexpr int D = DELTA_RING;
+  float4 *ring = reinterpret_cast<float4 *>(dyn + (size_t)WPC * wstride) + (size_t)warp * (D * (L + 1) * 32) + lane;
+  int ia2 = lane / vn, jv2 = lane % vn;
+  auto issue = [&](int p, int stage) {
+    if (p < NP) {
+      const float2 U = normal_velocity(ia2, jv2);
+      const bool first_ = U.x > 0.0f || U.y > 0.0f, last_ = !(U.x > 0.0f) || !(U.y > 0.0f);
+      float4 *r = ring + stage * ((L + 1) * 32);
+      const float4 *src = far + p;
+      if (first_) cp_async<16, true>(r, src);
+#pragma unroll
+      for (int s = 1; s < L; ++s) cp_async<16, true>(r + 32 * s, src + s * pstep);
+      if (last_) cp_async<16, true>(r + 32 * L, src + L * pstep);
+      advance(ia2, jv2);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < D; ++s) issue(lane + 32 * s, s);
+  int ia = lane / vn, jv = lane % vn, stage = 0;
 #pragma unroll 1
   for (int p = lane; p < NP; p += 32) {
     const float2 qx = *reinterpret_cast<const float2 *>(QXf + 2 * ia), qy = bc2(QYf[jv]);
-    const float2 U = fma2(qx, nx2, mul2(qy, ny2));
-    const bool ua = U.x > 0.0f, ub = U.y > 0.0f;
+    const float2 Un = fma2(qx, nx2, mul2(qy, ny2));
+    const bool ua = Un.x > 0.0f, ub = Un.y > 0.0f;
+    cp_async_wait<D - 1>();
+    const float4 *r = ring + stage * ((L + 1) * 32);
     float2 Sh[L], Sb[L];
-    if (ua == ub) {
-      const float4 *s0 = (ua ? up1 : up0) + p;
-      const int st = ua ? pstep : -pstep;
+    {
+      const float4 *s0 = ua ? r : r + 32 * L;
+      const int st = ua ? 32 : -32;
 #pragma unroll
       for (int s = 0; s < L; ++s) {
         const float4 x = s0[s * st];
         Sh[s] = lo2(x);
         Sb[s] = hi2(x);
       }
-    } else {
+    }
+    if (ua != ub) {
       // the two velocities of the pair are upwinded from opposite sides
-      const float4 *sa = (ua ? up1 : up0) + p, *sb = (ub ? up1 : up0) + p;
-      const int ta = ua ? pstep : -pstep, tb = ub ? pstep : -pstep;
+      const float4 *s0 = ub ? r : r + 32 * L;
+      const int st = ub ? 32 : -32;
 #pragma unroll
       for (int s = 0; s < L; ++s) {
-        const float4 x = sa[s * ta], y = sb[s * tb];
-        Sh[s] = make_float2(x.x, y.y);
-        Sb[s] = make_float2(x.z, y.w);
+        const float4 x = s0[s * st];
+        Sh[s].y = x.y;
+        Sb[s].y = x.w;
       }
     }
-    pair_work(p, Sh, Sb, qx, qy, ua, ub);
-    jv += rs;
-    ia += qs;
-    if (jv >= vn) { jv -= vn; ++ia; }
+    const float2 il = make_float2(ua ? il1 : il0, ub ? il1 : il0);
+    const float2 ds = make_float2(ua ? dist1 : dist0, ub ? dist1 : dist0);
+    const float2 ids = make_float2(ua ? idist1 : idist0, ub ? idist1 : idist0);
+    const float2 sh2 = slope_pair<FM>(Sh, il, ids), sb2 = slope_pair<FM>(Sb, il, ids);
+    const float2 fh = fma2(sh2, ds, Sh[MID]), fb = fma2(sb2, ds, Sb[MID]);
+    frow[p] = cat2(fh, fb);
+    issue(p + 32 * D, stage);
+    stage = stage + 1 == D ? 0 : stage + 1;
+    // raw moments (global frame); the padding velocity has df = 0
+    const float2 xh = mul2(qx, fh), yh = mul2(qy, fh);
+    const float2 tq = fma2(fma2(qx, qx, mul2(qy, qy)), fh, mul2(fb, Kinv));
+    acc[0] = add2(acc[0], fh);
+    acc[1] = add2(acc[1], xh);
+    acc[2] = add2(acc[2], yh);
+    acc[3] = fma2(qx, xh, acc[3]);
+    acc[4] = fma2(qy, xh, acc[4]);
+    acc[5] = fma2(qy, yh, acc[5]);
+    acc[6] = add2(acc[6], fb);
+    acc[7] = fma2(qx, tq, acc[7]);
+    acc[8] = fma2(qy, tq, acc[8]);
+    advance(ia, jv);
   }
-  double mom[RNMOM];
+  cp_async_wait<0>();
+  double mom[FACE_MOM];
 #pragma unroll
-  for (int k = 0; k < RNMOM; ++k) mom[k] = (double)acc[k].x + (double)acc[k].y;
-  const double tw = warp_spread_sum<RNMOM>(mom);
-  constexpr int S = spread_shift<RNMOM>();
-  if ((lane & ((1 << S) - 1)) == 0 && (lane >> S) < RNMOM)
+  for (int k = 0; k < FACE_MOM; ++k) mom[k] = (double)acc[k].x + (double)acc[k].y;
+  const double tw = warp_spread_sum<FACE_MOM>(mom);
+  constexpr int S = spread_shift<FACE_MOM>();
+  if ((lane & ((1 << S) - 1)) == 0 && (lane >> S) < FACE_MOM)
     blk.face_rec[(size_t)UGKS_FACE_REC * fk + FR_MOM + (lane >> S)] = tw;
 }
 
-// 3. flux (a warp per face): the FP64 sweep's terms (see face_item_fp64) with
+// ---------------------------------------------------------------------------
+// 3. flux, a face per warp: the FP64 sweep's terms (see face_item_fp64) with
 // f = M + df:
 //   dflux_h = u Mt0 len M r + Zh + u h0 (B - Mt0),
 //   dflux_b = u Mt0 len M ((kb - kb0) + kb r) + Zb + u h0 (kb (B - Mt0) + Mt1 u a3 X/2 + Mt2 aT3 X/2),
@@ -528,157 +535,20 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_moments_warp(const ugks_f
 //   h0 = len M (1 + r), r = g / M - 1,
 // and the discrete macro flux is Mt3 len sum(u M (1, u, v, |u|^2; kb0)) (the
 // reference's moments) plus the sums of the deviation Z terms
-template <int WPC, int MINB>
-__global__ void __launch_bounds__(WPC * 32, MINB) face_flux_warp(const ugks_fused_block *__restrict__ B, int nb,
-                                                                 ugks_solve_state *__restrict__ solves,
-                                                                 int n_faces, int wstride) {
-  extern __shared__ double dyn[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = (int)blockIdx.x * WPC + warp;
-  if (item >= n_faces) return;
-  FaceWork fwk;
-  if (!face_work<-1>(B, nb, solves, item, 0, fwk) || fwk.wall >= 0) return;
-  const ugks_fused_block &blk = B[fwk.bi];
-  const ugks_block_desc &d = blk.d;
-  const int dir = fwk.dir;
-  const long gi = fwk.gi, gj = fwk.gj;
-  const int NP = npairs(d), un = d.u_num, vn = d.v_num;
-  const RefMaxwellian ref = ref_of(blk);
-  const size_t fk = faceidx(d, gi, gj, dir);
-  const double *rec = blk.face_rec + (size_t)UGKS_FACE_REC * fk;
-  const V2 n = ld2(blk.normal, fk);
-  const double len = blk.side_length[fk];
-  double *fc = dyn + (size_t)warp * wstride;
-  float2 *EAU = reinterpret_cast<float2 *>(fc + 48), *EAV = EAU + (un + 1);  // (expm1 table, axis factor)
-  float *QX = reinterpret_cast<float *>(EAV + vn), *QY = QX + (un + 1);
-  const float4 *EAU2 = reinterpret_cast<const float4 *>(EAU);  // the two u-nodes of a pair row
-  const float2 *QX2 = reinterpret_cast<const float2 *>(QX);
-  fc[lane] = rec[lane];
-  if (lane < 16) fc[32 + lane] = rec[32 + lane];
-  __syncwarp();
-  {
-    // expm1 axis tables of the face Maxwellian against M, its axis factors
-    // (the face length on the u axis) and the axis velocities; entry un is
-    // the padding lane's: 0
-    const double lam = fc[FR_LAM], Ugx = fc[FR_UGX], Ugy = fc[FR_UGY], lnP = fc[FR_LNP];
-    for (int k = lane; k <= un + vn; k += 32) {
-      if (k < un) {
-        const double x = d.quad[2 * (size_t)k * vn];
-        EAU[k] = make_float2((float)axis_expm1(x, Ugx, lam, ref.lam0, lnP), (float)(ref.Au[k] * len));
-        QX[k] = (float)x;
-      } else if (k == un) {
-        EAU[k] = make_float2(0.0f, 0.0f);
-        QX[k] = 0.0f;
-      } else {
-        const int j = k - un - 1;
-        const double y = d.quad[2 * (size_t)j + 1];
-        EAV[j] = make_float2((float)axis_expm1(y, Ugy, lam, ref.lam0), (float)ref.Av[j]);
-        QY[j] = (float)y;
-      }
-    }
-  }
-  __syncwarp();
-  const double *c = fc + FR_C;
-  const double Mt0 = c[15];
-  const float2 nx2 = bc2((float)n.x), ny2 = bc2((float)n.y), mny2 = bc2(-(float)n.y);
-  const float2 fUx = bc2((float)fc[FR_UX]), fUy = bc2((float)fc[FR_UY]), flam2 = bc2((float)(2.0 * fc[FR_LAM]));
-  const float2 fsx = bc2((float)fc[FR_SX]), fsy = bc2((float)fc[FR_SY]);
-  const float2 fkb = bc2((float)fc[FR_KB]), fdkb = bc2((float)(fc[FR_KB] - ref.kb0));
-  const float2 fMt0 = bc2((float)Mt0), fMt3L = bc2((float)c[16]), fnMt4L = bc2((float)(-c[17]));
-  const float2 fT0 = bc2((float)(c[10] - Mt0)), fT1 = bc2((float)c[11]), fT2 = bc2((float)c[12]);
-  const float2 fT3 = bc2((float)c[13]), fCT = bc2((float)c[14]);
-  // upwind slope coefficients: aR for u <= 0, aR + dA for u > 0
-  const float2 AR0 = bc2((float)c[5]), AR1 = bc2((float)c[6]), AR2 = bc2((float)c[7]), AR3 = bc2((float)c[8]);
-  const float2 AR4 = bc2((float)c[9]);
-  const float2 dA0 = bc2((float)(c[0] - c[5])), dA1 = bc2((float)(c[1] - c[6])), dA2 = bc2((float)(c[2] - c[7]));
-  const float2 dA3 = bc2((float)(c[3] - c[8])), dA4 = bc2((float)(c[4] - c[9]));
-  float2 acc[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) acc[k] = make_float2(0.0f, 0.0f);
-  float4 *frow = reinterpret_cast<float4 *>(dir == SOUTH ? blk.flux_S : blk.flux_W) + pidx(d, gi, gj, 0);
-  const float4 *arow = reinterpret_cast<const float4 *>(dir == SOUTH ? blk.aux_S : blk.aux_W) + pidx(d, gi, gj, 0);
-  const int qs = 32 / vn, rs = 32 % vn;
-  int ia = lane / vn, jv = lane % vn;
-#pragma unroll 1
-  for (int p = lane; p < NP; p += 32) {
-    const float4 fd = frow[p], sg = arow[p];
-    const float4 eu = EAU2[ia];  // (a, len Au) of u-nodes 2ia and 2ia + 1
-    const float2 ev = EAV[jv];   // (b, Av), shared by the pair
-    const float2 qx = QX2[ia], qy = bc2(QY[jv]);
-    const float2 U = fma2(qx, nx2, mul2(qy, ny2)), T = fma2(qy, nx2, mul2(qx, mny2));
-    const float2 r = rel_excess(make_float2(eu.x, eu.z), bc2(ev.x));
-    const float2 ml = mul2(make_float2(eu.y, eu.w), bc2(ev.y));  // len M
-    const float2 h0 = fma2(ml, r, ml);
-    const float2 uu = fma2(U, U, mul2(T, T));
-    const float2 cx = sub2(U, fUx), cy = sub2(T, fUy), c2 = fma2(cx, cx, mul2(cy, cy));
-    const float2 Sp = fma2(cx, fsx, mul2(cy, fsy));
-    const float2 S4 = mul2(Sp, fma2(flam2, c2, bc2(-4.0f))), S2 = fma2(bc2(2.0f), Sp, S4);
-    const float2 pos = make_float2(U.x > 0.0f ? 1.0f : 0.0f, U.y > 0.0f ? 1.0f : 0.0f);
-    const float2 MPR = fma2(AR3, uu, fma2(AR2, T, fma2(AR1, U, AR0)));
-    const float2 dMP = fma2(dA3, uu, fma2(dA2, T, fma2(dA1, U, dA0)));
-    const float2 MP = fma2(pos, dMP, MPR), A4 = fma2(pos, dA4, AR4);
-    const float2 Bk = fma2(U, MP, fma2(fT3, uu, fma2(fT2, T, fma2(fT1, U, fT0))));  // B - Mt0
-    const float2 mu = mul2(fnMt4L, U);
-    const float2 Rh = fma2(mu, lo2(sg), mul2(fMt3L, lo2(fd))), Rb = fma2(mu, hi2(sg), mul2(fMt3L, hi2(fd)));
-    const float2 Zh = mul2(U, fma2(S4, h0, Rh)), Zb = mul2(U, fma2(mul2(S2, fkb), h0, Rb));
-    const float2 uh = mul2(U, h0), um0 = mul2(mul2(U, ml), fMt0);
-    const float2 hx = fma2(uh, Bk, fma2(um0, r, Zh));
-    const float2 hy = fma2(uh, fma2(fkb, Bk, fma2(A4, U, fCT)), fma2(um0, fma2(fkb, r, fdkb), Zb));
-    acc[0] = add2(acc[0], Zh);
-    acc[1] = fma2(U, Zh, acc[1]);
-    acc[2] = fma2(T, Zh, acc[2]);
-    acc[3] = fma2(uu, Zh, acc[3]);
-    acc[4] = add2(acc[4], Zb);
-    frow[p] = cat2(hx, hy);
-    jv += rs;
-    ia += qs;
-    if (jv >= vn) { jv -= vn; ++ia; }
-  }
-  // the per-lane FP32 sums, added in FP64 across the warp
-  double af[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) af[k] = (double)acc[k].x + (double)acc[k].y;
-  const double tw = warp_spread_sum<5>(af);
-  constexpr int S = spread_shift<5>();
-  double da[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) da[k] = __shfl_sync(0xffffffffu, tw, k << S);
-  if (lane == 0) {
-    // M's part of the discrete macro flux: sums of u_n M (1, u_n, u_t, |u|^2)
-    // and u_n M_b from the global moments
-    const double *R = ref.mom;
-    const double nx = n.x, ny = n.y, Mt3L = c[16];
-    const double K0 = nx * R[RM10] + ny * R[RM01];
-    const double K1 = nx * nx * R[RM20] + 2.0 * nx * ny * R[RM11] + ny * ny * R[RM02];
-    const double K2 = -nx * ny * R[RM20] + (nx * nx - ny * ny) * R[RM11] + nx * ny * R[RM02];
-    const double K3 = nx * (R[RM30] + R[RM12]) + ny * (R[RM21] + R[RM03]);
-    const double Kb = nx * R[RB10] + ny * R[RB01];
-    P4 out = p4(da[0] + Mt3L * K0 + c[18], da[1] + Mt3L * K1 + c[19], da[2] + Mt3L * K2 + c[20],
-                0.5 * ((da[3] + Mt3L * K3) + (da[4] + Mt3L * Kb)) + c[21]);
-    const V2 g = to_global(v2(out.s1, out.s2), n);
-    out.s1 = g.x;
-    out.s2 = g.y;
-    st4(dir == SOUTH ? blk.flux_macro_S : blk.flux_macro_W, gidx(d, gi, gj), out);
-  }
-}
-
+// The rows of a face (its values, and the cells before and after it, for the
+// slope (value - upwind cell) / distance) are copied into shared memory by the
+// bulk-copy engine in chunks of FLUX_CHUNK pairs, two chunks in flight (the copy
+// of chunk c + 1 runs while the lanes work on chunk c; the first overlaps the
+// axis tables)
 // ---------------------------------------------------------------------------
-// the flux sweep with its rows staged by the bulk-copy engine: a face per
-// warp, its stored face values and slopes copied into shared memory in chunks
-// of FLUX_CHUNK pairs, two chunks in flight (the copy of chunk c + 1 runs
-// while the lanes work on chunk c; the first overlaps the axis tables)
-// ---------------------------------------------------------------------------
-#ifndef UGKS_FLUX_CHUNK
-#define UGKS_FLUX_CHUNK 128
-#endif
-constexpr int FLUX_CHUNK = UGKS_FLUX_CHUNK;
+constexpr int FLUX_CHUNK = 96;  // face pass 472 us on the 2x2-block cavity; 128, 64, 32: 474, 499, 524
 static_assert(FLUX_CHUNK % 32 == 0, "whole trips of a warp per chunk");
 constexpr uint32_t kCopyWaitPolls = UGKS_MBAR_TRY_WAIT ? 1u << 20 : 1u << 24;  // about 1 s
 constexpr int STATUS_COPY_TIMEOUT = 8;
 // bytes of shared memory per warp: two barriers, two chunk buffers (values and
-// slopes), the face record and the axis tables
+// the two cells), the face record and the axis tables
 inline size_t flux_tma_warp_bytes(int max_axes) {
-  return 16 + 2 * 2 * (size_t)FLUX_CHUNK * 16 + 48 * 8 + (((size_t)12 * (max_axes + 2) + 15) & ~(size_t)15);
+  return 16 + 2 * 3 * (size_t)FLUX_CHUNK * 16 + 48 * 8 + (((size_t)12 * (max_axes + 2) + 15) & ~(size_t)15);
 }
 
 template <int WPC, int MINB>
@@ -704,22 +574,25 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_flux_tma(const ugks_fused
   // this warp's shared memory
   unsigned char *wm = dyn_b + (size_t)warp * wbytes;
   uint64_t *bar = reinterpret_cast<uint64_t *>(wm);
-  float4 *buf = reinterpret_cast<float4 *>(wm + 16);  // [2][values | slopes][FLUX_CHUNK]
-  double *fc = reinterpret_cast<double *>(buf + 4 * FLUX_CHUNK);
+  float4 *buf = reinterpret_cast<float4 *>(wm + 16);  // [2][values | cell before | after][FLUX_CHUNK]
+  double *fc = reinterpret_cast<double *>(buf + 6 * FLUX_CHUNK);
   float2 *EAU = reinterpret_cast<float2 *>(fc + 48), *EAV = EAU + (un + 1);  // (expm1 table, axis factor)
   float *QX = reinterpret_cast<float *>(EAV + vn), *QY = QX + (un + 1);
   const float4 *EAU2 = reinterpret_cast<const float4 *>(EAU);
   const float2 *QX2 = reinterpret_cast<const float2 *>(QX);
   float4 *frow = reinterpret_cast<float4 *>(dir == SOUTH ? blk.flux_S : blk.flux_W) + pidx(d, gi, gj, 0);
-  const float4 *arow = reinterpret_cast<const float4 *>(dir == SOUTH ? blk.aux_S : blk.aux_W) + pidx(d, gi, gj, 0);
+  const float4 *after = reinterpret_cast<const float4 *>(blk.f) + pidx(d, gi, gj, 0);
+  const float4 *before = after - (size_t)(dir == SOUTH ? 1 : d.Nj) * NP;
+  const float idist0 = (float)blk.face_geo[6 * fk + 1], idist1 = (float)blk.face_geo[6 * fk + 4];
   const int nchunks = (NP + FLUX_CHUNK - 1) / FLUX_CHUNK;
   auto issue = [&](int c) {  // lane 0: the copies of chunk c into buffer c & 1
     const int p0 = c * FLUX_CHUNK, m = min(FLUX_CHUNK, NP - p0);
     const uint32_t bytes = (uint32_t)m * 16u;
-    float4 *dst = buf + (c & 1) * 2 * FLUX_CHUNK;
-    mbar_arrive_expect_tx(&bar[c & 1], 2u * bytes);
+    float4 *dst = buf + (c & 1) * 3 * FLUX_CHUNK;
+    mbar_arrive_expect_tx(&bar[c & 1], 3u * bytes);
     bulk_g2s(dst, frow + p0, bytes, &bar[c & 1]);
-    bulk_g2s(dst + FLUX_CHUNK, arow + p0, bytes, &bar[c & 1]);
+    bulk_g2s(dst + FLUX_CHUNK, before + p0, bytes, &bar[c & 1]);
+    bulk_g2s(dst + 2 * FLUX_CHUNK, after + p0, bytes, &bar[c & 1]);
   };
   if (lane == 0) {
     mbar_init(&bar[0], 1);
@@ -778,13 +651,13 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_flux_tma(const ugks_fused
     // rows); a lane that ran out of polls stops the whole warp
     ok = __all_sync(0xffffffffu, mbar_wait(&bar[ch & 1], (uint32_t)((ch >> 1) & 1), kCopyWaitPolls));
     if (!ok) break;
-    const float4 *bv = buf + (ch & 1) * 2 * FLUX_CHUNK, *bs = bv + FLUX_CHUNK;
+    const float4 *bv = buf + (ch & 1) * 3 * FLUX_CHUNK;
     const int p0 = ch * FLUX_CHUNK, m = min(FLUX_CHUNK, NP - p0);
     int ia = (p0 + lane) / vn, jv = (p0 + lane) % vn;
     const int qs = 32 / vn, rs = 32 % vn;
 #pragma unroll 1
     for (int q = lane; q < m; q += 32) {
-      const float4 fd = bv[q], sg = bs[q];
+      const float4 fd = bv[q];
       const float4 eu = EAU2[ia];
       const float2 ev = EAV[jv];
       const float2 qx = QX2[ia], qy = bc2(QY[jv]);
@@ -801,8 +674,18 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_flux_tma(const ugks_fused
       const float2 dMP = fma2(dA3, uu, fma2(dA2, T, fma2(dA1, U, dA0)));
       const float2 MP = fma2(pos, dMP, MPR), A4 = fma2(pos, dA4, AR4);
       const float2 Bk = fma2(U, MP, fma2(fT3, uu, fma2(fT2, T, fma2(fT1, U, fT0))));  // B - Mt0
-      const float2 mu = mul2(fnMt4L, U);
-      const float2 Rh = fma2(mu, lo2(sg), mul2(fMt3L, lo2(fd))), Rb = fma2(mu, hi2(sg), mul2(fMt3L, hi2(fd)));
+      // upwind cell and 1 / distance of either velocity
+      const bool ua = U.x > 0.0f, ub = U.y > 0.0f;
+      const float4 ca = bv[q + (ua ? FLUX_CHUNK : 2 * FLUX_CHUNK)];
+      float2 ch2 = lo2(ca), cb2 = hi2(ca);
+      if (ua != ub) {
+        const float4 cb = bv[q + (ub ? FLUX_CHUNK : 2 * FLUX_CHUNK)];
+        ch2.y = cb.y;
+        cb2.y = cb.w;
+      }
+      const float2 mu = mul2(mul2(fnMt4L, U), make_float2(ua ? idist1 : idist0, ub ? idist1 : idist0));
+      const float2 Rh = fma2(mu, sub2(lo2(fd), ch2), mul2(fMt3L, lo2(fd)));
+      const float2 Rb = fma2(mu, sub2(hi2(fd), cb2), mul2(fMt3L, hi2(fd)));
       const float2 Zh = mul2(U, fma2(S4, h0, Rh)), Zb = mul2(U, fma2(mul2(S2, fkb), h0, Rb));
       const float2 uh = mul2(U, h0), um0 = mul2(mul2(U, ml), fMt0);
       const float2 hx = fma2(uh, Bk, fma2(um0, r, Zh));
@@ -862,9 +745,6 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_flux_tma(const ugks_fused
 // 1.1e-5 relative after 2000 steps; unbiased rounding gives 3.9e-6.  The
 // random bits hash (step, block within its solve, velocity pair), so a solve
 // gets the same bits alone and in any batch.
-#ifndef UGKS_SR_STORE
-#define UGKS_SR_STORE 1
-#endif
 // integer hash (a 32-bit xorshift-multiply mixer) for stochastic rounding
 __device__ __forceinline__ uint32_t sr_hash(uint32_t x) {
   x ^= x >> 16;
@@ -910,6 +790,10 @@ __device__ __forceinline__ float sr_pick(float hi, float lo, uint32_t u16) {
 // per-warp shared memory (doubles): per velocity-axis node a float4 (the old
 // and new states' expm1 tables, the axis factor, the axis velocity) for the
 // u_num + 1 and v_num nodes, then CELL_COEF coefficient slots
+// stages of cp.async of the update's five rows, in pairs of a lane ahead: with
+// plain loads the pass took 0.207 instead of 0.186 ms on the 2x2-block cavity,
+// three stages 0.185; 24 warps per SM at 80 registers 0.207
+constexpr int CELL_RING_F32 = 2;
 inline int delta_cell_stride(int max_axes) { return 2 * (max_axes + 1) + CELL_COEF; }
 
 template <int MINB>
@@ -930,6 +814,26 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
   const size_t cm = on ? midx(d, cw.mi, cw.mj) : 0;
   float4 *TU = reinterpret_cast<float4 *>(dyn + (size_t)warp * wstride), *TV = TU + (un + 1);
   const double *bc = dyn + (size_t)warp * wstride + (wstride - CELL_COEF);
+  const size_t base = on ? pidx(d, gi, gj, 0) : 0;
+  const size_t sj = (size_t)NP, si = (size_t)d.Nj * NP;
+  float4 *gf = reinterpret_cast<float4 *>(blk.f);
+  const float4 *gS = reinterpret_cast<const float4 *>(blk.flux_S), *gW = reinterpret_cast<const float4 *>(blk.flux_W);
+  float4 *ring = reinterpret_cast<float4 *>(dyn + (size_t)CW * wstride) + (size_t)warp * (CELL_RING_F32 * 160) + lane;
+  const int np = on ? NP : 0;
+  auto issue = [&](int p, int stage) {
+    if (p < np) {
+      const size_t k = base + p;
+      float4 *r = ring + stage * 160;
+      cp_async<16>(r, gf + k);
+      cp_async<16>(r + 32, gS + k);
+      cp_async<16>(r + 64, gS + k + sj);
+      cp_async<16>(r + 96, gW + k);
+      cp_async<16>(r + 128, gW + k + si);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < CELL_RING_F32; ++s) issue(lane + 32 * s, s);
   P4 old = p4(1.0, 0.0, 0.0, 1.0);
   V2 Q = v2(0.0, 0.0);
   if (on) {
@@ -968,13 +872,11 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
   const double a3 = bc[CC_A3], a4 = bc[CC_A4], kn = bc[CC_KN], sn = bc[CC_SN];
   const double ko = (0.5 * d.K) * nr_rcp(old.s3);
   const double so = 0.8 * (1 - d.Pr) * (old.s3 * old.s3) * nr_rcp(old.s0);
-  const float2 fa1 = bc2((float)bc[CC_A1]), fa2 = bc2((float)bc[CC_A2]), fa3 = bc2((float)a3), fa4 = bc2((float)a4);
-#if UGKS_SR_STORE
+  const float2 fa2 = bc2((float)bc[CC_A2]), fa3 = bc2((float)a3), fa4 = bc2((float)a4);
   const float a1h = (float)bc[CC_A1];
   const float2 fa1h = bc2(a1h), fna1h = bc2(-a1h), fna1l = bc2(-(float)(bc[CC_A1] - (double)a1h));
   const uint32_t srseed =
       sr_hash((uint32_t)sol.steps * 0x9e3779b9u + (uint32_t)(bi - sol.first_block) * 0x85ebca6bu);
-#endif
   const float2 fkbn = bc2((float)kn), fkbo = bc2((float)ko);
   const float2 fdkn = bc2((float)(kn - ref.kb0)), fdko = bc2((float)(ko - ref.kb0));
   // the Shakhov factors weighted by a4 / a3, times the heat flux
@@ -982,10 +884,6 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
   const float2 fSnQx = bc2((float)(a3 * sn * Q.x)), fSnQy = bc2((float)(a3 * sn * Q.y));
   const float2 fUox = bc2((float)old.s1), fUoy = bc2((float)old.s2), fUnx = bc2((float)nU), fUny = bc2((float)nV);
   const float2 flo2 = bc2((float)(2.0 * old.s3)), fln2 = bc2((float)(2.0 * nl));
-  const size_t base = pidx(d, gi, gj, 0);
-  const size_t sj = (size_t)NP, si = (size_t)d.Nj * NP;
-  float4 *gf = reinterpret_cast<float4 *>(blk.f);
-  const float4 *gS = reinterpret_cast<const float4 *>(blk.flux_S), *gW = reinterpret_cast<const float4 *>(blk.flux_W);
   // moments of df' in FP64, products included: the deviation's heat flux
   // nearly cancels the reference's (q is a small difference of large
   // moments), so FP32 sums would dominate its error
@@ -997,10 +895,13 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
   // pair p = a v_num + jv: velocities (2a, jv) and (2a + 1, jv)
   const int qs = 32 / vn, rs = 32 % vn;
   int ia = lane / vn, jv = lane % vn;
+  int stage = 0;
 #pragma unroll 1
   for (int p = lane; p < NP; p += 32) {
     const size_t k = base + p;
-    const float4 f = gf[k], s0 = gS[k], s1 = gS[k + sj], w0 = gW[k], w1 = gW[k + si];
+    cp_async_wait<CELL_RING_F32 - 1>();
+    const float4 *r = ring + stage * 160;
+    const float4 f = r[0], s0 = r[32], s1 = r[64], w0 = r[96], w1 = r[128];
     const float4 ta = TU[2 * ia], tb = TU[2 * ia + 1], tv = TV[jv];
     const float2 qx = make_float2(ta.w, tb.w), qy = bc2(tv.w);
     const float2 m = mul2(make_float2(ta.z, tb.z), bc2(tv.z));  // M of the pair
@@ -1020,7 +921,6 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
                                 mul2(m, fma2(fa4, fma2(fkbo, ro, fdko), mul2(fa3, fma2(fkbn, rn, fdkn))))));
     const float2 flh = add2(sub2(lo2(s0), lo2(s1)), sub2(lo2(w0), lo2(w1)));
     const float2 flb = add2(sub2(hi2(s0), hi2(s1)), sub2(hi2(w0), hi2(w1)));
-#if UGKS_SR_STORE
     // stochastic rounding of the new deviation: f a1 + increment as a float
     // pair, rounded to a neighbouring float with probability given by its
     // distance
@@ -1031,10 +931,9 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
     sr_parts(hi2(f), ib, fa1h, fna1h, fna1l, bh, bl);
     const float2 oh = make_float2(sr_pick(hh.x, hl.x, h1 & 0xffffu), sr_pick(hh.y, hl.y, h1 >> 16));
     const float2 ob = make_float2(sr_pick(bh.x, bl.x, h2 & 0xffffu), sr_pick(bh.y, bl.y, h2 >> 16));
-#else
-    const float2 oh = fma2(lo2(f), fa1, fma2(flh, fa2, eh)), ob = fma2(hi2(f), fa1, fma2(flb, fa2, eb));
-#endif
     gf[k] = cat2(oh, ob);
+    issue(p + 32 * CELL_RING_F32, stage);
+    stage = stage + 1 == CELL_RING_F32 ? 0 : stage + 1;
     // moments of df' for the next face pass and calcQ of f^{n+1} with the new
     // macro (the deviation's part); a NaN anywhere reaches mom[0] or mom[3].
     // The padding velocity of an odd u_num has df' = 0 and reads velocity 0.

@@ -52,23 +52,12 @@ template <> struct FaceShape<4> { static constexpr int wpc = 4, minb = 3; };
 // launch shapes of the mixed moments sweep (a face per warp): warps per CTA x
 // CTAs per SM
 template <int V> struct MomentsShape;
-template <> struct MomentsShape<1> { static constexpr int wpc = 4, minb = 5; };
-template <> struct MomentsShape<2> { static constexpr int wpc = 4, minb = 4; };
+template <> struct MomentsShape<1> { static constexpr int wpc = 4, minb = 4; };
+template <> struct MomentsShape<2> { static constexpr int wpc = 4, minb = 5; };
 template <> struct MomentsShape<3> { static constexpr int wpc = 8, minb = 3; };
 template <> struct MomentsShape<4> { static constexpr int wpc = 4, minb = 6; };
 // and of the mixed flux sweep
-// 7 CTAs (28 warps) per SM at 72 registers: 0.617 -> 0.598 ms of face pass on
-// the 2x2-block cavity, 13.0 -> 12.2 ms on the 64-solve batch, against 5
-#ifndef UGKS_FLUX_MINB
-#define UGKS_FLUX_MINB 7
-#endif
-constexpr int FLUX_WPC = 4, FLUX_MINB = UGKS_FLUX_MINB;
-// the flux sweep with bulk-copied rows (face_flux_tma) instead of per-lane
-// loads: 0.598 -> 0.529 ms of face pass on the 2x2-block cavity (the sweep
-// itself 252 -> 169 us under ncu, DRAM 42% -> 62% of peak)
-#ifndef UGKS_FLUX_TMA
-#define UGKS_FLUX_TMA 1
-#endif
+constexpr int FLUX_WPC = 4;
 #ifndef UGKS_FLUX_TMA_MINB
 #define UGKS_FLUX_TMA_MINB 5
 #endif
@@ -871,6 +860,15 @@ __device__ __forceinline__ void add_moments(double2 e, double Kinv, double h, do
   m[8] = fma(e.y, t, m[8]);
 }
 
+// calcQ of a distribution from its raw moments M about 0 (add_moments), relative
+// to velocity U, global frame
+__device__ __forceinline__ V2 face_heat_flux(const double (&M)[FACE_MOM], double Kinv, V2 U) {
+  const double cu = fma(U.x, M[1], U.y * M[2]), U2 = fma(U.x, U.x, U.y * U.y);
+  const double T = fma(Kinv, M[6], M[3] + M[5]) - 2.0 * cu + U2 * M[0];
+  return v2(0.5 * (M[7] - 2.0 * fma(U.x, M[3], U.y * M[4]) + U2 * M[1] - U.x * T),
+            0.5 * (M[8] - 2.0 * fma(U.x, M[4], U.y * M[5]) + U2 * M[2] - U.y * T));
+}
+
 // stages of cp.async in flight per lane: the stencil rows of FACE_RING
 // velocities in sweep 1, (face value, upwind cell) of as many as fit in the
 // same memory in sweep 2; a lane reads back only what it copied
@@ -925,11 +923,8 @@ __device__ __noinline__ void face_coefficients(const ugks_fused_block &blk, doub
                                    scale(Mt[2], moment_au(aT, Mu, Mv, Mxi, 1, 0))));
   // calcQ of the face values (calcFaceQ, clUGKS.c:522-585) from their raw
   // moments about 0, global frame; times the Shakhov factor and Mt0
-  const double cu = fma(Ug.x, M[1], Ug.y * M[2]), U2 = fma(Ug.x, Ug.x, Ug.y * Ug.y);
-  const double T = fma(Kinv, M[6], M[3] + M[5]) - 2.0 * cu + U2 * M[0];
-  const double qx = M[7] - 2.0 * fma(Ug.x, M[3], Ug.y * M[4]) + U2 * M[1] - Ug.x * T;
-  const double qy = M[8] - 2.0 * fma(Ug.x, M[4], Ug.y * M[5]) + U2 * M[2] - Ug.y * T;
-  const double s0 = 0.4 * (1 - d.Pr) * (prim.s3 * prim.s3) * rc.rho * Mt[0];  // 0.8 ..., q = 1/2 sum
+  const V2 q = face_heat_flux(M, Kinv, Ug);
+  const double s0 = 0.8 * (1 - d.Pr) * (prim.s3 * prim.s3) * rc.rho * Mt[0];
   const double xk = Mxi[2] - kb * kb;
   // a1 u + a2 v = x (a1 n.x - a2 n.y) + y (a1 n.y + a2 n.x)
   auto put = [&](double *c, P4 z, double w, double w0) {
@@ -944,8 +939,8 @@ __device__ __noinline__ void face_coefficients(const ugks_fused_block &blk, doub
   if (lane == 3) {
     rec[FK_MT3] = Mt[3] * len;
     rec[FK_MT4] = Mt[4] * len;
-    rec[FK_SX] = s0 * qx;
-    rec[FK_SY] = s0 * qy;
+    rec[FK_SX] = s0 * q.x;
+    rec[FK_SY] = s0 * q.y;
     const V2 g = to_global(v2(g0.s1, g0.s2), n);
     rec[FK_G0] = len * g0.s0;
     rec[FK_G0 + 1] = len * g.x;
@@ -1896,9 +1891,21 @@ cudaError_t set_wall_attributes() {
   }
   return cudaSuccess;
 }
+template <int V>
+cudaError_t set_moments_shape() {
+  constexpr int W = MomentsShape<V>::wpc, M = MomentsShape<V>::minb;
+  cudaError_t r[3] = {allow_smem(face_moments_warp<0, W, M>), allow_smem(face_moments_warp<1, W, M>),
+                      allow_smem(face_moments_warp<3, W, M>)};
+  for (cudaError_t e : r)
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
 template <typename T>
 cudaError_t set_flux_attributes() {
   if constexpr (std::is_same<T, float>::value) {
+    cudaError_t r[4] = {set_moments_shape<1>(), set_moments_shape<2>(), set_moments_shape<3>(), set_moments_shape<4>()};
+    for (cudaError_t x : r)
+      if (x != cudaSuccess) return x;
     cudaError_t e = cudaFuncSetAttribute(face_flux_tma<FLUX_WPC, FLUX_TMA_MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e == cudaSuccess)
@@ -2040,9 +2047,9 @@ void launch_moments_shape(const ugks_fused_block *B, int nb, ugks_solve_state *s
   const unsigned g = (unsigned)((count + WPC - 1) / WPC);
   const size_t sm = (size_t)WPC * ws * sizeof(double);
   switch (method) {
-    case 0: face_moments_warp<0, WPC, MINB><<<g, WPC * 32, sm, st>>>(B, nb, solves, first, count, ws); break;
-    case 1: face_moments_warp<1, WPC, MINB><<<g, WPC * 32, sm, st>>>(B, nb, solves, first, count, ws); break;
-    case 3: face_moments_warp<3, WPC, MINB><<<g, WPC * 32, sm, st>>>(B, nb, solves, first, count, ws); break;
+    case 0: face_moments_warp<0, WPC, MINB><<<g, WPC * 32, sm + WPC * delta_ring_bytes<0>(), st>>>(B, nb, solves, first, count, ws); break;
+    case 1: face_moments_warp<1, WPC, MINB><<<g, WPC * 32, sm + WPC * delta_ring_bytes<1>(), st>>>(B, nb, solves, first, count, ws); break;
+    case 3: face_moments_warp<3, WPC, MINB><<<g, WPC * 32, sm + WPC * delta_ring_bytes<3>(), st>>>(B, nb, solves, first, count, ws); break;
     default: break;
   }
 }
@@ -2073,7 +2080,7 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   constexpr bool mixed = std::is_same<T, float>::value;
   // doubles of shared memory per cell warp
   const int cstride = mixed ? delta_cell_stride(z->max_axes) : 2 * z->max_axes + CELL_COEF;
-  const size_t csmem = (size_t)CW * cstride * sizeof(double) + (mixed ? 0 : (size_t)CW * cell_ring_bytes());
+  const size_t csmem = (size_t)CW * cstride * sizeof(double) + (mixed ? (size_t)CW * CELL_RING_F32 * 160 * 16 : (size_t)CW * cell_ring_bytes());
   const cudaError_t attr = set_step_attributes<T>();
   if (attr != cudaSuccess) return -(int)attr;
   if (face_limit_bytes<T>(z->max_nv, z->max_axes) > 200 * 1024 || csmem > 200 * 1024) return -(int)cudaErrorInvalidValue;
@@ -2125,15 +2132,9 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   launch_retry<T>(B, nb, z, solves, ns, st);
   if (mixed && z->n_faces) {
     face_coef_delta<<<(unsigned)((z->n_faces + 127) / 128), 128, 0, st>>>(B, nb, solves, z->n_faces);
-    if (UGKS_FLUX_TMA) {
-      const int wb = (int)flux_tma_warp_bytes(z->max_axes);
-      face_flux_tma<FLUX_WPC, FLUX_TMA_MINB><<<(unsigned)((z->n_faces + FLUX_WPC - 1) / FLUX_WPC), FLUX_WPC * 32,
-                                               (size_t)FLUX_WPC * wb, st>>>(B, nb, solves, z->n_faces, wb);
-    } else {
-      const int fs = delta_flux_stride(z->max_axes);
-      face_flux_warp<FLUX_WPC, FLUX_MINB><<<(unsigned)((z->n_faces + FLUX_WPC - 1) / FLUX_WPC), FLUX_WPC * 32,
-                                            (size_t)FLUX_WPC * fs * sizeof(double), st>>>(B, nb, solves, z->n_faces, fs);
-    }
+    const int wb = (int)flux_tma_warp_bytes(z->max_axes);
+    face_flux_tma<FLUX_WPC, FLUX_TMA_MINB><<<(unsigned)((z->n_faces + FLUX_WPC - 1) / FLUX_WPC), FLUX_WPC * 32,
+                                             (size_t)FLUX_WPC * wb, st>>>(B, nb, solves, z->n_faces, wb);
   }
   if (mixed) {
     mark(1);

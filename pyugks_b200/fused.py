@@ -275,10 +275,7 @@ class FusedSolver:
         blk.Q_next = z(ni, nj, 2)
         blk.face_geo = z(Ni, Nj, 2, 6)
         if self.precision != "fp64":
-            # the mixed face pass's scratch: slopes beside the stored face
-            # deviations, and a record per face between its three launches
-            blk.aux_S = z(*shape, dt=self.sdtype)
-            blk.aux_W = z(*shape, dt=self.sdtype)
+            # the mixed face pass's record per face between its three launches
             blk.face_rec = z(Ni, Nj, 2, _lib.FACE_REC)
         x = _lib.FusedBlock()
         d = x.d
@@ -307,7 +304,7 @@ class FusedSolver:
         if "ref" in tabs:
             x.ref = tabs["ref"].data_ptr()
         if self.precision != "fp64":
-            x.aux_S, x.aux_W, x.face_rec = blk.aux_S.data_ptr(), blk.aux_W.data_ptr(), blk.face_rec.data_ptr()
+            x.face_rec = blk.face_rec.data_ptr()
         blk.struct = x
         return blk
 
