@@ -225,7 +225,7 @@ __device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restri
     const int step = dir == SOUTH ? 1 : d.Nj;                  // cells
     const float4 *fcell = reinterpret_cast<const float4 *>(blk.f) + pidx(d, gi, gj, 0);
     const double2 *qd = reinterpret_cast<const double2 *>(d.quad);
-    for (int v = threadIdx.x; v < Nv; v += NT) {
+    auto face_value = [&](int v, double &h, double &b) {
       const double2 e = qd[v];
       const double u = e.x * n.x + e.y * n.y;
       const bool up = u > 0.0;
@@ -237,11 +237,11 @@ __device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restri
       float fh, fb, sx, sy;
       reconstruct_f<FM>(xs, up ? il1 : il0, up ? dist1 : dist0, up ? idist1 : idist0, fh, fb, sx, sy);
       const double m = ref.mh[v];
-      fw[2 * v] = m + (double)fh;
-      fw[2 * v + 1] = ref.kb0 * m + (double)fb;
-    }
+      h = m + (double)fh;
+      b = ref.kb0 * m + (double)fb;
+    };
     const double dl = dt * len;
-    wall_face<NT>(blk, sol, sh, fw, rin, wall, dir, gi, gj, mi, mj, n, len, dt, [&](int v, double hx, double hy) {
+    wall_face<NT>(blk, sol, sh, fw, rin, wall, dir, gi, gj, mi, mj, n, len, dt, face_value, [&](int v, double hx, double hy) {
       const double2 e = qd[v];
       const double m = dl * (e.x * n.x + e.y * n.y) * ref.mh[v];
       pair_put(frow, v, vn, (float)(hx - m), (float)(hy - ref.kb0 * m));

@@ -496,16 +496,18 @@ __device__ __forceinline__ void block_sum_to0(double (&x)[N], double *scratch) {
 // accommodatingWallDist (clUGKS.c:774-906) or adsorbingWall_P1 (clAdsorb.c:253-482)
 // followed by the re-emission stage (adsorbingWallD_P2 / S_P2 / CL_P2,
 // clAdsorb.c:488-975), then wallFlux (clUGKS.c:910-1011) and
-// wallMassEnergyFluxes (1019-1147).  fw holds the reconstructed face
-// distribution (h, b) per velocity in FP64 and is rewritten in place; rin is
-// shared scratch of Nv (h, b) pairs (double2, or float2 in the mixed path) for
-// the reflected incoming distribution; store_flux(v, h, b) writes the
-// face-flux row of velocity v.
-template <int NT, typename RIN, typename StoreFlux>
+// wallMassEnergyFluxes (1019-1147).  face_value(v, h, b) gives the reconstructed
+// face distribution; fw holds Nv (h, b) pairs (each thread reads back only what
+// it wrote); rin is shared scratch of Nv (h, b) pairs (FP64: the wall_dist row
+// itself) for the reflected incoming distribution; store_flux(v, h, b) writes
+// the face-flux row of velocity v.  A diffuse wall takes two sweeps: the face
+// values of the incoming half and the wall Maxwellian of the outgoing half (one
+// exp each) with their two sums, then the fluxes with their eight sums.
+template <int NT, typename RIN, typename FaceValue, typename StoreFlux>
 __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solve_state &sol, FaceShared<NT> &sh,
                                           double *fw, RIN *rin, const int wall, const int dir, const long gi,
                                           const long gj, const long mi, const long mj, const V2 n, const double len,
-                                          const double dt, StoreFlux store_flux) {
+                                          const double dt, FaceValue face_value, StoreFlux store_flux) {
   using R = double;
   const ugks_block_desc &d = blk.d;
   const int Nv = d.Nv;
@@ -523,26 +525,29 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
     wl.s1 = t.x;
     wl.s2 = t.y;
   }
-  __syncthreads();
+  double ratio_out = 1.0;  // diffuse: the outgoing half of fw is scaled by this
   if (blk.bc_type[wall] == BC_DIFFUSE) {
     // accommodatingWallDist (clUGKS.c:774-906)
     double s[2] = {0.0, 0.0};
     for (int v = threadIdx.x; v < Nv; v += NT) {
       const V2 uv = fvel(v);
-      const int delta = upwind_flag(uv.x, rot);
-      s[0] += uv.x * (1 - delta) * fw[2 * v];
-      s[1] -= uv.x * delta * maxwellian(d, wl, uv, v).x;
+      double h, b;
+      if (upwind_flag(uv.x, rot)) {
+        const V2 M = maxwellian(d, wl, uv, v);
+        h = M.x;
+        b = M.y;
+        s[1] -= uv.x * h;
+      } else {
+        face_value(v, h, b);
+        s[0] += uv.x * h;
+      }
+      fw[2 * v] = h;
+      fw[2 * v + 1] = b;
     }
-    block_sum<2>(s, sh.scratch);
-    const double ratio = s[0] / s[1];
-    for (int v = threadIdx.x; v < Nv; v += NT) {
-      const V2 uv = fvel(v);
-      const int delta = upwind_flag(uv.x, rot);
-      const V2 M = maxwellian(d, wl, uv, v);
-      fw[2 * v] = (R)(ratio * delta * M.x + (1 - delta) * fw[2 * v]);
-      fw[2 * v + 1] = (R)(ratio * delta * M.y + (1 - delta) * fw[2 * v + 1]);
-    }
+    block_sum_spread<2>(s, sh.scratch);
+    ratio_out = s[0] / s[1];
   } else {
+    for (int v = threadIdx.x; v < Nv; v += NT) face_value(v, fw[2 * v], fw[2 * v + 1]);
     // adsorbingWall_P1 (clAdsorb.c:253-482)
     const long ti = dir == SOUTH ? mi : (wall == GEAST ? d.ni - 1 : 0);
     const long tj = dir == SOUTH ? (wall == GNORTH ? d.nj - 1 : 0) : mj;
@@ -692,33 +697,29 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
       fw[2 * v + 1] = (R)y;
     }
   }
-  // wallFlux (clUGKS.c:910-1011) and wallMassEnergyFluxes (1019-1147)
-  double s[12];
+  // wallFlux (clUGKS.c:910-1011) and wallMassEnergyFluxes (1019-1147): the
+  // incoming and outgoing sums; the face macro flux is both together
+  double s[8];
 #pragma unroll
-  for (int k = 0; k < 12; ++k) s[k] = 0.0;
+  for (int k = 0; k < 8; ++k) s[k] = 0.0;
+  const double ld = len * dt;
   for (int v = threadIdx.x; v < Nv; v += NT) {
     const V2 uv = fvel(v);
-    const double wh = fw[2 * v], wb = fw[2 * v + 1];
-    const double oh = uv.x * wh * len * dt, ob = uv.x * wb * len * dt;
+    const bool out = upwind_flag(uv.x, rot) != 0;
+    const double k = uv.x * ld * (out ? ratio_out : 1.0);
+    const double oh = k * fw[2 * v], ob = k * fw[2 * v + 1];
     store_flux(v, oh, ob);
-    const double uu = uv.x * uv.x + uv.y * uv.y;
-    s[0] += uv.x * wh;
-    s[1] += uv.x * uv.x * wh;
-    s[2] += uv.x * uv.y * wh;
-    s[3] += 0.5 * uv.x * (uu * wh + wb);
-    const int delta = upwind_flag(uv.x, rot);
-    const double ix = (1 - delta) * oh, iy = (1 - delta) * ob, ox = delta * oh, oy = delta * ob;
-    s[4] += ix; s[5] += uv.x * ix; s[6] += uv.y * ix; s[7] += 0.5 * (uu * ix + iy);
-    s[8] += ox; s[9] += uv.x * ox; s[10] += uv.y * ox; s[11] += 0.5 * (uu * ox + oy);
+    const double e = 0.5 * ((uv.x * uv.x + uv.y * uv.y) * oh + ob), px = uv.x * oh, py = uv.y * oh;
+    s[0] += out ? 0.0 : oh; s[1] += out ? 0.0 : px; s[2] += out ? 0.0 : py; s[3] += out ? 0.0 : e;
+    s[4] += out ? oh : 0.0; s[5] += out ? px : 0.0; s[6] += out ? py : 0.0; s[7] += out ? e : 0.0;
   }
-  block_sum<12>(s, sh.scratch);
+  block_sum_spread_to0<8>(s, sh.scratch);
   if (threadIdx.x == 0) {
-    const V2 g = to_global(v2(s[1], s[2]), n);
-    st4(dir == SOUTH ? blk.flux_macro_S : blk.flux_macro_W, gidx(d, gi, gj),
-        scale(dt * len, p4(s[0], g.x, g.y, s[3])));
+    const V2 g = to_global(v2(s[1] + s[5], s[2] + s[6]), n);
+    st4(dir == SOUTH ? blk.flux_macro_S : blk.flux_macro_W, gidx(d, gi, gj), p4(s[0] + s[4], g.x, g.y, s[3] + s[7]));
     double *wf = blk.wall_fluxes + 8 * (ci * 4 + wall);
-    wf[0] = -rot * s[4]; wf[1] = rot * s[8]; wf[2] = -rot * s[5]; wf[3] = rot * s[9];
-    wf[4] = -rot * s[6]; wf[5] = rot * s[10]; wf[6] = -rot * s[7]; wf[7] = rot * s[11];
+    wf[0] = -rot * s[0]; wf[1] = rot * s[4]; wf[2] = -rot * s[1]; wf[3] = rot * s[5];
+    wf[4] = -rot * s[2]; wf[5] = rot * s[6]; wf[6] = -rot * s[3]; wf[7] = rot * s[7];
   }
 }
 
@@ -1102,9 +1103,8 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, cons
 }
 
 // A wall face in FP64 (all NT threads of the CTA take part): the face values
-// are reconstructed into the face's flux row, which the wall procedure works
-// on in place (each thread reads back only what it wrote); the reflected
-// incoming distribution it gathers from is read where P1 put it, wall_dist.
+// live in the face's flux row, which the wall procedure works on in place; the
+// reflected incoming distribution it gathers from is read where P1 put it, wall_dist.
 template <int FM, int NT>
 __device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_solve_state &sol, const double dt,
                                             FaceShared<NT> &sh, const FaceWork fwk) {
@@ -1120,20 +1120,19 @@ __device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_so
   const double2 *up1 = fcell - (MID + 1) * step, *up0 = fcell + MID * step;
   const double2 *qd = reinterpret_cast<const double2 *>(d.quad);
   double2 *row = reinterpret_cast<double2 *>(dir == SOUTH ? blk.flux_S : blk.flux_W) + base;
-  for (int v = threadIdx.x; v < Nv; v += NT) {
+  auto face_value = [&](int v, double &h, double &b) {
     const double2 e = qd[v];
     const bool up = fma(e.x, n.x, e.y * n.y) > 0.0;
     const double *g = fg + (up ? 3 : 0);
     double2 xs[L];
     load_stencil((up ? up1 : up0) + v, up ? step : -step, xs);
-    double h, b, sx, sy;
+    double sx, sy;
     reconstruct<FM>(xs, g[2], g[0], g[1], h, b, sx, sy);
-    row[v] = make_double2(h, b);
-  }
+  };
   const long ci = dir == SOUTH ? fwk.mi : fwk.mj;
   wall_face<NT>(blk, sol, sh, reinterpret_cast<double *>(row),
                 reinterpret_cast<double2 *>(blk.wall_dist) + (size_t)ci * Nv, fwk.wall, dir, gi, gj, fwk.mi, fwk.mj, n,
-                blk.side_length[fk], dt, [&](int v, double hx, double hy) { row[v] = make_double2(hx, hy); });
+                blk.side_length[fk], dt, face_value, [&](int v, double hx, double hy) { row[v] = make_double2(hx, hy); });
 }
 
 // wall work item (2 (ni + nj) per block: the S faces of rows 0 and nj, then
@@ -2165,10 +2164,29 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   return launch_status();
 }
 
-// residual (getResidual, clUGKS.c:1259-1277, and ugks_block.py:1316-1327):
-// one CTA per solve walks its blocks
-__global__ void residual_kernel(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int ns) {
-  __shared__ double scratch[8 * (FT / 32)];
+// the stop rule of an active solve (ugks_stop_check)
+__device__ __forceinline__ void stop_rule(ugks_solve_state &x) {
+  int why = 0;
+  if (x.status != 0) why = UGKS_STOP_ERROR;
+  else if (x.stop_residual > 0.0 && x.steps >= x.stop_after && x.residual[0] < x.stop_residual)
+    why = UGKS_STOP_CONVERGED;
+  else if (x.stop_steps > 0 && x.steps >= x.stop_steps) why = UGKS_STOP_STEPS;
+  if (why) {
+    x.stopped = why;
+    x.active = 0;
+  }
+}
+
+// residual (getResidual, clUGKS.c:1259-1277, and ugks_block.py:1316-1327): one CTA
+// per solve walks its blocks, and with STOP applies the solve's stop rule.  The
+// sums are short (a few cells per thread), so the CTA is as wide as it can be: with
+// 128 threads six solves of up to 48 x 48 cells took 17 us, with 1024 and the stop
+// rule in it 7.
+constexpr int RES_NT = 1024;
+template <bool STOP>
+__global__ void __launch_bounds__(RES_NT) residual_kernel(const ugks_fused_block *B, int nb, ugks_solve_state *solves,
+                                                          int ns) {
+  __shared__ double scratch[8 * (RES_NT / 32)];
   const int s = blockIdx.x;
   if (s >= ns || !solves[s].active) return;  // a stopped solve keeps its last residual
   double r[4] = {0.0, 0.0, 0.0, 0.0};
@@ -2178,7 +2196,7 @@ __global__ void residual_kernel(const ugks_fused_block *B, int nb, ugks_solve_st
     const ugks_fused_block &blk = B[b];
     const int cells = blk.d.ni * blk.d.nj;
     double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int c = threadIdx.x; c < cells; c += blockDim.x) {
+    for (int c = threadIdx.x; c < cells; c += RES_NT) {
       const P4 p = ld4(blk.macro, c), o = ld4(blk.prim_old, c);
       a[0] += (p.s0 - o.s0) * (p.s0 - o.s0);
       a[1] += (p.s1 - o.s1) * (p.s1 - o.s1);
@@ -2189,15 +2207,18 @@ __global__ void residual_kernel(const ugks_fused_block *B, int nb, ugks_solve_st
       a[6] += fabs(p.s2);
       a[7] += fabs(p.s3);
     }
-    block_sum<8>(a, scratch);
-    for (int k = 0; k < 4; ++k) {
-      const double v = sqrt((double)cells * a[k]) / (a[4 + k] + DBL_MIN);
-      r[k] += v <= 0.0 ? 1.0 : v;
-    }
+    block_sum_spread_to0<8>(a, scratch);
+    if (threadIdx.x == 0)
+      for (int k = 0; k < 4; ++k) {
+        const double v = sqrt((double)cells * a[k]) / (a[4 + k] + DBL_MIN);
+        r[k] += v <= 0.0 ? 1.0 : v;
+      }
     ++n;
   }
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
     for (int k = 0; k < 4; ++k) solves[s].residual[k] = n ? r[k] / n : 0.0;
+    if (STOP) stop_rule(solves[s]);
+  }
 }
 
 // The bounded wait of the face pass's bulk copies, exercised on its own: a
@@ -2227,17 +2248,7 @@ __global__ void copy_wait_check(const float4 *src, unsigned polls, int *status) 
 __global__ void stop_check(ugks_solve_state *solves, int ns) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
-  ugks_solve_state &x = solves[s];
-  if (!x.active) return;
-  int why = 0;
-  if (x.status != 0) why = UGKS_STOP_ERROR;
-  else if (x.stop_residual > 0.0 && x.steps >= x.stop_after && x.residual[0] < x.stop_residual)
-    why = UGKS_STOP_CONVERGED;
-  else if (x.stop_steps > 0 && x.steps >= x.stop_steps) why = UGKS_STOP_STEPS;
-  if (why) {
-    x.stopped = why;
-    x.active = 0;
-  }
+  if (solves[s].active) stop_rule(solves[s]);
 }
 
 }  // namespace
@@ -2272,7 +2283,7 @@ int ugks_step_launches(const ugks_fused_sizes *z, int mixed) {
 int ugks_residual(const ugks_fused_block *blocks_dev, int nblocks, ugks_solve_state *solves_dev,
                   int nsolves, void *stream) {
   if (nsolves <= 0) return 0;
-  residual_kernel<<<nsolves, FT, 0, S(stream)>>>(blocks_dev, nblocks, solves_dev, nsolves);
+  residual_kernel<false><<<nsolves, RES_NT, 0, S(stream)>>>(blocks_dev, nblocks, solves_dev, nsolves);
   return launch_status();
 }
 
@@ -2287,8 +2298,10 @@ int ugks_serve_steps(int mixed, const ugks_fused_block *blocks_dev, int nblocks,
   for (int k = 0; k < nsteps; ++k) {
     int rc = mixed ? step_impl<float>(blocks_dev, nblocks, sizes, solves_dev, nsolves, stream)
                    : step_impl<double>(blocks_dev, nblocks, sizes, solves_dev, nsolves, stream);
-    if (rc == 0) rc = ugks_residual(blocks_dev, nblocks, solves_dev, nsolves, stream);
-    if (rc == 0) rc = ugks_stop_check(solves_dev, nsolves, stream);
+    if (rc == 0 && nsolves > 0) {
+      residual_kernel<true><<<nsolves, RES_NT, 0, S(stream)>>>(blocks_dev, nblocks, solves_dev, nsolves);
+      rc = launch_status();
+    }
     if (rc != 0) return rc;
   }
   return 0;
