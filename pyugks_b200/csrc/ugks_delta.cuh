@@ -160,11 +160,11 @@ __device__ __forceinline__ float2 slope_pair(const float2 (&S)[FM == 1 ? 5 : 3],
 // The per-face scalar work (face state, heat flux, half-range moments, slopes,
 // time weights: a chain of FP64 transcendentals) would otherwise run on one or
 // two lanes of every face CTA while the rest of the CTA waits.  Here it runs
-// one face per thread, between two sweeps that take one face per warp:
+// on its own, between two sweeps that take one face per warp:
 //   1. face_moments_warp: the reconstruction of every velocity pair, stored
 //      as the face deviation in the face's flux row, and nine raw moments of
 //      the deviation into the face record;
-//   2. face_coef_delta (a thread per face): the face state and every per-face
+//   2. face_coef_delta (two lanes per face): the face state and every per-face
 //      coefficient of the flux into the face record;
 //   3. face_flux_tma: the deviation flux of every velocity pair over the
 //      stored face deviations, written over them, and the macro flux.
@@ -188,13 +188,12 @@ inline size_t delta_wall_smem(int max_nv) { return 24 * (size_t)max_nv + 16; }
 // a wall face (a CTA per face): its whole procedure, in the main pass's wall
 // launch and in the retry pass, where interior faces have nothing to redo
 // (their moments do not depend on dt)
-template <int FM, int NT, bool WALLS>
-__device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restrict__ B, int nb,
+template <int FM, int NT>
+__device__ __forceinline__ void wall_item_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                 ugks_solve_state *__restrict__ solves, const int w, int retry_pass) {
   extern __shared__ double dyn[];
   FaceWork fwk;
   if (!face_work<FM>(B, nb, solves, w, retry_pass, fwk)) return;
-  static_assert(WALLS, "interior faces run in face_moments_warp");
   if (fwk.wall < 0) return;
   const ugks_fused_block &blk = B[fwk.bi];
   const ugks_block_desc &d = blk.d;
@@ -249,34 +248,53 @@ __device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restri
   }
 }
 
-// wall faces of the main pass: a CTA per wall work item (2 (ni + nj) per
-// block: the S faces of rows 0 and nj, then the W faces of columns 0 and ni),
-// running the wall procedure when that side of the block is a wall
-template <int NT>
-__global__ void __launch_bounds__(NT) wall_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
-                                                      ugks_solve_state *__restrict__ solves) {
-  const int w = (int)blockIdx.x;
+// a wall work item (2 (ni + nj) per block), when that side of the block is a wall
+constexpr int WALL_NT = 128;
+__device__ __forceinline__ void wall_work_delta(const ugks_fused_block *__restrict__ B, int nb,
+                                                ugks_solve_state *__restrict__ solves, int w, int retry_pass) {
   const ugks_fused_block &blk = B[find_block<3>(B, nb, w)];
-  const ugks_block_desc &d = blk.d;
   UGKS_CHECK_ITEM(3, blk, w, solves);
   const int fw = wall_to_face(blk, w);
-  switch (d.flux_method) {
-    case 0: face_item_delta<0, NT, true>(B, nb, solves, fw, 0); break;
-    case 1: face_item_delta<1, NT, true>(B, nb, solves, fw, 0); break;
-    case 3: face_item_delta<3, NT, true>(B, nb, solves, fw, 0); break;
+  switch (blk.d.flux_method) {
+    case 0: wall_item_delta<0, WALL_NT>(B, nb, solves, fw, retry_pass); break;
+    case 1: wall_item_delta<1, WALL_NT>(B, nb, solves, fw, retry_pass); break;
+    case 3: wall_item_delta<3, WALL_NT>(B, nb, solves, fw, retry_pass); break;
     default: break;
   }
 }
-constexpr int WALL_NT = 128;
+// wall faces of the main pass: a CTA per wall work item
+__global__ void __launch_bounds__(WALL_NT) wall_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
+                                                           ugks_solve_state *__restrict__ solves) {
+  pdl_begin();
+  wall_work_delta(B, nb, solves, (int)blockIdx.x, 0);
+}
+// and redone after a dt change
+__global__ void __launch_bounds__(WALL_NT) wall_retry_delta(const ugks_fused_block *__restrict__ B, int nb,
+                                                            ugks_solve_state *__restrict__ solves, int ns,
+                                                            int per_solve) {
+  pdl_begin();
+  int b0, bl;
+  if (!retry_solve(B, solves, ns, per_solve, b0, bl)) return;
+  const int end = B[bl].wall_begin + 2 * (B[bl].d.ni + B[bl].d.nj);
+  for (int w = B[b0].wall_begin + blockIdx.x % per_solve; w < end; w += per_solve) {
+    wall_work_delta(B, nb, solves, w, 1);
+    __syncthreads();  // the next item reuses the shared tables
+  }
+}
 
-// 2. coefficients: the per-face block of face_coefficients, one face per
-// thread (the same chain as the lanes of a face CTA run there)
-__global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *__restrict__ B, int nb,
-                                                       ugks_solve_state *__restrict__ solves, int n_faces) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n_faces) return;
+// 2. coefficients: the chain of face_coefficients, an interior face on two
+// neighbouring lanes (even: the side before the face, odd: after it).  A thread
+// per face with both sides in turn, in CTAs of 128, took 9.6 us on a 24x24 cavity
+// (10 CTAs) and 17 us on the 2x2-block cavity.
+constexpr int COEF_NT = 64;
+__global__ void __launch_bounds__(COEF_NT) face_coef_delta(const ugks_fused_block *__restrict__ B, int nb,
+                                                           ugks_solve_state *__restrict__ solves, int n_faces) {
+  pdl_begin();
+  const int th = blockIdx.x * COEF_NT + threadIdx.x, w = th >> 1, side = th & 1;
   FaceWork fwk;
-  if (!face_work<-1>(B, nb, solves, w, 0, fwk) || fwk.wall >= 0) return;
+  const bool on = w < n_faces && face_work<-1>(B, nb, solves, w, 0, fwk) && fwk.wall < 0;
+  const unsigned mask = __ballot_sync(0xffffffffu, on);
+  if (!on) return;
   const ugks_fused_block &blk = B[fwk.bi];
   const ugks_block_desc &d = blk.d;
   const double dt = step_dt(solves[blk.solve]).flux;
@@ -285,7 +303,10 @@ __global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *_
   const RefMaxwellian ref = ref_of(blk);
   const size_t fk = faceidx(d, gi, gj, dir);
   double *rec = blk.face_rec + (size_t)UGKS_FACE_REC * fk;
-  const V2 n = ld2(blk.normal, fk), mid = ld2(blk.mid_side, fk);
+  // the cell on this lane's side (getAL / getAR inputs, getPLR slopes)
+  const size_t ck = side == 0 ? gidx(d, gi - dir, gj - (1 - dir)) : gidx(d, gi, gj);
+  const P4 mc = ld4(blk.cell_mom, ck);
+  const V2 cc = ld2(blk.centre, ck), n = ld2(blk.normal, fk), mid = ld2(blk.mid_side, fk);
   const double len = blk.side_length[fk];
   double dm[FACE_MOM];
 #pragma unroll
@@ -297,77 +318,59 @@ __global__ void __launch_bounds__(128) face_coef_delta(const ugks_fused_block *_
   Rcp rc;
   const P4 prim = to_primary_rcp(d, W, rc);
   const V2 Ug = to_global(v2(prim.s1, prim.s2), n);
-  // face heat flux (calcFaceQ, clUGKS.c:522-585): M's part and the deviation's,
-  // in the global frame, from their raw moments
-  V2 Q = heat_flux_from_moments(R, d.K, Ug);
-  {
-    const V2 qd_ = face_heat_flux(dm, nr_rcp(d.K), Ug);
-    Q = to_local(v2(Q.x + qd_.x, Q.y + qd_.y), n);
-  }
-  // the two cells beside the face (getAL / getAR inputs, getPLR slopes)
-  double nbr[2][5];
-  for (int side = 0; side < 2; ++side) {
-    const size_t k = side == 0 ? gidx(d, gi - dir, gj - (1 - dir)) : gidx(d, gi, gj);
-    const P4 mc = ld4(blk.cell_mom, k);
-    const V2 uc = to_local(v2(mc.s1, mc.s2), n);
-    const V2 cc = ld2(blk.centre, k);
-    nbr[side][0] = mc.s0;
-    nbr[side][1] = uc.x;
-    nbr[side][2] = uc.y;
-    nbr[side][3] = mc.s3;
-    nbr[side][4] = nr_rcp(sqrt((mid.x - cc.x) * (mid.x - cc.x) + (mid.y - cc.y) * (mid.y - cc.y)));
-  }
   // getPLR slopes (clUGKS.c:424-436) and initMacroFlux (446-518)
-  const double kb = (0.5 * d.K) * rc.lam;
-  double Mh[2][MNUM], Mv[MTUM], Mxi[3];
-  P4 a[2], t1[2], t2[2];
-  for (int side = 0; side < 2; ++side) {
-    const double sg = side == 0 ? 1.0 : -1.0;
-    half_moments_rcp(d.PI, d.K, prim, rc, sg, Mh[side], Mv, Mxi);
-    const double id = sg * nbr[side][4];
-    a[side] = micro_slope_rcp(d.K, prim, rc,
-                              p4((W.s0 - nbr[side][0]) * id, (W.s1 - nbr[side][1]) * id,
-                                 (W.s2 - nbr[side][2]) * id, (W.s3 - nbr[side][3]) * id));
-    t1[side] = moment_au(a[side], Mh[side], Mv, Mxi, 1, 0);
-    t2[side] = moment_au(a[side], Mh[side], Mv, Mxi, 2, 0);
-  }
+  const double kb = (0.5 * d.K) * rc.lam, sg = side == 0 ? 1.0 : -1.0;
+  double Mh[MNUM], Mv[MTUM], Mxi[3];
+  half_moments_rcp(d.PI, d.K, prim, rc, sg, Mh, Mv, Mxi);
+  const V2 uc = to_local(v2(mc.s1, mc.s2), n);
+  const double id = sg * nr_rcp(sqrt((mid.x - cc.x) * (mid.x - cc.x) + (mid.y - cc.y) * (mid.y - cc.y)));
+  const P4 a = micro_slope_rcp(d.K, prim, rc,
+                               p4((W.s0 - mc.s0) * id, (W.s1 - uc.x) * id, (W.s2 - uc.y) * id, (W.s3 - mc.s3) * id));
+  auto both = [&](double z) { return z + __shfl_xor_sync(mask, z, 1); };
+  auto both4 = [&](P4 z) { return p4(both(z.s0), both(z.s1), both(z.s2), both(z.s3)); };
+  const P4 t1 = both4(moment_au(a, Mh, Mv, Mxi, 1, 0)), t2 = both4(moment_au(a, Mh, Mv, Mxi, 2, 0));
+  double Mu[MNUM];
+#pragma unroll
+  for (int k = 0; k < MNUM; ++k) Mu[k] = both(Mh[k]);
   double Mt[5];
   time_weights_rcp(inv_relax_time_rcp(d, prim, rc), dt, Mt);
   double *c = rec + FR_C;
   const double xk = Mxi[2] - kb * kb;
-  for (int side = 0; side < 2; ++side) {
-    double *ck = c + 5 * side;
-    ck[0] = Mt[1] * fma(0.5 * a[side].s3, kb, a[side].s0);
-    ck[1] = Mt[1] * a[side].s1;
-    ck[2] = Mt[1] * a[side].s2;
-    ck[3] = Mt[1] * (0.5 * a[side].s3);
-    ck[4] = Mt[1] * (0.5 * a[side].s3 * xk);
+  double *ck5 = c + 5 * side;
+  ck5[0] = Mt[1] * fma(0.5 * a.s3, kb, a.s0);
+  ck5[1] = Mt[1] * a.s1;
+  ck5[2] = Mt[1] * a.s2;
+  ck5[3] = Mt[1] * (0.5 * a.s3);
+  ck5[4] = Mt[1] * (0.5 * a.s3 * xk);
+  if (side == 0) {
+    const P4 aT = micro_slope_rcp(d.K, prim, rc, scale(-prim.s0, t1));
+    const P4 g0 = scale(prim.s0, add(add(scale(Mt[0], moment_uv(Mu, Mv, Mxi, 1, 0, 0)), scale(Mt[1], t2)),
+                                     scale(Mt[2], moment_au(aT, Mu, Mv, Mxi, 1, 0))));
+    c[10] = Mt[2] * fma(0.5 * aT.s3, kb, aT.s0) + Mt[0];
+    c[11] = Mt[2] * aT.s1;
+    c[12] = Mt[2] * aT.s2;
+    c[13] = Mt[2] * (0.5 * aT.s3);
+    c[14] = Mt[2] * (0.5 * aT.s3 * xk);
+    c[15] = Mt[0];
+    c[16] = Mt[3] * len;
+    c[17] = Mt[4] * len;
+    c[18] = len * g0.s0; c[19] = len * g0.s1; c[20] = len * g0.s2; c[21] = len * g0.s3;
+  } else {
+    // face heat flux (calcFaceQ, clUGKS.c:522-585): M's part and the deviation's,
+    // in the global frame, from their raw moments
+    const V2 qr = heat_flux_from_moments(R, d.K, Ug), qd_ = face_heat_flux(dm, nr_rcp(d.K), Ug);
+    const V2 Q = to_local(v2(qr.x + qd_.x, qr.y + qd_.y), n);
+    const double s0 = 0.8 * (1 - d.Pr) * (prim.s3 * prim.s3) * rc.rho;
+    rec[FR_UX] = prim.s1;
+    rec[FR_UY] = prim.s2;
+    rec[FR_LAM] = prim.s3;
+    rec[FR_KB] = kb;
+    rec[FR_SX] = (Mt[0] * s0) * Q.x;
+    rec[FR_SY] = (Mt[0] * s0) * Q.y;
+    rec[FR_LNP] = log((prim.s0 * prim.s3) / (ref.P0 * d.PI));  // ln(P / P0), P = rho lambda / pi
+    rec[FR_UGX] = Ug.x;
+    rec[FR_UGY] = Ug.y;
   }
-  double Mu[MNUM];
-#pragma unroll
-  for (int k = 0; k < MNUM; ++k) Mu[k] = Mh[0][k] + Mh[1][k];
-  const P4 aT = micro_slope_rcp(d.K, prim, rc, scale(-prim.s0, add(t1[0], t1[1])));
-  const P4 g0 = scale(prim.s0, add(add(scale(Mt[0], moment_uv(Mu, Mv, Mxi, 1, 0, 0)), scale(Mt[1], add(t2[0], t2[1]))),
-                                   scale(Mt[2], moment_au(aT, Mu, Mv, Mxi, 1, 0))));
-  c[10] = Mt[2] * fma(0.5 * aT.s3, kb, aT.s0) + Mt[0];
-  c[11] = Mt[2] * aT.s1;
-  c[12] = Mt[2] * aT.s2;
-  c[13] = Mt[2] * (0.5 * aT.s3);
-  c[14] = Mt[2] * (0.5 * aT.s3 * xk);
-  c[15] = Mt[0];
-  c[16] = Mt[3] * len;
-  c[17] = Mt[4] * len;
-  c[18] = len * g0.s0; c[19] = len * g0.s1; c[20] = len * g0.s2; c[21] = len * g0.s3;
-  const double s0 = 0.8 * (1 - d.Pr) * (prim.s3 * prim.s3) * rc.rho;
-  rec[FR_UX] = prim.s1;
-  rec[FR_UY] = prim.s2;
-  rec[FR_LAM] = prim.s3;
-  rec[FR_KB] = kb;
-  rec[FR_SX] = (Mt[0] * s0) * Q.x;
-  rec[FR_SY] = (Mt[0] * s0) * Q.y;
-  rec[FR_LNP] = log((prim.s0 * prim.s3) / (ref.P0 * d.PI));  // ln(P / P0), P = rho lambda / pi
-  rec[FR_UGX] = Ug.x;
-  rec[FR_UGY] = Ug.y;
 }
 
 // ---------------------------------------------------------------------------
@@ -393,8 +396,9 @@ constexpr size_t delta_ring_bytes() { return (size_t)DELTA_RING * ((FM == 1 ? 5 
 template <int FM, int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB) face_moments_warp(const ugks_fused_block *__restrict__ B, int nb,
                                                                     ugks_solve_state *__restrict__ solves,
-                                                                    int first, int count, int wstride) {
+                                                                    int first, int count, int wstride, int chained) {
   extern __shared__ double dyn[];
+  pdl_begin(chained);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = (int)blockIdx.x * WPC + warp;
   if (item >= count) return;
@@ -555,6 +559,7 @@ template <int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB) face_flux_tma(const ugks_fused_block *__restrict__ B, int nb,
                                                                 ugks_solve_state *__restrict__ solves,
                                                                 int n_faces, int wbytes) {
+  pdl_begin();
   extern __shared__ __align__(128) unsigned char dyn_b[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = (int)blockIdx.x * WPC + warp;
@@ -800,6 +805,7 @@ template <int MINB>
 __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                                    ugks_solve_state *__restrict__ solves,
                                                                    int n_cells, int wstride) {
+  pdl_begin();
   extern __shared__ double dyn[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   CellWork cw;
@@ -977,6 +983,7 @@ __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_delta(const 
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(FT) ghost_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                        ugks_solve_state *solves, int finish) {
+  pdl_begin();
   __shared__ double scratch[4 * (FT / 32)];
   finish_steps(solves, finish);
   const int w = blockIdx.x;

@@ -36,10 +36,6 @@ constexpr int FT = 128;  // threads per face / cell / ghost CTA
 // the ghost copies, issued before the first store (a store may alias a later
 // load, so the compiler keeps them in program order)
 constexpr int GHOST_U = 4;
-// mixed retry pass (wall faces, a CTA per face): narrow, FT threads per face,
-// or wide for velocity grids above RETRY_NARROW_NV nodes, whose shared memory
-// lets only two or three faces on an SM
-constexpr int RETRY_NARROW_MINB = 5, RETRY_NARROW_NV = 1800, RETRY_WIDE_NT = 256, RETRY_WIDE_MINB = 2;
 // Launch shapes a face-pass segment can run with (ugks_fused_sizes.seg_variant;
 // the tuner in pyugks_b200/tuner.py picks them by timing): variant 0 is the
 // default 1, 1..4 are (warps per CTA, CTAs per SM of the register budget).
@@ -87,6 +83,32 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 inline cudaStream_t S(void *s) { return reinterpret_cast<cudaStream_t>(s); }
+// Where a step's kernels are launched: a stream, and for steps of few faces
+// (`carve` > 0) programmatic launches that share one split of L1 and shared
+// memory, `carve` percent.  An SM changes that split only when it is idle, so a
+// kernel that starts beside its predecessor runs with the predecessor's, and with
+// one that suits neither the reconfiguration costs more than the early launch
+// gives.  On large grids each pass is better off with the split that fits it.
+struct StepStream {
+  cudaStream_t st;
+  int carve = 0;
+};
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, StepStream to, A... args) {
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attr[1].val.sharedMemCarveout = (unsigned)to.carve;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = to.st;
+  cfg.attrs = attr;
+  cfg.numAttrs = to.carve > 0 ? 2 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 inline int launch_status() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
@@ -135,6 +157,31 @@ __device__ __forceinline__ bool item_in_block(const ugks_fused_block &b, int w) 
       return __VA_ARGS__;                                                                                  \
     }                                                                                                      \
   } while (0)
+
+// Programmatic dependent launch (launch() below): the kernels of a step follow
+// one another with the next one's launch under way while its predecessor runs.
+// pdl_wait returns once the grids before this one are complete and their writes
+// visible; pdl_trigger lets the next grid's CTAs start (once every CTA of this
+// one has run it).  A kernel waits before it touches anything its predecessors
+// write.  The launches of a face pass depend on the step before, not on one
+// another: those after the first (`chained`) start at once, since the first has
+// waited before it let them start, and have one CTA more, which waits, so that
+// their completion stands for the first's.  (A wait at the end of the last working
+// CTA cost the mixed moments sweep 3%: no warp left before its CTA's last.)  Between the small kernels of a 24x24
+// cavity this replaces about 1 us of drain and launch per boundary.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_trigger();
+}
+__device__ __forceinline__ void pdl_begin(int chained) {
+  if (!chained) pdl_wait();
+  pdl_trigger();
+  if (!chained) return;
+  if (blockIdx.x == gridDim.x - 1) pdl_wait();
+  else __threadfence();  // acquire: nothing this SM cached before the first launch's wait
+}
 
 // dt update of updateTimeStep (ugks_sim.py:285-311) with limit = True
 __device__ __forceinline__ double limited_dt(double dt_old, double dt_new, double delta) {
@@ -244,7 +291,9 @@ __device__ __forceinline__ V2 heat_flux_from_moments(const double *M, double K, 
 
 // 1 / relaxTime
 __device__ __forceinline__ double inv_relax_time_rcp(const ugks_block_desc &d, P4 prim, Rcp r) {
-  const double p = pow(prim.s3, 1.0 - d.omega);
+  // lambda^(1 - omega) as exp((1 - omega) ln lambda): the exponent is of order 1,
+  // so its rounding stays within that of pow, in half of pow's dependent chain
+  const double p = exp((1.0 - d.omega) * log(prim.s3));
   double c = 1.0;
   switch (d.relax_type) {
     case 0: c = 0.79788456080286541; break;
@@ -1181,59 +1230,53 @@ __device__ __forceinline__ double2 *face_ring(double *dyn, int wstride, int warp
 template <int FM, int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB) face_pass_fp64(const ugks_fused_block *__restrict__ B, int nb,
                                                                  ugks_solve_state *__restrict__ solves, int n_wall,
-                                                                 int first, int count, int wstride) {
+                                                                 int first, int count, int wstride, int chained) {
   extern __shared__ double dyn[];
-  if ((int)blockIdx.x < n_wall) {
-    wall_work_fp64<WPC * 32>(B, nb, solves, (int)blockIdx.x, 0);
-    return;
-  }
+  pdl_begin(chained);
   const int warp = threadIdx.x >> 5;
   const int item = ((int)blockIdx.x - n_wall) * WPC + warp;
-  if (item >= count) return;
   FaceWork fwk;
-  if (!face_work<FM, true>(B, nb, solves, first + item, 0, fwk) || fwk.wall >= 0) return;
-  const ugks_fused_block &blk = B[fwk.bi];
-  face_item_fp64<FM>(blk, solves[blk.solve].dt, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
+  if ((int)blockIdx.x < n_wall) {
+    wall_work_fp64<WPC * 32>(B, nb, solves, (int)blockIdx.x, 0);
+  } else if (item < count && face_work<FM, true>(B, nb, solves, first + item, 0, fwk) && fwk.wall < 0) {
+    const ugks_fused_block &blk = B[fwk.bi];
+    face_item_fp64<FM>(blk, solves[blk.solve].dt, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
+  }
 }
 
-// the mixed path's face work item (ugks_delta.cuh, included further down):
-// WALLS, the wall faces (main pass: the wall launch; retry pass), else the
-// reconstruction and moments of the interior faces
-template <int FM, int NT, bool WALLS>
-__device__ __forceinline__ void face_item_delta(const ugks_fused_block *__restrict__ B, int nb,
-                                                ugks_solve_state *__restrict__ solves, const int w, int retry_pass);
-
-// the flux pass redone after a dt change (ugks_sim.py:432-441): RETRY_CTAS
-// CTAs per solve; a solve whose retry flag is clear costs one early exit each
-constexpr int RETRY_CTAS = 148;
-// the solve of a retry CTA of flux method FM, or false
-template <int FM>
+// the flux pass redone after a dt change (ugks_sim.py:432-441): some CTAs per
+// solve; a solve whose dt did not change costs one early exit each
+// (fewer for many solves: at least 8, 592 in all)
+inline int retry_ctas(int ns) { return std::max(8, std::min(148, 592 / std::max(ns, 1))); }
+// the solve of a retry CTA, or false
 __device__ __forceinline__ bool retry_solve(const ugks_fused_block *__restrict__ B,
-                                            const ugks_solve_state *__restrict__ solves, int ns, int &b0, int &bl) {
-  const int s = blockIdx.x / RETRY_CTAS;
+                                            const ugks_solve_state *__restrict__ solves, int ns, int per_solve, int &b0,
+                                            int &bl) {
+  const int s = blockIdx.x / per_solve;
   if (s >= ns) return false;
   const ugks_solve_state &x = solves[s];
   if (!x.active || x.nblocks <= 0 || !step_dt(x).retry) return false;
   b0 = x.first_block;
   bl = x.first_block + x.nblocks - 1;
-  return B[b0].d.flux_method == FM;
+  return true;
 }
 template <int FM, int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB) face_retry_fp64(const ugks_fused_block *__restrict__ B, int nb,
                                                                   ugks_solve_state *__restrict__ solves, int ns,
-                                                                  int wstride) {
+                                                                  int per_solve, int wstride) {
+  pdl_begin();
   extern __shared__ double dyn[];
   int b0, bl;
-  if (!retry_solve<FM>(B, solves, ns, b0, bl)) return;
-  const int r = blockIdx.x % RETRY_CTAS, warp = threadIdx.x >> 5;
+  if (!retry_solve(B, solves, ns, per_solve, b0, bl) || B[b0].d.flux_method != FM) return;
+  const int r = blockIdx.x % per_solve, warp = threadIdx.x >> 5;
   const ugks_block_desc &e = B[bl].d;
   const int wall_end = B[bl].wall_begin + 2 * (e.ni + e.nj);
-  for (int w = B[b0].wall_begin + r; w < wall_end; w += RETRY_CTAS) {
+  for (int w = B[b0].wall_begin + r; w < wall_end; w += per_solve) {
     wall_work_fp64<WPC * 32>(B, nb, solves, w, 1);
     __syncthreads();  // the next item reuses the shared tables
   }
   const int end = B[bl].face_begin + 2 * (e.ni + 1) * (e.nj + 1);
-  for (int w = B[b0].face_begin + r * WPC + warp; w < end; w += RETRY_CTAS * WPC) {
+  for (int w = B[b0].face_begin + r * WPC + warp; w < end; w += per_solve * WPC) {
     FaceWork fwk;
     if (!face_work<FM>(B, nb, solves, w, 1, fwk) || fwk.wall >= 0) continue;
     const ugks_fused_block &blk = B[fwk.bi];
@@ -1241,20 +1284,6 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_retry_fp64(const ugks_fus
                        fwk);
   }
 }
-// mixed: only the wall faces have anything to redo (the interior faces take the
-// dt after the first check)
-template <int FM, int MINB, int NT>
-__global__ void __launch_bounds__(NT, MINB) face_retry(const ugks_fused_block *__restrict__ B, int nb,
-                                                       ugks_solve_state *__restrict__ solves, int ns) {
-  int b0, bl;
-  if (!retry_solve<FM>(B, solves, ns, b0, bl)) return;
-  const int end = B[bl].face_begin + 2 * (B[bl].d.ni + 1) * (B[bl].d.nj + 1);
-  for (int w = B[b0].face_begin + blockIdx.x % RETRY_CTAS; w < end; w += RETRY_CTAS) {
-    face_item_delta<FM, NT, true>(B, nb, solves, w, 1);
-    __syncthreads();  // the next item reuses the shared tables
-  }
-}
-
 // ---------------------------------------------------------------------------
 // cell pass: calcQ (clKernel.c:480-543) + updateMacro (clUGKS.c:1158-1187) +
 // UGKS_update (clUGKS.c:1189-1257) + clFindDT (clKernel.c:224-308)
@@ -1366,6 +1395,7 @@ template <int MINB>
 __global__ void __launch_bounds__(CW * 32, MINB * 8 / CW) cell_pass_fp64(const ugks_fused_block *__restrict__ B, int nb,
                                                                 ugks_solve_state *__restrict__ solves, int n_cells,
                                                                 int wstride) {
+  pdl_begin();
   extern __shared__ double dyn[];
   using St = Store<double>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1510,7 +1540,10 @@ __device__ __forceinline__ void finish_step(ugks_solve_state &x) {
 __device__ __forceinline__ void finish_steps(ugks_solve_state *solves, int ns) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) finish_step(solves[s]);
 }
-__global__ void dt_update(ugks_solve_state *solves, int ns) { finish_steps(solves, ns); }
+__global__ void dt_update(ugks_solve_state *solves, int ns) {
+  pdl_begin();
+  finish_steps(solves, ns);
+}
 
 // ---------------------------------------------------------------------------
 // ghost pass (UGKSBlock.updateBC, ugks_block.py:621-665): one CTA per ghost
@@ -1519,6 +1552,7 @@ __global__ void dt_update(ugks_solve_state *solves, int ns) { finish_steps(solve
 template <typename T>
 __global__ void __launch_bounds__(FT) ghost_pass(const ugks_fused_block *__restrict__ B, int nb,
                                                  ugks_solve_state *solves, int finish) {
+  pdl_begin();
   __shared__ double scratch[4 * (FT / 32)];
   finish_steps(solves, finish);
   using St = Store<T>;
@@ -1814,13 +1848,12 @@ __global__ void dt_init(ugks_solve_state *solves, int ns) {
 // solves the end of their step
 template <typename T>
 void launch_ghosts(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves,
-                   int finish, cudaStream_t st) {
+                   int finish, StepStream st) {
   if (!z->n_ghost) {
-    if (finish) dt_update<<<(finish + 127) / 128, 128, 0, st>>>(solves, finish);
+    if (finish) launch(dt_update, (finish + 127) / 128, 128, 0, st, solves, finish);
     return;
   }
-  if (std::is_same<T, float>::value) ghost_pass_delta<<<z->n_ghost, FT, 0, st>>>(B, nb, solves, finish);
-  else ghost_pass<double><<<z->n_ghost, FT, 0, st>>>(B, nb, solves, finish);
+  launch(std::is_same<T, float>::value ? ghost_pass_delta : ghost_pass<double>, z->n_ghost, FT, 0, st, B, nb, solves, finish);
 }
 
 template <typename T>
@@ -1834,7 +1867,7 @@ int init_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     else init_cells<double><<<z->n_cells, FT, 0, st>>>(B, nb, solves);
   }
   dt_init<<<(ns + 127) / 128, 128, 0, st>>>(solves, ns);
-  launch_ghosts<T>(B, nb, z, solves, 0, st);
+  launch_ghosts<T>(B, nb, z, solves, 0, {st});
   return launch_status();
 }
 
@@ -1849,7 +1882,7 @@ int restart_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, u
     else restart_cells<double><<<z->n_cells, FT, 0, st>>>(B, nb, solves);
   }
   dt_init<<<(ns + 127) / 128, 128, 0, st>>>(solves, ns);
-  launch_ghosts<T>(B, nb, z, solves, 0, st);
+  launch_ghosts<T>(B, nb, z, solves, 0, {st});
   return launch_status();
 }
 
@@ -1879,14 +1912,9 @@ cudaError_t set_wall_attributes() {
       if (e != cudaSuccess) return e;
   }
   if constexpr (std::is_same<T, float>::value) {
-    // the wall launch and the retry pass's wall faces (both budgets)
-    constexpr int NN = FT, NW = RETRY_WIDE_NT, MN = RETRY_NARROW_MINB, MW = RETRY_WIDE_MINB;
-    cudaError_t r[7] = {allow_smem(wall_pass_delta<WALL_NT>), allow_smem(face_retry<0, MN, NN>),
-                        allow_smem(face_retry<1, MN, NN>), allow_smem(face_retry<3, MN, NN>),
-                        allow_smem(face_retry<0, MW, NW>), allow_smem(face_retry<1, MW, NW>),
-                        allow_smem(face_retry<3, MW, NW>)};
-    for (cudaError_t e : r)
-      if (e != cudaSuccess) return e;
+    const cudaError_t e = allow_smem(wall_pass_delta);
+    if (e != cudaSuccess) return e;
+    return allow_smem(wall_retry_delta);
   }
   return cudaSuccess;
 }
@@ -1926,12 +1954,12 @@ cudaError_t set_cell_attributes() {
 // once for each device a step runs on, with that device current.
 constexpr int kMaxDevices = 64;
 
-// The mixed step's wall launch needs only this step's f and writes only wall
-// faces, so it runs on a side stream beside the interior moments sweep: a
-// fork and a join by events, which stream capture turns into graph edges.
-// One side stream per device, created with the device's kernel attributes
-// (before any capture: ugks_prepare); `lock` keeps the record-wait pairs of
-// concurrent host threads from interleaving.
+// A large mixed step's wall launch runs on a side stream beside the moments sweep
+// (it needs only this step's f and writes only wall faces): a fork and a join by
+// events, which stream capture turns into graph edges.  One side stream per
+// device, created with the device's kernel attributes (before any capture:
+// ugks_prepare); `lock` keeps the record-wait pairs of concurrent host threads
+// from interleaving.
 struct WallStream {
   cudaStream_t s = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -1992,73 +2020,65 @@ size_t face_smem(int wstride) {
 // first segment's launch takes the wall faces of the whole table with it
 template <int WPC, int MINB>
 void launch_faces_shape(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall, int first,
-                        int count, int axes, cudaStream_t st) {
+                        int count, int axes, int chained, StepStream st) {
   const int ws = face_stride(axes);
-  const unsigned g = (unsigned)(n_wall + (count + WPC - 1) / WPC), t = WPC * 32;
+  const unsigned g = (unsigned)(n_wall + (count + WPC - 1) / WPC + chained), t = WPC * 32;
   switch (method) {
-    case 0: face_pass_fp64<0, WPC, MINB><<<g, t, face_smem<0, WPC>(ws), st>>>(B, nb, solves, n_wall, first, count, ws); break;
-    case 1: face_pass_fp64<1, WPC, MINB><<<g, t, face_smem<1, WPC>(ws), st>>>(B, nb, solves, n_wall, first, count, ws); break;
-    case 3: face_pass_fp64<3, WPC, MINB><<<g, t, face_smem<3, WPC>(ws), st>>>(B, nb, solves, n_wall, first, count, ws); break;
+    case 0: launch(face_pass_fp64<0, WPC, MINB>, g, t, face_smem<0, WPC>(ws), st, B, nb, solves, n_wall, first, count, ws, chained); break;
+    case 1: launch(face_pass_fp64<1, WPC, MINB>, g, t, face_smem<1, WPC>(ws), st, B, nb, solves, n_wall, first, count, ws, chained); break;
+    case 3: launch(face_pass_fp64<3, WPC, MINB>, g, t, face_smem<3, WPC>(ws), st, B, nb, solves, n_wall, first, count, ws, chained); break;
     default: break;
   }
 }
 inline void launch_faces(int v, const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall,
-                         int first, int count, int axes, cudaStream_t st) {
+                         int first, int count, int axes, int chained, StepStream st) {
   switch (v) {
-    case 2: launch_faces_shape<FaceShape<2>::wpc, FaceShape<2>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
-    case 3: launch_faces_shape<FaceShape<3>::wpc, FaceShape<3>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
-    case 4: launch_faces_shape<FaceShape<4>::wpc, FaceShape<4>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
-    default: launch_faces_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, solves, method, n_wall, first, count, axes, st); break;
+    case 2: launch_faces_shape<FaceShape<2>::wpc, FaceShape<2>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
+    case 3: launch_faces_shape<FaceShape<3>::wpc, FaceShape<3>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
+    case 4: launch_faces_shape<FaceShape<4>::wpc, FaceShape<4>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
+    default: launch_faces_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
   }
 }
 
 // the retry pass of every flux method (per solve; rare)
 template <typename T>
 void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves, int ns,
-                  cudaStream_t st) {
-  const unsigned rg = (unsigned)ns * RETRY_CTAS;
+                  StepStream st) {
+  const int per = retry_ctas(ns);
+  const unsigned rg = (unsigned)ns * per;
   if constexpr (std::is_same<T, float>::value) {
-    const size_t sm = delta_wall_smem(z->max_nv);
-    constexpr int NN = FT, NW = RETRY_WIDE_NT, MN = RETRY_NARROW_MINB, MW = RETRY_WIDE_MINB;
-    if (z->max_nv <= RETRY_NARROW_NV) {
-      if (z->face_count[0]) face_retry<0, MN, NN><<<rg, NN, sm, st>>>(B, nb, solves, ns);
-      if (z->face_count[1]) face_retry<1, MN, NN><<<rg, NN, sm, st>>>(B, nb, solves, ns);
-      if (z->face_count[3]) face_retry<3, MN, NN><<<rg, NN, sm, st>>>(B, nb, solves, ns);
-    } else {
-      if (z->face_count[0]) face_retry<0, MW, NW><<<rg, NW, sm, st>>>(B, nb, solves, ns);
-      if (z->face_count[1]) face_retry<1, MW, NW><<<rg, NW, sm, st>>>(B, nb, solves, ns);
-      if (z->face_count[3]) face_retry<3, MW, NW><<<rg, NW, sm, st>>>(B, nb, solves, ns);
-    }
+    // only the wall faces have anything to redo
+    if (z->n_wall) launch(wall_retry_delta, rg, WALL_NT, delta_wall_smem(z->max_nv), st, B, nb, solves, ns, per);
   } else {
     constexpr int WPC = FaceShape<1>::wpc, MINB = FaceShape<1>::minb, NT = WPC * 32;
     const int ws = face_stride(z->max_axes);
-    if (z->face_count[0]) face_retry_fp64<0, WPC, MINB><<<rg, NT, face_smem<0, WPC>(ws), st>>>(B, nb, solves, ns, ws);
-    if (z->face_count[1]) face_retry_fp64<1, WPC, MINB><<<rg, NT, face_smem<1, WPC>(ws), st>>>(B, nb, solves, ns, ws);
-    if (z->face_count[3]) face_retry_fp64<3, WPC, MINB><<<rg, NT, face_smem<3, WPC>(ws), st>>>(B, nb, solves, ns, ws);
+    if (z->face_count[0]) launch(face_retry_fp64<0, WPC, MINB>, rg, NT, face_smem<0, WPC>(ws), st, B, nb, solves, ns, per, ws);
+    if (z->face_count[1]) launch(face_retry_fp64<1, WPC, MINB>, rg, NT, face_smem<1, WPC>(ws), st, B, nb, solves, ns, per, ws);
+    if (z->face_count[3]) launch(face_retry_fp64<3, WPC, MINB>, rg, NT, face_smem<3, WPC>(ws), st, B, nb, solves, ns, per, ws);
   }
 }
 
 // the mixed moments sweep of one segment, in launch shape v (ugks_fused_sizes.seg_variant)
 template <int WPC, int MINB>
 void launch_moments_shape(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int first,
-                          int count, int axes, cudaStream_t st) {
+                          int count, int axes, int chained, StepStream st) {
   const int ws = delta_moments_stride(axes);
-  const unsigned g = (unsigned)((count + WPC - 1) / WPC);
+  const unsigned g = (unsigned)((count + WPC - 1) / WPC + chained);
   const size_t sm = (size_t)WPC * ws * sizeof(double);
   switch (method) {
-    case 0: face_moments_warp<0, WPC, MINB><<<g, WPC * 32, sm + WPC * delta_ring_bytes<0>(), st>>>(B, nb, solves, first, count, ws); break;
-    case 1: face_moments_warp<1, WPC, MINB><<<g, WPC * 32, sm + WPC * delta_ring_bytes<1>(), st>>>(B, nb, solves, first, count, ws); break;
-    case 3: face_moments_warp<3, WPC, MINB><<<g, WPC * 32, sm + WPC * delta_ring_bytes<3>(), st>>>(B, nb, solves, first, count, ws); break;
+    case 0: launch(face_moments_warp<0, WPC, MINB>, g, WPC * 32, sm + WPC * delta_ring_bytes<0>(), st, B, nb, solves, first, count, ws, chained); break;
+    case 1: launch(face_moments_warp<1, WPC, MINB>, g, WPC * 32, sm + WPC * delta_ring_bytes<1>(), st, B, nb, solves, first, count, ws, chained); break;
+    case 3: launch(face_moments_warp<3, WPC, MINB>, g, WPC * 32, sm + WPC * delta_ring_bytes<3>(), st, B, nb, solves, first, count, ws, chained); break;
     default: break;
   }
 }
 inline void launch_moments(int v, const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method,
-                           int first, int count, int axes, cudaStream_t st) {
+                           int first, int count, int axes, int chained, StepStream st) {
   switch (v) {
-    case 2: launch_moments_shape<MomentsShape<2>::wpc, MomentsShape<2>::minb>(B, nb, solves, method, first, count, axes, st); break;
-    case 3: launch_moments_shape<MomentsShape<3>::wpc, MomentsShape<3>::minb>(B, nb, solves, method, first, count, axes, st); break;
-    case 4: launch_moments_shape<MomentsShape<4>::wpc, MomentsShape<4>::minb>(B, nb, solves, method, first, count, axes, st); break;
-    default: launch_moments_shape<MomentsShape<1>::wpc, MomentsShape<1>::minb>(B, nb, solves, method, first, count, axes, st); break;
+    case 2: launch_moments_shape<MomentsShape<2>::wpc, MomentsShape<2>::minb>(B, nb, solves, method, first, count, axes, chained, st); break;
+    case 3: launch_moments_shape<MomentsShape<3>::wpc, MomentsShape<3>::minb>(B, nb, solves, method, first, count, axes, chained, st); break;
+    case 4: launch_moments_shape<MomentsShape<4>::wpc, MomentsShape<4>::minb>(B, nb, solves, method, first, count, axes, chained, st); break;
+    default: launch_moments_shape<MomentsShape<1>::wpc, MomentsShape<1>::minb>(B, nb, solves, method, first, count, axes, chained, st); break;
   }
 }
 
@@ -2071,10 +2091,25 @@ struct NvtxRange {
   NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
+// The line between the two ways to launch a step.  A boundary saves about 2 us
+// whatever the work; the shared split costs a share of the passes it fits less
+// well.  Mixed: by work, faces times velocities.  FP64: up to as many cells as the
+// cell pass holds in one wave of the 3 CTAs an SM has with that split (4 with its
+// own).  Step in us without and with programmatic launches, square cavities (cells
+// a side, velocities): mixed 24, 17^2 (0.4 M) 55.6 and 42.9; 56, 25^2 (4.1 M) 126
+// and 113; 80, 25^2 (8.2 M) 193 and 184; 62, 33^2 (8.6 M) 190 and 182; 88, 33^2
+// (17 M) 339 and 355.  FP64 24, 17^2 45.4 and 41.3; 40, 25^2 91.1 and 83.6; 36,
+// 41^2 203 and 200; 44, 33^2 157 and 183; 63, 33^2 293 and 310.
+template <typename T>
+inline StepStream step_stream(cudaStream_t st, const ugks_fused_sizes *z) {
+  if (std::is_same<T, float>::value) return {st, (double)z->n_faces * z->max_nv <= 1e7 ? 70 : 0};
+  return {st, z->n_cells <= 3 * 148 * CW ? 50 : 0};
+}
+
 template <typename T>
 int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves,
               int ns, void *stream, void *const *events = nullptr) {
-  cudaStream_t st = S(stream);
+  const StepStream st = step_stream<T>(S(stream), z);
   // cell pass: the axis factor tables of the old and new macro state
   constexpr bool mixed = std::is_same<T, float>::value;
   // doubles of shared memory per cell warp
@@ -2084,26 +2119,34 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   if (attr != cudaSuccess) return -(int)attr;
   if (face_limit_bytes<T>(z->max_nv, z->max_axes) > 200 * 1024 || csmem > 200 * 1024) return -(int)cudaErrorInvalidValue;
   auto mark = [&](int k) {
-    if (events && events[k]) cudaEventRecord(reinterpret_cast<cudaEvent_t>(events[k]), st);
+    if (events && events[k]) cudaEventRecord(reinterpret_cast<cudaEvent_t>(events[k]), st.st);
   };
   // NVTX: the step, and within it the face, cell and ghost phases
   NvtxRange step_range(mixed ? "ugks step (mixed)" : "ugks step (fp64)");
   std::optional<NvtxRange> phase;
   phase.emplace("ugks face pass");
   mark(0);
-  // mixed: the wall faces on the device's side stream, beside the segments
+  // the launches of the face pass depend only on the step before: of programmatic
+  // ones all but the first are chained.  Mixed: the wall faces first, beside which
+  // the moments run, chained or from the side stream
+  int chained = 0;
   WallStream *ws = nullptr;
   std::unique_lock<std::mutex> ws_guard;
   if (mixed && z->n_wall) {
-    int dev = 0;
-    const cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return -(int)e;
-    ws = &wall_stream(dev);
-    ws_guard = std::unique_lock<std::mutex>(ws->lock);
-    cudaEventRecord(ws->fork, st);
-    cudaStreamWaitEvent(ws->s, ws->fork, 0);
-    wall_pass_delta<WALL_NT><<<(unsigned)z->n_wall, WALL_NT, delta_wall_smem(z->max_nv), ws->s>>>(B, nb, solves);
-    cudaEventRecord(ws->join, ws->s);
+    StepStream to = st;
+    if (!st.carve) {
+      int dev = 0;
+      const cudaError_t e = cudaGetDevice(&dev);
+      if (e != cudaSuccess) return -(int)e;
+      ws = &wall_stream(dev);
+      ws_guard = std::unique_lock<std::mutex>(ws->lock);
+      cudaEventRecord(ws->fork, st.st);
+      cudaStreamWaitEvent(ws->s, ws->fork, 0);
+      to = {ws->s};
+    }
+    launch(wall_pass_delta, z->n_wall, WALL_NT, delta_wall_smem(z->max_nv), to, B, nb, solves);
+    if (ws) cudaEventRecord(ws->join, ws->s);
+    chained = st.carve > 0;
   }
   int walls = z->n_wall;
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) {
@@ -2112,14 +2155,15 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     const int m = z->seg_method[k], b0 = z->seg_begin[k], n = z->seg_count[k];
     if (v <= 0 || v > 4) v = 1;
     if constexpr (mixed) {
-      launch_moments(v, B, nb, solves, m, b0, n, z->seg_max_axes[k], st);
+      launch_moments(v, B, nb, solves, m, b0, n, z->seg_max_axes[k], chained, st);
     } else {
-      launch_faces(v, B, nb, solves, m, walls, b0, n, z->seg_max_axes[k], st);
+      launch_faces(v, B, nb, solves, m, walls, b0, n, z->seg_max_axes[k], chained, st);
       walls = 0;
     }
+    chained = st.carve > 0;
   }
   if (ws) {
-    cudaStreamWaitEvent(st, ws->join, 0);
+    cudaStreamWaitEvent(st.st, ws->join, 0);
     ws_guard.unlock();
   }
   // mixed: the interior faces' coefficient and flux launches take the dt of the
@@ -2130,10 +2174,10 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   }
   launch_retry<T>(B, nb, z, solves, ns, st);
   if (mixed && z->n_faces) {
-    face_coef_delta<<<(unsigned)((z->n_faces + 127) / 128), 128, 0, st>>>(B, nb, solves, z->n_faces);
+    launch(face_coef_delta, (unsigned)((2l * z->n_faces + COEF_NT - 1) / COEF_NT), COEF_NT, 0, st, B, nb, solves, z->n_faces);
     const int wb = (int)flux_tma_warp_bytes(z->max_axes);
-    face_flux_tma<FLUX_WPC, FLUX_TMA_MINB><<<(unsigned)((z->n_faces + FLUX_WPC - 1) / FLUX_WPC), FLUX_WPC * 32,
-                                             (size_t)FLUX_WPC * wb, st>>>(B, nb, solves, z->n_faces, wb);
+    launch(face_flux_tma<FLUX_WPC, FLUX_TMA_MINB>, (unsigned)((z->n_faces + FLUX_WPC - 1) / FLUX_WPC), FLUX_WPC * 32,
+           (size_t)FLUX_WPC * wb, st, B, nb, solves, z->n_faces, wb);
   }
   if (mixed) {
     mark(1);
@@ -2147,13 +2191,8 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     // cell_variant: 0 the default register budget, 2 or 3 times 8 warps per SM
     const unsigned cg = (unsigned)((z->n_cells + CW - 1) / CW);
     const int cv = z->cell_variant == 2 || z->cell_variant == 3 ? z->cell_variant : CELL_MINB;
-    if (mixed) {
-      if (cv == 3) cell_pass_delta<3><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
-      else cell_pass_delta<2><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
-    } else {
-      if (cv == 3) cell_pass_fp64<3><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
-      else cell_pass_fp64<2><<<cg, CW * 32, csmem, st>>>(B, nb, solves, z->n_cells, cstride);
-    }
+    if (mixed) launch(cv == 3 ? cell_pass_delta<3> : cell_pass_delta<2>, cg, CW * 32, csmem, st, B, nb, solves, z->n_cells, cstride);
+    else launch(cv == 3 ? cell_pass_fp64<3> : cell_pass_fp64<2>, cg, CW * 32, csmem, st, B, nb, solves, z->n_cells, cstride);
   }
   mark(5);
   phase.reset();
@@ -2186,6 +2225,7 @@ constexpr int RES_NT = 1024;
 template <bool STOP>
 __global__ void __launch_bounds__(RES_NT) residual_kernel(const ugks_fused_block *B, int nb, ugks_solve_state *solves,
                                                           int ns) {
+  pdl_begin();
   __shared__ double scratch[8 * (RES_NT / 32)];
   const int s = blockIdx.x;
   if (s >= ns || !solves[s].active) return;  // a stopped solve keeps its last residual
@@ -2274,7 +2314,8 @@ int ugks_step_launches(const ugks_fused_sizes *z, int mixed) {
   if (mixed && z->n_faces) n += 2;  // the mixed face pass's coefficient and flux launches
   if (mixed && z->n_wall) n += 1;   // and its wall launch
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) n += z->seg_count[k] > 0 ? 1 : 0;
-  for (int m = 0; m < 4; ++m) n += z->face_count[m] > 0 ? 1 : 0;  // retry passes
+  if (mixed) n += z->n_wall ? 1 : 0;  // retry pass (mixed: walls)
+  else for (int m = 0; m < 4; ++m) n += z->face_count[m] > 0 ? 1 : 0;
   n += z->n_cells ? 1 : 0;
   n += 1;                                                          // ghost pass (or the dt update alone)
   return n;
@@ -2283,7 +2324,7 @@ int ugks_step_launches(const ugks_fused_sizes *z, int mixed) {
 int ugks_residual(const ugks_fused_block *blocks_dev, int nblocks, ugks_solve_state *solves_dev,
                   int nsolves, void *stream) {
   if (nsolves <= 0) return 0;
-  residual_kernel<false><<<nsolves, RES_NT, 0, S(stream)>>>(blocks_dev, nblocks, solves_dev, nsolves);
+  launch(residual_kernel<false>, nsolves, RES_NT, 0, {S(stream)}, blocks_dev, nblocks, solves_dev, nsolves);
   return launch_status();
 }
 
@@ -2295,11 +2336,12 @@ int ugks_stop_check(ugks_solve_state *solves_dev, int nsolves, void *stream) {
 
 int ugks_serve_steps(int mixed, const ugks_fused_block *blocks_dev, int nblocks, const ugks_fused_sizes *sizes,
                      ugks_solve_state *solves_dev, int nsolves, int nsteps, void *stream) {
+  const StepStream st = mixed ? step_stream<float>(S(stream), sizes) : step_stream<double>(S(stream), sizes);
   for (int k = 0; k < nsteps; ++k) {
     int rc = mixed ? step_impl<float>(blocks_dev, nblocks, sizes, solves_dev, nsolves, stream)
                    : step_impl<double>(blocks_dev, nblocks, sizes, solves_dev, nsolves, stream);
     if (rc == 0 && nsolves > 0) {
-      residual_kernel<true><<<nsolves, RES_NT, 0, S(stream)>>>(blocks_dev, nblocks, solves_dev, nsolves);
+      launch(residual_kernel<true>, nsolves, RES_NT, 0, st, blocks_dev, nblocks, solves_dev, nsolves);
       rc = launch_status();
     }
     if (rc != 0) return rc;
