@@ -84,14 +84,19 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 inline cudaStream_t S(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 // Where a step's kernels are launched: a stream, and for steps of few faces
-// (`carve` > 0) programmatic launches that share one split of L1 and shared
+// (`carve` > 0) programmatic launches, that share one split of L1 and shared
 // memory, `carve` percent.  An SM changes that split only when it is idle, so a
 // kernel that starts beside its predecessor runs with the predecessor's, and with
 // one that suits neither the reconfiguration costs more than the early launch
 // gives.  On large grids each pass is better off with the split that fits it.
+// There only the launches of a face pass after its first are programmatic
+// (`chained`): they fill the SMs that the last CTAs of the one before leave idle
+// (16 cavities of eight velocity grids and limiters, step in us without and with:
+// FP64 7029 and 6430, mixed 3934 and 3900).
 struct StepStream {
   cudaStream_t st;
   int carve = 0;
+  bool chained = false;
 };
 template <typename... P, typename... A>
 void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, StepStream to, A... args) {
@@ -106,7 +111,7 @@ void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, St
   cfg.dynamicSmemBytes = smem;
   cfg.stream = to.st;
   cfg.attrs = attr;
-  cfg.numAttrs = to.carve > 0 ? 2 : 0;
+  cfg.numAttrs = to.carve > 0 ? 2 : to.chained ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 inline int launch_status() {
@@ -2126,9 +2131,9 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   std::optional<NvtxRange> phase;
   phase.emplace("ugks face pass");
   mark(0);
-  // the launches of the face pass depend only on the step before: of programmatic
-  // ones all but the first are chained.  Mixed: the wall faces first, beside which
-  // the moments run, chained or from the side stream
+  // the launches of the face pass depend only on the step before: all but the
+  // first are chained.  Mixed: the wall faces first, beside which the moments run,
+  // chained or, on large tables, with the wall faces on the side stream
   int chained = 0;
   WallStream *ws = nullptr;
   std::unique_lock<std::mutex> ws_guard;
@@ -2152,15 +2157,17 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) {
     if (z->seg_count[k] <= 0) continue;
     int v = z->seg_variant[k];
+    StepStream to = st;
+    to.chained = chained;
     const int m = z->seg_method[k], b0 = z->seg_begin[k], n = z->seg_count[k];
     if (v <= 0 || v > 4) v = 1;
     if constexpr (mixed) {
-      launch_moments(v, B, nb, solves, m, b0, n, z->seg_max_axes[k], chained, st);
+      launch_moments(v, B, nb, solves, m, b0, n, z->seg_max_axes[k], chained, to);
     } else {
-      launch_faces(v, B, nb, solves, m, walls, b0, n, z->seg_max_axes[k], chained, st);
+      launch_faces(v, B, nb, solves, m, walls, b0, n, z->seg_max_axes[k], chained, to);
       walls = 0;
     }
-    chained = st.carve > 0;
+    chained = 1;
   }
   if (ws) {
     cudaStreamWaitEvent(st.st, ws->join, 0);
