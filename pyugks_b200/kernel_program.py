@@ -16,6 +16,8 @@ from __future__ import annotations
 
 import ctypes as C
 
+import torch
+
 from . import _lib
 
 
@@ -40,32 +42,34 @@ class KernelProgram:
         fn = getattr(self._lib, "ugks_" + name)
         sig = _lib.KERNEL_SIGNATURES[name]
         desc = C.byref(self.desc)
+        count = len(sig)
+
+        def pointer(a):
+            if not a.is_cuda or not a.is_contiguous():
+                raise ValueError("%s: buffers must be contiguous CUDA tensors" % name)
+            return a.data_ptr()
+
+        convert = [pointer if k == "p" else int if k == "i" else float for k in sig]
 
         def call(queue, global_size, local_size, *args):
-            if len(args) != len(sig):
-                raise TypeError("%s takes %d kernel arguments, got %d" % (name, len(sig), len(args)))
-            conv = []
-            for k, a in zip(sig, args):
-                if k == "p":
-                    if not a.is_cuda or not a.is_contiguous():
-                        raise ValueError("%s: buffers must be contiguous CUDA tensors" % name)
-                    conv.append(a.data_ptr())
-                elif k == "i":
-                    conv.append(int(a))
-                else:
-                    conv.append(float(a))
+            if len(args) != count:
+                raise TypeError("%s takes %d kernel arguments, got %d" % (name, count, len(args)))
+            conv = [f(a) for f, a in zip(convert, args)]
             g0 = int(global_size[0])
             g1 = int(global_size[1]) if len(global_size) > 1 else 1
-            _lib.check(fn(desc, g0, g1, *conv, _stream_ptr(queue)), name)
+            rc = fn(desc, g0, g1, *conv, _stream_ptr(queue))
+            if rc:
+                _lib.check(rc, name)
 
         call.__name__ = name
         return call
 
 
 def _stream_ptr(queue):
-    import torch
     if queue is None:
-        return torch.cuda.current_stream().cuda_stream
+        # the current device's current stream, without the Stream object that
+        # torch.cuda.current_stream() makes (13 us of a 26 us call)
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     if isinstance(queue, int):
         return queue
     return queue.cuda_stream
