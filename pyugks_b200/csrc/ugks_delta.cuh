@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_moments_warp(const ugks_f
                                                                     ugks_solve_state *__restrict__ solves,
                                                                     int first, int count, int wstride, int chained) {
   extern __shared__ double dyn[];
-  pdl_begin(chained);
+  pdl_begin_face(chained);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = (int)blockIdx.x * WPC + warp;
   if (item >= count) return;

@@ -20,6 +20,20 @@ constexpr int BC_ADJACENT = 0, BC_EXTRAPOLATE_OUT = 1, BC_CONSTANT = 2, BC_REFLE
               BC_ADSORBING = 8, BC_BOUNCE_BACK = 9;
 constexpr int MNUM = 7, MTUM = 5;
 
+// Programmatic dependent launch: kernels that follow one another on a stream, with
+// the next one's launch under way while its predecessor runs.  pdl_wait returns
+// once the grids before this one are complete and their writes visible;
+// pdl_trigger lets the next grid's CTAs start (once every CTA of this one has run
+// it).  A kernel waits before it touches anything its predecessors write; launched
+// plainly it returns from the wait at once.  Between the small kernels of a 24x24
+// cavity this takes out about 2 us of drain and launch per boundary.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_trigger();
+}
+
 struct V2 { double x, y; };
 // (rho, U, V, lambda) or conserved (rho, rho U, rho V, E)
 struct P4 { double s0, s1, s2, s3; };

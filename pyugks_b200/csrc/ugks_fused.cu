@@ -163,24 +163,12 @@ __device__ __forceinline__ bool item_in_block(const ugks_fused_block &b, int w) 
     }                                                                                                      \
   } while (0)
 
-// Programmatic dependent launch (launch() below): the kernels of a step follow
-// one another with the next one's launch under way while its predecessor runs.
-// pdl_wait returns once the grids before this one are complete and their writes
-// visible; pdl_trigger lets the next grid's CTAs start (once every CTA of this
-// one has run it).  A kernel waits before it touches anything its predecessors
-// write.  The launches of a face pass depend on the step before, not on one
-// another: those after the first (`chained`) start at once, since the first has
-// waited before it let them start, and have one CTA more, which waits, so that
-// their completion stands for the first's.  (A wait at the end of the last working
-// CTA cost the mixed moments sweep 3%: no warp left before its CTA's last.)  Between the small kernels of a 24x24
-// cavity this replaces about 1 us of drain and launch per boundary.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_begin() {
-  pdl_wait();
-  pdl_trigger();
-}
-__device__ __forceinline__ void pdl_begin(int chained) {
+// The launches of a face pass depend on the step before, not on one another: those
+// after the first (`chained`) start at once, since the first has waited before it
+// let them start, and have one CTA more, which waits, so that their completion
+// stands for the first's.  (A wait at the end of the last working CTA cost the
+// mixed moments sweep 3%: no warp left before its CTA's last.)
+__device__ __forceinline__ void pdl_begin_face(int chained) {
   if (!chained) pdl_wait();
   pdl_trigger();
   if (!chained) return;
@@ -1237,7 +1225,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_pass_fp64(const ugks_fuse
                                                                  ugks_solve_state *__restrict__ solves, int n_wall,
                                                                  int first, int count, int wstride, int chained) {
   extern __shared__ double dyn[];
-  pdl_begin(chained);
+  pdl_begin_face(chained);
   const int warp = threadIdx.x >> 5;
   const int item = ((int)blockIdx.x - n_wall) * WPC + warp;
   FaceWork fwk;

@@ -24,6 +24,20 @@ inline int launch_status() {
   return e == cudaSuccess ? 0 : -(int)e;
 }
 inline cudaStream_t S(void *s) { return reinterpret_cast<cudaStream_t>(s); }
+// programmatic launch: every kernel here waits for its predecessor itself
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), unsigned grid, unsigned block, void *stream, const A &...args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = S(stream);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 inline unsigned grid_of(size_t g0, size_t g1) { return (unsigned)(g0 * g1); }
 inline unsigned grid_threads(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -45,6 +59,7 @@ __global__ void __launch_bounds__(VT) k_iFace(ugks_block_desc d, size_t g1, cons
                                               double *iface_f, double *fsigma,
                                               const double *centre, const double *mid_side,
                                               const double *normal, int face) {
+  pdl_begin();
   size_t mi, mj;
   work_group(g1, mi, mj);
   if (!(((face == SOUTH) && (mi < (size_t)d.ni) && (mj < (size_t)d.nj + 1)) ||
@@ -116,6 +131,7 @@ __device__ __forceinline__ P4 frame_moments(const ugks_block_desc &d, const doub
 __global__ void __launch_bounds__(VT) k_face_moments(ugks_block_desc d, size_t g1, const double *f,
                                                      const double *normal, int face, double *out,
                                                      int off_bot, int off_top, int which) {
+  pdl_begin();
   __shared__ double scratch[4 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -134,6 +150,7 @@ __global__ void __launch_bounds__(VT) k_face_moments(ugks_block_desc d, size_t g
 __global__ void k_getPLR(ugks_block_desc d, size_t g0, size_t g1, const double *centre,
                          const double *mid_side, int face, double *primary, double *gaL,
                          double *gaR, int off_bot, int off_top) {
+  pdl_begin();
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= g0 * g1) return;
   size_t mi = t / g1 + face * off_bot, mj = t % g1 + (1 - face) * off_bot;
@@ -173,6 +190,7 @@ __global__ void k_initMacroFlux(ugks_block_desc d, size_t g0, size_t g1, double 
                                 int face, double dt, const double *primary, const double *gaL,
                                 const double *gaR, double *gaT, double *gMxi, int off_bot,
                                 int off_top) {
+  pdl_begin();
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= g0 * g1) return;
   size_t mi = t / g1 + face * off_bot, mj = t % g1 + (1 - face) * off_bot;
@@ -196,6 +214,7 @@ __global__ void k_initMacroFlux(ugks_block_desc d, size_t g0, size_t g1, double 
 __global__ void __launch_bounds__(VT) k_calcFaceQ(ugks_block_desc d, size_t g1, const double *iface_f,
                                                   const double *primary, const double *normal,
                                                   double *faceQ, int face, int off_bot, int off_top) {
+  pdl_begin();
   __shared__ double scratch[2 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -221,6 +240,7 @@ __global__ void __launch_bounds__(VT) k_macroFlux(ugks_block_desc d, size_t g1, 
                                                   const double *normal, const double *side_length,
                                                   int face, double dt, const double *primary,
                                                   const double *faceQ, int off_bot, int off_top) {
+  pdl_begin();
   __shared__ double scratch[4 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -283,6 +303,7 @@ __global__ void __launch_bounds__(VT) k_distFlux(ugks_block_desc d, size_t g1, d
                                                  const double *gaR, const double *gaT,
                                                  const double *gMxi, const double *faceQ,
                                                  int off_bot, int off_top) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   size_t mi = a + face * off_bot, mj = b + (1 - face) * off_bot;
@@ -325,6 +346,7 @@ __global__ void __launch_bounds__(VT) k_accommodatingWallDist(ugks_block_desc d,
                                                               const double *normal, int face,
                                                               const double *wall_prop,
                                                               double *flux_f) {
+  pdl_begin();
   __shared__ double scratch[2 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -360,6 +382,7 @@ __global__ void __launch_bounds__(VT) k_accommodatingWallDist(ugks_block_desc d,
 __global__ void __launch_bounds__(VT) k_wallFlux(ugks_block_desc d, size_t g1, const double *normal,
                                                  const double *side_length, int face,
                                                  double *flux_f, double *flux_macro, double dt) {
+  pdl_begin();
   __shared__ double scratch[4 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -391,6 +414,7 @@ __global__ void __launch_bounds__(VT) k_wallMassEnergyFluxes(ugks_block_desc d, 
                                                              const double *normal, int face,
                                                              const double *flux_f,
                                                              double *wall_flux) {
+  pdl_begin();
   __shared__ double scratch[8 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -424,6 +448,7 @@ __global__ void __launch_bounds__(VT) k_wallMassEnergyFluxes(ugks_block_desc d, 
 __global__ void k_updateMacro(ugks_block_desc d, size_t g0, size_t g1, const double *fmS,
                               const double *fmW, const double *area, double *macro,
                               double *residual) {
+  pdl_begin();
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= g0 * g1) return;
   size_t mi = t / g1, mj = t % g1;
@@ -445,6 +470,7 @@ __global__ void __launch_bounds__(VT) k_UGKS_update(ugks_block_desc d, size_t g1
                                                     const double *area, const double *macro,
                                                     const double *gQ, const double *residual,
                                                     double dt, double *flag) {
+  pdl_begin();
   size_t mi, mj;
   work_group(g1, mi, mj);
   long gi = mi + d.ghost, gj = mj + d.ghost;
@@ -475,6 +501,7 @@ __global__ void __launch_bounds__(VT) k_UGKS_update(ugks_block_desc d, size_t g1
 
 __global__ void k_getResidual(ugks_block_desc d, size_t g0, size_t g1, const double *macro,
                               double *residual) {
+  pdl_begin();
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= g0 * g1) return;
   size_t mi = t / g1, mj = t % g1;
@@ -488,6 +515,7 @@ __global__ void k_getResidual(ugks_block_desc d, size_t g0, size_t g1, const dou
 __global__ void k_edgeMassFlow(ugks_block_desc d, size_t g0, const double *macro,
                                const double *normal, const double *side_length, double *mdot,
                                int this_face) {
+  pdl_begin();
   size_t ci = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (ci >= g0) return;
   long mi, mj, gi, gj;
@@ -505,6 +533,7 @@ __global__ void k_edgeMassFlow(ugks_block_desc d, size_t g0, const double *macro
 
 __global__ void __launch_bounds__(VT) k_calcQ(ugks_block_desc d, size_t g1, const double *Fin,
                                               const double *macro, double *gQ) {
+  pdl_begin();
   __shared__ double scratch[2 * VT / 32];
   size_t mi, mj;
   work_group(g1, mi, mj);
@@ -525,6 +554,7 @@ __global__ void __launch_bounds__(VT) k_calcQ(ugks_block_desc d, size_t g1, cons
 
 __global__ void __launch_bounds__(VT) k_calcMacro(ugks_block_desc d, size_t g1, const double *Fin,
                                                   double *macro) {
+  pdl_begin();
   __shared__ double scratch[4 * VT / 32];
   size_t mi, mj;
   work_group(g1, mi, mj);
@@ -545,6 +575,7 @@ __global__ void __launch_bounds__(VT) k_calcMacro(ugks_block_desc d, size_t g1, 
 
 __global__ void __launch_bounds__(VT) k_initFunctions(ugks_block_desc d, size_t g1, double *Fin,
                                                       const double *macro, const double *gQ) {
+  pdl_begin();
   size_t mi, mj;
   work_group(g1, mi, mj);
   if (!(mi < (size_t)d.ni && mj < (size_t)d.nj)) return;
@@ -558,6 +589,7 @@ __global__ void __launch_bounds__(VT) k_initFunctions(ugks_block_desc d, size_t 
 // clFindDT (clKernel.c:224-308): cfl_frequency of ugks_device.cuh per cell
 __global__ void k_clFindDT(ugks_block_desc d, size_t g0, size_t g1, const double *xy,
                            const double *area, const double *macro, double *time_step, double Kn) {
+  pdl_begin();
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= g0 * g1) return;
   long mi = t / g1, mj = t % g1;
@@ -565,6 +597,7 @@ __global__ void k_clFindDT(ugks_block_desc d, size_t g0, size_t g1, const double
 }
 
 __global__ void k_array_max(const double *x, size_t n, double *out) {
+  pdl_begin();
   __shared__ double sm[32];
   double m = -INFINITY;
   for (size_t i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, x[i]);
@@ -580,6 +613,7 @@ __global__ void k_array_max(const double *x, size_t n, double *out) {
 }
 
 __global__ void k_paraBC(ugks_block_desc d, size_t g0, double *wall_prop) {
+  pdl_begin();
   size_t ci = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (ci >= g0) return;
   for (int f = 0; f < 4; ++f) {
@@ -620,6 +654,7 @@ __global__ void __launch_bounds__(VT) k_edgeExchange(ugks_block_desc d, size_t g
                                                      const double *xyA, int this_face,
                                                      const double *fB, const double *xyB, int NIB,
                                                      int NJB, int that_face, int ori, int flip) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   const int G = d.ghost, NI = d.Ni, NJ = d.Nj;
@@ -647,6 +682,7 @@ __global__ void __launch_bounds__(VT) k_edgeExchange(ugks_block_desc d, size_t g
 
 __global__ void __launch_bounds__(VT) k_edgeExtrapolate(ugks_block_desc d, size_t g1, double *Fin,
                                                         int this_face) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   long gi = a, gj = b, ei, ej;
@@ -663,6 +699,7 @@ __global__ void __launch_bounds__(VT) k_edgeExtrapolate(ugks_block_desc d, size_
 
 __global__ void __launch_bounds__(VT) k_edgeConstant(ugks_block_desc d, size_t g1, double *Fin,
                                                      int this_face, const double *wall_prop) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   long gi = a, gj = b;
@@ -677,6 +714,7 @@ __global__ void __launch_bounds__(VT) k_edgeInOut(ugks_block_desc d, size_t g1, 
                                                   int this_face, const double *normal,
                                                   const double *macro, const double *gQ,
                                                   const double *wall_prop, int outflow) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   long gi = a, gj = b, ei, ej, noi, noj;
@@ -707,6 +745,7 @@ __global__ void __launch_bounds__(VT) k_edgeInOut(ugks_block_desc d, size_t g1, 
 
 __global__ void __launch_bounds__(VT) k_edgeMirror(ugks_block_desc d, size_t g1, double *Fin,
                                                    int this_face, int bounce) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   long gi = a, gj = b, mi, mj;
@@ -725,6 +764,7 @@ __global__ void __launch_bounds__(VT) k_edgeMirror(ugks_block_desc d, size_t g1,
 
 __global__ void __launch_bounds__(VT) k_edgeConstGrad(ugks_block_desc d, size_t g1, double *Fin,
                                                       int this_face) {
+  pdl_begin();
   size_t a, b;
   work_group(g1, a, b);
   long gi = a, gj = b, ei0, ej0, ei1, ej1;
@@ -754,6 +794,7 @@ __global__ void __launch_bounds__(VT) k_adsorbingWall_P1(ugks_block_desc d, size
                                                          double *wall_cover, double *wall_dist,
                                                          const double *flux_f, const double *macro,
                                                          double dt, double *flag) {
+  pdl_begin();
   __shared__ double scratch[3 * VT / 32];
   __shared__ double correct_sh;
   size_t a, b;
@@ -849,6 +890,7 @@ __global__ void __launch_bounds__(VT) k_adsorbingWall_P1(ugks_block_desc d, size
 // the moments of f
 __global__ void __launch_bounds__(VT) k_getInternal(ugks_block_desc d, size_t g1, const double *Fin, double *Txyz,
                                                     double *Stress) {
+  pdl_begin();
   __shared__ double scratch[7 * VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -890,6 +932,7 @@ __global__ void __launch_bounds__(VT) k_adsorbingWallSCL_P2(ugks_block_desc d, s
                                                             const double *wall_prop,
                                                             const double *wall_cover,
                                                             const double *wall_dist, double *flux_f) {
+  pdl_begin();
   __shared__ double scratch[VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -964,6 +1007,7 @@ __global__ void __launch_bounds__(VT) k_adsorbingWallD_P2(ugks_block_desc d, siz
                                                           const double *wall_prop,
                                                           const double *wall_cover,
                                                           double *flux_f) {
+  pdl_begin();
   __shared__ double scratch[VT / 32];
   size_t a, b;
   work_group(g1, a, b);
@@ -1022,13 +1066,13 @@ __global__ void __launch_bounds__(VT) k_adsorbingWallD_P2(ugks_block_desc d, siz
 #define VEL_LAUNCH(kernel, ...)                                                       \
   do {                                                                                \
     if (g0 * g1 == 0) return 0;                                                       \
-    kernel<<<grid_of(g0, g1), VT, 0, S(stream)>>>(*d, g1, __VA_ARGS__);               \
+    launch(kernel, grid_of(g0, g1), VT, stream, *d, g1, __VA_ARGS__);                 \
     return launch_status();                                                           \
   } while (0)
 #define PT_LAUNCH(kernel, n, ...)                                                     \
   do {                                                                                \
     if ((n) == 0) return 0;                                                           \
-    kernel<<<grid_threads((n), 128), 128, 0, S(stream)>>>(*d, __VA_ARGS__);           \
+    launch(kernel, grid_threads((n), 128), 128, stream, *d, __VA_ARGS__);             \
     return launch_status();                                                           \
   } while (0)
 
@@ -1155,7 +1199,7 @@ int ugks_clFindDT(const ugks_block_desc *d, size_t g0, size_t g1, const double *
 }
 int ugks_array_max(const double *x, size_t n, double *out, void *stream) {
   if (n == 0) return 0;
-  k_array_max<<<1, 1024, 0, S(stream)>>>(x, n, out);
+  launch(k_array_max, 1, 1024, stream, x, n, out);
   return launch_status();
 }
 int ugks_paraBC(const ugks_block_desc *d, size_t g0, size_t g1, const double *para_def,
