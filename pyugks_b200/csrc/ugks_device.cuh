@@ -137,6 +137,12 @@ __device__ __forceinline__ V2 maxwellian(const ugks_block_desc &d, P4 prim, V2 u
   double w = d.weight[v];
   return v2(w * h, w * b);
 }
+// the same for loops over many velocities: kb = K / (2 lambda), taken once
+__device__ __forceinline__ V2 maxwellian(const ugks_block_desc &d, P4 prim, double kb, V2 uv, int v) {
+  double cx = uv.x - prim.s1, cy = uv.y - prim.s2;
+  double h = d.weight[v] * (prim.s0 * (prim.s3 / d.PI) * exp(-prim.s3 * (cx * cx + cy * cy)));
+  return v2(h, kb * h);
+}
 // fS (clFunctions.c:64-77)
 __device__ __forceinline__ V2 shakhov(const ugks_block_desc &d, P4 prim, V2 Q, V2 uv, V2 M) {
   double cx = uv.x - prim.s1, cy = uv.y - prim.s2;
