@@ -8,9 +8,11 @@ compiled into the library:
 
 * the face pass runs one launch per *segment* (a run of blocks with one flux
   method and one velocity grid, ``ugks_fused_layout``), and each segment can
-  use any of four shapes, threads per face CTA x CTAs per SM
-  (``ugks_fused_sizes.seg_variant`` 1..4, ``ugks_fused.cu`` FaceShape);
-* the cell pass runs with 2 or 3 CTAs of 8 warps per SM (``cell_variant``).
+  use any of four shapes, warps (faces) per CTA x CTAs per SM
+  (``ugks_fused_sizes.seg_variant`` 1..4, ``ugks_fused.cu`` FaceShape and
+  MomentsShape);
+* the cell pass runs with registers for 2 or 3 times 8 warps per SM
+  (``cell_variant``).
 
 ``tune`` times the candidates on a scratch copy of a solver's table (so the
 solver itself does not advance), one segment at a time with the others
