@@ -509,31 +509,6 @@ __global__ void face_geometry(const ugks_fused_block *__restrict__ B, int nb, in
                    blk.face_geo + 6 * faceidx(d, gi, gj, dir));
 }
 
-// block_sum whose result only thread 0 needs
-template <int N>
-__device__ __forceinline__ void block_sum_to0(double (&x)[N], double *scratch) {
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x[k] += __shfl_xor_sync(0xffffffffu, x[k], o);
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) scratch[k * nw + warp] = x[k];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += scratch[k * nw + w];
-      x[k] = s;
-    }
-  }
-}
-
 // The wall procedure of one wall face (all threads of the CTA take part):
 // accommodatingWallDist (clUGKS.c:774-906) or adsorbingWall_P1 (clAdsorb.c:253-482)
 // followed by the re-emission stage (adsorbingWallD_P2 / S_P2 / CL_P2,
