@@ -1092,8 +1092,6 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, cons
       const double Bk = fma(u, MP, fma(T3, uu, fma(T2, e.y, fma(T1, e.x, T0))));
       cp_async_wait<D2 - 1>();
       const double2 fd = ring[stage * 64], fc = ring[stage * 64 + 32];
-      issue(v + 32 * D2, stage);
-      stage = stage + 1 == D2 ? 0 : stage + 1;
       const double mu = (Mt4 * u) * (u > 0.0 ? F.idist1 : F.idist0);
       const double Rh = fma(-mu, fd.x - fc.x, Mt3 * fd.x), Rb = fma(-mu, fd.y - fc.y, Mt3 * fd.y);
       const double Zh = u * fma(S4, h0, Rh), Zb = u * fma(S2, h0 * kb, Rb);
@@ -1106,6 +1104,10 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, cons
       acc[3] = fma(uu, Zh, acc[3]) + Zb;
       // streamed: read next by the cell pass, a gigabyte of other traffic later
       __stcs(F.row + v, make_double2(hx, hy));
+      // refilled only after the store that consumed the stage's values: a copy is
+      // not ordered after loads of its target that are still under way
+      issue(v + 32 * D2, stage);
+      stage = stage + 1 == D2 ? 0 : stage + 1;
     }
     cp_async_wait<0>();
   }
