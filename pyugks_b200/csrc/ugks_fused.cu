@@ -509,17 +509,29 @@ __global__ void face_geometry(const ugks_fused_block *__restrict__ B, int nb, in
                    blk.face_geo + 6 * faceidx(d, gi, gj, dir));
 }
 
+// whether wall is the last adsorbing wall in the order N, S, E, W with a face ci
+__device__ __forceinline__ bool last_on_row(const ugks_fused_block &blk, int wall, long ci) {
+  auto rank = [](int f) { return ((f & 1) << 1) | (f >> 1); };
+  for (int f = 0; f < 4; ++f)
+    if (blk.bc_type[f] == BC_ADSORBING && rank(f) > rank(wall) && ci < ((f & 1) ? blk.d.nj : blk.d.ni)) return false;
+  return true;
+}
+
 // The wall procedure of one wall face (all threads of the CTA take part):
 // accommodatingWallDist (clUGKS.c:774-906) or adsorbingWall_P1 (clAdsorb.c:253-482)
 // followed by the re-emission stage (adsorbingWallD_P2 / S_P2 / CL_P2,
 // clAdsorb.c:488-975), then wallFlux (clUGKS.c:910-1011) and
 // wallMassEnergyFluxes (1019-1147).  face_value(v, h, b) gives the reconstructed
 // face distribution; fw holds Nv (h, b) pairs (each thread reads back only what
-// it wrote); rin is shared scratch of Nv (h, b) pairs (FP64: the wall_dist row
-// itself) for the reflected incoming distribution; store_flux(v, h, b) writes
-// the face-flux row of velocity v.  A diffuse wall takes two sweeps: the face
-// values of the incoming half and the wall Maxwellian of the outgoing half (one
-// exp each) with their two sums, then the fluxes with their eight sums.
+// it wrote); rin is scratch of this face alone, Nv (h, b) pairs, from which
+// specular and Cercignani-Lampis walls gather the reflected incoming
+// distribution; store_flux(v, h, b) writes the face-flux row of velocity v.
+// wall_dist has one row per ci for all four walls of the block, whose CTAs run
+// side by side, so nothing is read back from it: the wall the reference treats
+// last (N, S, E, W) leaves its reflected distribution there, the others nothing.
+// A diffuse wall takes two sweeps: the face values of the incoming half and the
+// wall Maxwellian of the outgoing half (one exp each) with their two sums, then
+// the fluxes with their eight sums.
 template <int NT, typename RIN, typename FaceValue, typename StoreFlux>
 __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solve_state &sol, FaceShared<NT> &sh,
                                           double *fw, RIN *rin, const int wall, const int dir, const long gi,
@@ -573,20 +585,25 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
     const double theta = cover[0];
     const double gf = d.gamma_f[wall];
     double s[3] = {0.0, 0.0, 0.0};
-    for (int v = threadIdx.x; v < Nv; v += NT) {
-      const V2 uv = fvel(v);
+    // the parts of the incoming flux of velocity v: reflected, adsorbed, beta times all
+    auto incoming = [&](int v, V2 uv, V2 &refl, V2 &ads, double &stick) {
       const int delta = upwind_flag(uv.x, rot);
       const double k = -rot * uv.x * (1 - delta);
       const V2 total = v2(k * fw[2 * v], k * fw[2 * v + 1]);
       const double beta = sticking(d, uv, Tw, wall);
-      V2 ads = v2(beta * total.x * gf * (1.0 - theta), beta * total.y * gf * (1.0 - theta));
+      ads = v2(beta * total.x * gf * (1.0 - theta), beta * total.y * gf * (1.0 - theta));
       const double fs = ocl_sign(total.x);
       if ((fs * ads.x) > (fs * total.x)) ads = total;
-      const V2 refl = v2(total.x - ads.x, total.y - ads.y);
+      refl = v2(total.x - ads.x, total.y - ads.y);
+      stick = beta * total.x;
+    };
+    for (int v = threadIdx.x; v < Nv; v += NT) {
+      V2 refl, ads;
+      double stick;
+      incoming(v, fvel(v), refl, ads, stick);
       s[0] += refl.x;
       s[1] += ads.x;
-      s[2] += beta * total.x;
-      st2(blk.wall_dist, (size_t)ci * Nv + v, v2(refl.x / uv.x, refl.y / uv.x));
+      s[2] += stick;
     }
     block_sum<3>(s, sh.scratch);
     if (threadIdx.x == 0) {
@@ -633,11 +650,21 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
     __syncthreads();
     const double corr = sh.bcast[0];
     const bool ok = sh.bcast[1] != 0.0;
-    if (corr != 1.0)
+    const int kind = d.reflect[wall];
+    const bool keep = last_on_row(blk, wall, ci), gather = ok && kind != UGKS_REFLECT_DIFFUSE;
+    if (keep || gather)
       for (int v = threadIdx.x; v < Nv; v += NT) {
-        const size_t k = (size_t)ci * Nv + v;
-        const V2 x = ld2(blk.wall_dist, k);
-        st2(blk.wall_dist, k, v2(x.x * corr, x.y * corr));
+        const V2 uv = fvel(v);
+        V2 x, ads;
+        double stick;
+        incoming(v, uv, x, ads, stick);
+        x = v2(x.x / uv.x, x.y / uv.x);
+        if (corr != 1.0) x = v2(x.x * corr, x.y * corr);
+        if (keep) st2(blk.wall_dist, (size_t)ci * Nv + v, x);
+        if (gather) {
+          rin[v].x = x.x;
+          rin[v].y = x.y;
+        }
       }
     if (!ok) {
       // the reference skips the rest of this wall face and carries on
@@ -651,19 +678,9 @@ __device__ __forceinline__ void wall_face(const ugks_fused_block &blk, ugks_solv
     // diffuse), adsorbingWallS_P2 (656-816, specular) or adsorbingWallCL_P2
     // (488-651, Cercignani-Lampis)
     const double refl = cover[1], des = cover[3], ads = cover[2];
-    const int kind = d.reflect[wall];
     double ratio = 1.0;
     if (refl > 0.0) {
-      // the reflected incoming distribution (wall_dist) of every velocity
-      // (FP64: read in place, mixed: staged in shared memory)
-      __syncthreads();
-      if (!std::is_same<RIN, double2>::value && kind != UGKS_REFLECT_DIFFUSE)
-        for (int v = threadIdx.x; v < Nv; v += NT) {
-          const V2 x = ld2(blk.wall_dist, (size_t)ci * Nv + v);
-          rin[v].x = x.x;
-          rin[v].y = x.y;
-        }
-      __syncthreads();
+      __syncthreads();  // rin is complete
       const double an = d.alpha_n[wall], at = d.alpha_t[wall], Tw = 1.0 / wl.s3;
       double r[1] = {0.0};
       for (int v = threadIdx.x; v < Nv; v += NT) {
@@ -1123,7 +1140,8 @@ __device__ __forceinline__ void face_item_fp64(const ugks_fused_block &blk, cons
 
 // A wall face in FP64 (all NT threads of the CTA take part): the face values
 // live in the face's flux row, which the wall procedure works on in place; the
-// reflected incoming distribution it gathers from is read where P1 put it, wall_dist.
+// reflected incoming distribution it gathers from lies in the row behind the
+// wall, a ghost face that nothing else touches (there are two ghost layers or more).
 template <int FM, int NT>
 __device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_solve_state &sol, const double dt,
                                             FaceShared<NT> &sh, const FaceWork fwk) {
@@ -1148,9 +1166,8 @@ __device__ __noinline__ void wall_item_fp64(const ugks_fused_block &blk, ugks_so
     double sx, sy;
     reconstruct<FM>(xs, g[2], g[0], g[1], h, b, sx, sy);
   };
-  const long ci = dir == SOUTH ? fwk.mi : fwk.mj;
-  wall_face<NT>(blk, sol, sh, reinterpret_cast<double *>(row),
-                reinterpret_cast<double2 *>(blk.wall_dist) + (size_t)ci * Nv, fwk.wall, dir, gi, gj, fwk.mi, fwk.mj, n,
+  double2 *behind = row + (fwk.wall == GNORTH || fwk.wall == GEAST ? step : -step);
+  wall_face<NT>(blk, sol, sh, reinterpret_cast<double *>(row), behind, fwk.wall, dir, gi, gj, fwk.mi, fwk.mj, n,
                 blk.side_length[fk], dt, face_value, [&](int v, double hx, double hy) { row[v] = make_double2(hx, hy); });
 }
 
