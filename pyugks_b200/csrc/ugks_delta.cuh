@@ -270,16 +270,21 @@ __global__ void __launch_bounds__(WALL_NT) wall_pass_delta(const ugks_fused_bloc
 }
 // and redone after a dt change
 __global__ void __launch_bounds__(WALL_NT) wall_retry_delta(const ugks_fused_block *__restrict__ B, int nb,
-                                                            ugks_solve_state *__restrict__ solves, int ns,
-                                                            int per_solve) {
+                                                            ugks_solve_state *__restrict__ solves, int ns) {
   pdl_begin();
-  int b0, bl;
-  if (!retry_solve(B, solves, ns, per_solve, b0, bl)) return;
-  const int end = B[bl].wall_begin + 2 * (B[bl].d.ni + B[bl].d.nj);
-  for (int w = B[b0].wall_begin + blockIdx.x % per_solve; w < end; w += per_solve) {
-    wall_work_delta(B, nb, solves, w, 1);
-    __syncthreads();  // the next item reuses the shared tables
-  }
+  int walls = 0;  // items of the solves before
+  each_solve(
+      ns, [&](int s) { return retries(solves[s]); },
+      [&](int s) {
+        const ugks_solve_state &x = solves[s];
+        const ugks_fused_block &b = B[x.first_block], &e = B[x.first_block + x.nblocks - 1];
+        const int n = e.wall_begin + 2 * (e.d.ni + e.d.nj) - b.wall_begin;
+        for (int w = first_item(blockIdx.x, walls, gridDim.x); w < n; w += gridDim.x) {
+          wall_work_delta(B, nb, solves, b.wall_begin + w, 1);
+          __syncthreads();  // the next item reuses the shared tables
+        }
+        walls += n;
+      });
 }
 
 // 2. coefficients: the chain of face_coefficients, an interior face on two
