@@ -361,6 +361,10 @@ typedef struct ugks_solve_state {
 #define UGKS_STOP_ERROR 3
 
 #define UGKS_MAX_FACE_SEGMENTS 16
+/* seg_method of a last segment that stands for a launch of wall faces instead of a
+   run of blocks: the *_fp64 step's Cercignani-Lampis walls of blocks of more than
+   1100 velocities, present when the table has any (seg_count: n_wall) */
+#define UGKS_SEG_CL_WALLS 4
 
 /* Work sizes of a block table, computed on the host by ugks_fused_layout. */
 typedef struct ugks_fused_sizes {

@@ -101,6 +101,7 @@ _CT = {"p": vp, "i": C.c_int, "d": f64}
 # layout of the mixed path's reference Maxwellian (UGKS_REF_*, include/ugks_b200.h)
 REF_LAMBDA, REF_P0, REF_KB0, REF_MOM, REF_TAB = 0, 1, 2, 4, 32
 FACE_REC = 48       # UGKS_FACE_REC
+SEG_CL_WALLS = 4    # UGKS_SEG_CL_WALLS
 
 # ugks_getDT_noalloc limits and error codes (include/ugks_b200.h)
 NOALLOC_MAX_CELLS = 1 << 20

@@ -1189,15 +1189,33 @@ __device__ __forceinline__ int wall_to_face(const ugks_fused_block &blk, int w) 
   return blk.face_begin + ((mi * (d.nj + 1) + mj) << 1) + dir;
 }
 
-// a wall work item of any flux method (all threads of the CTA)
+// Cercignani-Lampis walls of more than WIDE_NV velocities, FP64: the Nv^2 loop of
+// such a face is as long as its CTA is narrow, so that tables that have any (a
+// segment of method UGKS_SEG_CL_WALLS) take them in a launch of their own, in CTAs
+// of WIDE_NT threads, beside which the faces run.  Step in ms with these walls in
+// the face pass's CTAs of 128 threads and so: 32 wall faces of 1681 velocities 11.2
+// and 3.8, 256 of 1369 8.7 and 5.4, 256 of 2401 25.0 and 14.3.
+constexpr int WIDE_NV = 1100, WIDE_NT = 512;
+__host__ __device__ inline bool wide_cl_wall(const ugks_fused_block &blk, int wall) {
+  return blk.d.Nv > WIDE_NV && blk.bc_type[wall] == BC_ADSORBING && blk.d.reflect[wall] == UGKS_REFLECT_CL;
+}
+inline bool has_cl_walls(const ugks_fused_sizes *z) {
+  return z->n_segments > 0 && z->seg_method[z->n_segments - 1] == UGKS_SEG_CL_WALLS;
+}
+
+// a wall work item of any flux method (all threads of the CTA): every wall, the wide
+// Cercignani-Lampis walls only, or the others only
+enum WallKind { WALL_ANY, WALL_WIDE_CL, WALL_OTHER };
 template <int NT>
 __device__ __forceinline__ void wall_work_fp64(const ugks_fused_block *__restrict__ B, int nb,
-                                               ugks_solve_state *__restrict__ solves, const int w, int retry_pass) {
+                                               ugks_solve_state *__restrict__ solves, const int w, int retry_pass,
+                                               WallKind kind) {
   __shared__ FaceShared<NT> sh;
   const ugks_fused_block &blk = B[find_block<3>(B, nb, w)];
   UGKS_CHECK_ITEM(3, blk, w, solves);
   FaceWork fwk;
   if (!face_work<-1>(B, nb, solves, wall_to_face(blk, w), retry_pass, fwk) || fwk.wall < 0) return;
+  if (kind != WALL_ANY && wide_cl_wall(blk, fwk.wall) != (kind == WALL_WIDE_CL)) return;
   ugks_solve_state &sol = solves[blk.solve];
   const double dt = retry_pass ? step_dt(sol).flux : sol.dt;
   switch (blk.d.flux_method) {
@@ -1206,6 +1224,12 @@ __device__ __forceinline__ void wall_work_fp64(const ugks_fused_block *__restric
     case 3: wall_item_fp64<3, NT>(blk, sol, dt, sh, fwk); break;
     default: break;
   }
+}
+
+__global__ void __launch_bounds__(WIDE_NT) cl_wall_pass_fp64(const ugks_fused_block *__restrict__ B, int nb,
+                                                             ugks_solve_state *__restrict__ solves) {
+  pdl_begin();
+  wall_work_fp64<WIDE_NT>(B, nb, solves, (int)blockIdx.x, 0, WALL_WIDE_CL);
 }
 
 // FP64 face pass: the first n_wall CTAs take a wall work item each (they are
@@ -1217,14 +1241,15 @@ __device__ __forceinline__ double2 *face_ring(double *dyn, int wstride, int warp
 template <int FM, int WPC, int MINB>
 __global__ void __launch_bounds__(WPC * 32, MINB) face_pass_fp64(const ugks_fused_block *__restrict__ B, int nb,
                                                                  ugks_solve_state *__restrict__ solves, int n_wall,
-                                                                 int first, int count, int wstride, int chained) {
+                                                                 WallKind kind, int first, int count, int wstride,
+                                                                 int chained) {
   extern __shared__ double dyn[];
   pdl_begin_face(chained);
   const int warp = threadIdx.x >> 5;
   const int item = ((int)blockIdx.x - n_wall) * WPC + warp;
   FaceWork fwk;
   if ((int)blockIdx.x < n_wall) {
-    wall_work_fp64<WPC * 32>(B, nb, solves, (int)blockIdx.x, 0);
+    wall_work_fp64<WPC * 32>(B, nb, solves, (int)blockIdx.x, 0, kind);
   } else if (item < count && face_work<FM, true>(B, nb, solves, first + item, 0, fwk) && fwk.wall < 0) {
     const ugks_fused_block &blk = B[fwk.bi];
     face_item_fp64<FM>(blk, solves[blk.solve].dt, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
@@ -1272,7 +1297,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_retry_fp64(const ugks_fus
         const ugks_fused_block &b = B[x.first_block], &e = B[x.first_block + x.nblocks - 1];
         const int nw = e.wall_begin + 2 * (e.d.ni + e.d.nj) - b.wall_begin;
         for (int w = first_item(blockIdx.x, walls, ctas); w < nw; w += ctas) {
-          wall_work_fp64<WPC * 32>(B, nb, solves, b.wall_begin + w, 1);
+          wall_work_fp64<WPC * 32>(B, nb, solves, b.wall_begin + w, 1, WALL_ANY);
           __syncthreads();  // the next item reuses the shared tables
         }
         walls += nw;
@@ -1896,13 +1921,16 @@ cudaError_t allow_smem(K kernel) {
 template <int V>
 cudaError_t set_face_shape() {
   constexpr int W = FaceShape<V>::wpc, M = FaceShape<V>::minb;
-  cudaError_t r[6] = {allow_smem(face_pass_fp64<0, W, M>), allow_smem(face_pass_fp64<1, W, M>),
-                      allow_smem(face_pass_fp64<3, W, M>), cudaSuccess, cudaSuccess, cudaSuccess};
-  if constexpr (V == 1) {
-    r[3] = allow_smem(face_retry_fp64<0, W, M>);
-    r[4] = allow_smem(face_retry_fp64<1, W, M>);
-    r[5] = allow_smem(face_retry_fp64<3, W, M>);
-  }
+  cudaError_t r[3] = {allow_smem(face_pass_fp64<0, W, M>), allow_smem(face_pass_fp64<1, W, M>),
+                      allow_smem(face_pass_fp64<3, W, M>)};
+  for (cudaError_t e : r)
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
+template <int W, int M>
+cudaError_t set_retry_shape() {
+  cudaError_t r[3] = {allow_smem(face_retry_fp64<0, W, M>), allow_smem(face_retry_fp64<1, W, M>),
+                      allow_smem(face_retry_fp64<3, W, M>)};
   for (cudaError_t e : r)
     if (e != cudaSuccess) return e;
   return cudaSuccess;
@@ -1910,7 +1938,8 @@ cudaError_t set_face_shape() {
 template <typename T>
 cudaError_t set_wall_attributes() {
   if constexpr (std::is_same<T, double>::value) {
-    cudaError_t r[4] = {set_face_shape<1>(), set_face_shape<2>(), set_face_shape<3>(), set_face_shape<4>()};
+    cudaError_t r[6] = {set_face_shape<1>(), set_face_shape<2>(), set_face_shape<3>(), set_face_shape<4>(),
+                        set_retry_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(), set_retry_shape<WIDE_NT / 32, 1>()};
     for (cudaError_t e : r)
       if (e != cudaSuccess) return e;
   }
@@ -2022,28 +2051,37 @@ size_t face_smem(int wstride) {
 // the FP64 face pass of one segment (one flux method) in launch shape v; the
 // first segment's launch takes the wall faces of the whole table with it
 template <int WPC, int MINB>
-void launch_faces_shape(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall, int first,
+void launch_faces_shape(const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall, WallKind kind, int first,
                         int count, int axes, int chained, StepStream st) {
   const int ws = face_stride(axes);
   const unsigned g = (unsigned)(n_wall + (count + WPC - 1) / WPC + chained), t = WPC * 32;
   switch (method) {
-    case 0: launch(face_pass_fp64<0, WPC, MINB>, g, t, face_smem<0, WPC>(ws), st, B, nb, solves, n_wall, first, count, ws, chained); break;
-    case 1: launch(face_pass_fp64<1, WPC, MINB>, g, t, face_smem<1, WPC>(ws), st, B, nb, solves, n_wall, first, count, ws, chained); break;
-    case 3: launch(face_pass_fp64<3, WPC, MINB>, g, t, face_smem<3, WPC>(ws), st, B, nb, solves, n_wall, first, count, ws, chained); break;
+    case 0: launch(face_pass_fp64<0, WPC, MINB>, g, t, face_smem<0, WPC>(ws), st, B, nb, solves, n_wall, kind, first, count, ws, chained); break;
+    case 1: launch(face_pass_fp64<1, WPC, MINB>, g, t, face_smem<1, WPC>(ws), st, B, nb, solves, n_wall, kind, first, count, ws, chained); break;
+    case 3: launch(face_pass_fp64<3, WPC, MINB>, g, t, face_smem<3, WPC>(ws), st, B, nb, solves, n_wall, kind, first, count, ws, chained); break;
     default: break;
   }
 }
 inline void launch_faces(int v, const ugks_fused_block *B, int nb, ugks_solve_state *solves, int method, int n_wall,
-                         int first, int count, int axes, int chained, StepStream st) {
+                         WallKind kind, int first, int count, int axes, int chained, StepStream st) {
   switch (v) {
-    case 2: launch_faces_shape<FaceShape<2>::wpc, FaceShape<2>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
-    case 3: launch_faces_shape<FaceShape<3>::wpc, FaceShape<3>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
-    case 4: launch_faces_shape<FaceShape<4>::wpc, FaceShape<4>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
-    default: launch_faces_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, solves, method, n_wall, first, count, axes, chained, st); break;
+    case 2: launch_faces_shape<FaceShape<2>::wpc, FaceShape<2>::minb>(B, nb, solves, method, n_wall, kind, first, count, axes, chained, st); break;
+    case 3: launch_faces_shape<FaceShape<3>::wpc, FaceShape<3>::minb>(B, nb, solves, method, n_wall, kind, first, count, axes, chained, st); break;
+    case 4: launch_faces_shape<FaceShape<4>::wpc, FaceShape<4>::minb>(B, nb, solves, method, n_wall, kind, first, count, axes, chained, st); break;
+    default: launch_faces_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, solves, method, n_wall, kind, first, count, axes, chained, st); break;
   }
 }
 
-// the retry pass of every flux method (per solve; rare)
+template <int WPC, int MINB>
+void launch_retry_shape(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves, int ns,
+                        StepStream st) {
+  const unsigned g = std::min(retry_grid(ns), 148u * MINB), t = WPC * 32;
+  const int ws = face_stride(z->max_axes);
+  if (z->face_count[0]) launch(face_retry_fp64<0, WPC, MINB>, g, t, face_smem<0, WPC>(ws), st, B, nb, solves, ns, ws);
+  if (z->face_count[1]) launch(face_retry_fp64<1, WPC, MINB>, g, t, face_smem<1, WPC>(ws), st, B, nb, solves, ns, ws);
+  if (z->face_count[3]) launch(face_retry_fp64<3, WPC, MINB>, g, t, face_smem<3, WPC>(ws), st, B, nb, solves, ns, ws);
+}
+// the retry pass of every flux method (rare)
 template <typename T>
 void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves, int ns,
                   StepStream st) {
@@ -2052,11 +2090,8 @@ void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, 
     // only the wall faces have anything to redo
     if (z->n_wall) launch(wall_retry_delta, rg, WALL_NT, delta_wall_smem(z->max_nv), st, B, nb, solves, ns);
   } else {
-    constexpr int WPC = FaceShape<1>::wpc, MINB = FaceShape<1>::minb, NT = WPC * 32;
-    const int ws = face_stride(z->max_axes);
-    if (z->face_count[0]) launch(face_retry_fp64<0, WPC, MINB>, rg, NT, face_smem<0, WPC>(ws), st, B, nb, solves, ns, ws);
-    if (z->face_count[1]) launch(face_retry_fp64<1, WPC, MINB>, rg, NT, face_smem<1, WPC>(ws), st, B, nb, solves, ns, ws);
-    if (z->face_count[3]) launch(face_retry_fp64<3, WPC, MINB>, rg, NT, face_smem<3, WPC>(ws), st, B, nb, solves, ns, ws);
+    if (has_cl_walls(z)) launch_retry_shape<WIDE_NT / 32, 1>(B, nb, z, solves, ns, st);
+    else launch_retry_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, z, solves, ns, st);
   }
 }
 
@@ -2151,8 +2186,13 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     chained = st.carve > 0;
   }
   int walls = z->n_wall;
+  const bool cl_walls = !mixed && walls && has_cl_walls(z);
+  if (cl_walls) {
+    launch(cl_wall_pass_fp64, walls, WIDE_NT, 0, st, B, nb, solves);
+    chained = 1;
+  }
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) {
-    if (z->seg_count[k] <= 0) continue;
+    if (z->seg_count[k] <= 0 || z->seg_method[k] == UGKS_SEG_CL_WALLS) continue;
     int v = z->seg_variant[k];
     StepStream to = st;
     to.chained = chained;
@@ -2161,7 +2201,7 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
     if constexpr (mixed) {
       launch_moments(v, B, nb, solves, m, b0, n, z->seg_max_axes[k], chained, to);
     } else {
-      launch_faces(v, B, nb, solves, m, walls, b0, n, z->seg_max_axes[k], chained, to);
+      launch_faces(v, B, nb, solves, m, walls, cl_walls ? WALL_OTHER : WALL_ANY, b0, n, z->seg_max_axes[k], chained, to);
       walls = 0;
     }
     chained = 1;
@@ -2317,7 +2357,8 @@ int ugks_step_launches(const ugks_fused_sizes *z, int mixed) {
   int n = 0;
   if (mixed && z->n_faces) n += 2;  // the mixed face pass's coefficient and flux launches
   if (mixed && z->n_wall) n += 1;   // and its wall launch
-  for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) n += z->seg_count[k] > 0 ? 1 : 0;
+  for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k)
+    n += z->seg_count[k] > 0 && !(mixed && z->seg_method[k] == UGKS_SEG_CL_WALLS) ? 1 : 0;
   if (mixed) n += z->n_wall ? 1 : 0;  // retry pass (mixed: walls)
   else for (int m = 0; m < 4; ++m) n += z->face_count[m] > 0 ? 1 : 0;
   n += z->n_cells ? 1 : 0;
@@ -2407,6 +2448,7 @@ int ugks_fused_layout(ugks_fused_block *blocks, int nblocks, ugks_fused_sizes *z
   };
   std::vector<Run> runs;
   int last_method = -1, seen = 0, last_solve = -1;
+  bool cl_walls = false;
   for (int b = 0; b < nblocks; ++b) {
     ugks_fused_block &x = blocks[b];
     const int m = x.d.flux_method;
@@ -2426,6 +2468,7 @@ int ugks_fused_layout(ugks_fused_block *blocks, int nblocks, ugks_fused_sizes *z
     x.ghost_begin = (int32_t)g;
     x.wall_begin = (int32_t)wl;
     wl += 2ll * (x.d.ni + x.d.nj);
+    for (int w = 0; w < 4; ++w) cl_walls |= wide_cl_wall(x, w);
     const int64_t nf = 2ll * (x.d.ni + 1) * (x.d.nj + 1);
     const int axes_b = (x.d.u_num > 0 && x.d.u_num * x.d.v_num == x.d.Nv && x.d.u_num + x.d.v_num <= 512)
                            ? x.d.u_num + x.d.v_num : 0;
@@ -2451,7 +2494,8 @@ int ugks_fused_layout(ugks_fused_block *blocks, int nblocks, ugks_fused_sizes *z
   // at most UGKS_MAX_FACE_SEGMENTS launches: merge the adjacent pair of one
   // method whose merged Nv is smallest (methods are contiguous, so this ends
   // at one run per method at worst)
-  while ((int)runs.size() > UGKS_MAX_FACE_SEGMENTS) {
+  const int limit = UGKS_MAX_FACE_SEGMENTS - (cl_walls ? 1 : 0);
+  while ((int)runs.size() > limit) {
     int best = -1;
     for (int k = 0; k + 1 < (int)runs.size(); ++k)
       if (runs[k].method == runs[k + 1].method &&
@@ -2464,6 +2508,7 @@ int ugks_fused_layout(ugks_fused_block *blocks, int nblocks, ugks_fused_sizes *z
     runs[best].count += runs[best + 1].count;
     runs.erase(runs.begin() + best + 1);
   }
+  if (cl_walls) runs.push_back(Run{UGKS_SEG_CL_WALLS, 0, max_nv, 0, 0, wl});
   z->n_segments = (int32_t)runs.size();
   for (int k = 0; k < UGKS_MAX_FACE_SEGMENTS; ++k) {
     const bool on = k < (int)runs.size();

@@ -91,9 +91,10 @@ def update_cache(entries: dict, path: str | None = None) -> dict:
 
 
 def segments(sizes):
-    """(index, flux method, velocity count) of every face-pass segment."""
+    """(index, flux method, velocity count) of every face-pass segment that has a
+    choice of shapes."""
     return [(k, sizes.seg_method[k], sizes.seg_max_nv[k]) for k in range(sizes.n_segments)
-            if sizes.seg_count[k] > 0]
+            if sizes.seg_count[k] > 0 and sizes.seg_method[k] != _lib.SEG_CL_WALLS]
 
 
 def apply(solver, choices: dict):
