@@ -374,7 +374,7 @@ typedef struct ugks_fused_sizes {
   int32_t max_nv;         /* largest Nv (sizes the face pass's shared memory)  */
   int32_t face_begin[4];  /* first face work item of the blocks of flux_method k */
   int32_t face_count[4];  /* their number (0 when no block uses method k)      */
-  int32_t max_axes;       /* largest u_num + v_num of a tensor velocity grid   */
+  int32_t max_axes;       /* largest u_num + v_num, up to 512, of a tensor velocity grid */
   /* face-pass launches: runs of consecutive blocks with one flux method and
      one Nv (merged within a method when there are more than
      UGKS_MAX_FACE_SEGMENTS), each launched with shared memory for its own Nv */
@@ -383,7 +383,7 @@ typedef struct ugks_fused_sizes {
   int32_t seg_count[UGKS_MAX_FACE_SEGMENTS];
   int32_t seg_method[UGKS_MAX_FACE_SEGMENTS];
   int32_t seg_max_nv[UGKS_MAX_FACE_SEGMENTS];
-  int32_t seg_max_axes[UGKS_MAX_FACE_SEGMENTS];
+  int32_t seg_max_axes[UGKS_MAX_FACE_SEGMENTS];  /* largest u_num + v_num, of any size */
   /* launch shape per face-pass segment (0 by velocity count; 1..4 force one
      of the compiled shapes, ugks_fused.cu FaceShape) and of the cell pass
      (0 default; 2 or 3 CTAs of 8 warps per SM); ugks_fused_layout sets 0, a

@@ -2041,8 +2041,14 @@ inline size_t face_limit_bytes(int max_nv, int max_axes) {
 }
 
 // doubles of shared memory per FP64 face warp beside its ring: the face record
-// and the axis factors
-inline int face_stride(int max_axes) { return FACE_TAB + ((max_axes + 1) & ~1); }
+// and the axis factors (of grids with up to 512 axis nodes; larger ones go without)
+inline int face_stride(int max_axes) { return FACE_TAB + ((std::min(max_axes, 512) + 1) & ~1); }
+// the mixed kernels keep axis tables of any tensor grid
+inline int mixed_axes(const ugks_fused_sizes *z) {
+  int n = z->max_axes;
+  for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k) n = std::max(n, (int)z->seg_max_axes[k]);
+  return n;
+}
 template <int FM, int WPC>
 size_t face_smem(int wstride) {
   return (size_t)WPC * (wstride * sizeof(double) + face_ring_elems<FM>() * sizeof(double2));
@@ -2150,11 +2156,14 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   // cell pass: the axis factor tables of the old and new macro state
   constexpr bool mixed = std::is_same<T, float>::value;
   // doubles of shared memory per cell warp
-  const int cstride = mixed ? delta_cell_stride(z->max_axes) : 2 * z->max_axes + CELL_COEF;
+  const int axes = mixed ? mixed_axes(z) : z->max_axes;
+  const int cstride = mixed ? delta_cell_stride(axes) : 2 * axes + CELL_COEF;
   const size_t csmem = (size_t)CW * cstride * sizeof(double) + (mixed ? (size_t)CW * CELL_RING_F32 * 160 * 16 : (size_t)CW * cell_ring_bytes());
   const cudaError_t attr = set_step_attributes<T>();
   if (attr != cudaSuccess) return -(int)attr;
-  if (face_limit_bytes<T>(z->max_nv, z->max_axes) > 200 * 1024 || csmem > 200 * 1024) return -(int)cudaErrorInvalidValue;
+  const size_t fsmem = mixed ? FLUX_WPC * flux_tma_warp_bytes(axes) : 0;
+  if (face_limit_bytes<T>(z->max_nv, z->max_axes) > 200 * 1024 || csmem > 200 * 1024 || fsmem > 200 * 1024)
+    return -(int)cudaErrorInvalidValue;
   auto mark = [&](int k) {
     if (events && events[k]) cudaEventRecord(reinterpret_cast<cudaEvent_t>(events[k]), st.st);
   };
@@ -2219,9 +2228,9 @@ int step_impl(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks
   launch_retry<T>(B, nb, z, solves, ns, st);
   if (mixed && z->n_faces) {
     launch(face_coef_delta, (unsigned)((2l * z->n_faces + COEF_NT - 1) / COEF_NT), COEF_NT, 0, st, B, nb, solves, z->n_faces);
-    const int wb = (int)flux_tma_warp_bytes(z->max_axes);
+    const int wb = (int)flux_tma_warp_bytes(axes);
     launch(face_flux_tma<FLUX_WPC, FLUX_TMA_MINB>, (unsigned)((z->n_faces + FLUX_WPC - 1) / FLUX_WPC), FLUX_WPC * 32,
-           (size_t)FLUX_WPC * wb, st, B, nb, solves, z->n_faces, wb);
+           fsmem, st, B, nb, solves, z->n_faces, wb);
   }
   if (mixed) {
     mark(1);
@@ -2470,8 +2479,7 @@ int ugks_fused_layout(ugks_fused_block *blocks, int nblocks, ugks_fused_sizes *z
     wl += 2ll * (x.d.ni + x.d.nj);
     for (int w = 0; w < 4; ++w) cl_walls |= wide_cl_wall(x, w);
     const int64_t nf = 2ll * (x.d.ni + 1) * (x.d.nj + 1);
-    const int axes_b = (x.d.u_num > 0 && x.d.u_num * x.d.v_num == x.d.Nv && x.d.u_num + x.d.v_num <= 512)
-                           ? x.d.u_num + x.d.v_num : 0;
+    const int axes_b = x.d.u_num > 0 ? x.d.u_num + x.d.v_num : 0;
     if (runs.empty() || runs.back().method != m || runs.back().nv != x.d.Nv)
       runs.push_back(Run{m, x.d.Nv, x.d.Nv, axes_b, f, 0});
     runs.back().count += nf;
