@@ -484,6 +484,10 @@ int ugks_prepare(int mixed);
    bound) when the wait ran out, -1 on a mismatch. */
 int ugks_check_copy_wait(const void *src_dev, unsigned polls, int *status_dev, UGKS_STREAM);
 
+/* The reciprocal that the fused kernels use in place of a division, on its own:
+   y[k] ~ 1 / x[k] for n device doubles. */
+int ugks_check_reciprocal(const double *x_dev, int64_t n, double *y_dev, UGKS_STREAM);
+
 /* ------------------------------------------------------------------------
  * 3. Time-step frequency without device allocation.  No counterpart in the
  *    reference.  For callers that cannot allocate device memory (a host

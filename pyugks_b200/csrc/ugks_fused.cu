@@ -2337,6 +2337,12 @@ __global__ void copy_wait_check(const float4 *src, unsigned polls, int *status) 
   if (lane == 0) *status = !ok ? STATUS_COPY_TIMEOUT : (same ? 0 : -1);
 }
 
+// the reciprocal of the face and cell coefficients, on its own (ugks_check_reciprocal)
+__global__ void reciprocal_check(const double *x, int64_t n, double *y) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k < n) y[k] = nr_rcp(x[k]);
+}
+
 // the stop rule of every active solve (ugks_stop_check)
 __global__ void stop_check(ugks_solve_state *solves, int ns) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2405,6 +2411,12 @@ int ugks_serve_steps(int mixed, const ugks_fused_block *blocks_dev, int nblocks,
 
 int ugks_check_copy_wait(const void *src_dev, unsigned polls, int *status_dev, void *stream) {
   copy_wait_check<<<1, 32, 0, S(stream)>>>(reinterpret_cast<const float4 *>(src_dev), polls, status_dev);
+  return launch_status();
+}
+
+int ugks_check_reciprocal(const double *x_dev, int64_t n, double *y_dev, void *stream) {
+  if (n <= 0) return 0;
+  reciprocal_check<<<(unsigned)((n + 255) / 256), 256, 0, S(stream)>>>(x_dev, n, y_dev);
   return launch_status();
 }
 
