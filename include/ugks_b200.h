@@ -488,6 +488,10 @@ int ugks_check_copy_wait(const void *src_dev, unsigned polls, int *status_dev, U
    y[k] ~ 1 / x[k] for n device doubles. */
 int ugks_check_reciprocal(const double *x_dev, int64_t n, double *y_dev, UGKS_STREAM);
 
+/* The fused kernels' relaxation rate (1 / relaxTime) of gas at density 1 and n values
+   of lambda = 1/T (device); d is a host descriptor (relax_type, Kn_eff, omega). */
+int ugks_check_relax_rate(const ugks_block_desc *d, const double *lambda_dev, int64_t n, double *rate_dev, UGKS_STREAM);
+
 /* ------------------------------------------------------------------------
  * 3. Time-step frequency without device allocation.  No counterpart in the
  *    reference.  For callers that cannot allocate device memory (a host

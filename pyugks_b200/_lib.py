@@ -154,6 +154,8 @@ def lib():
     L.ugks_check_copy_wait.argtypes = [vp, C.c_uint, vp, vp]
     L.ugks_check_reciprocal.restype = C.c_int
     L.ugks_check_reciprocal.argtypes = [vp, C.c_int64, vp, vp]
+    L.ugks_check_relax_rate.restype = C.c_int
+    L.ugks_check_relax_rate.argtypes = [C.POINTER(BlockDesc), vp, C.c_int64, vp, vp]
     L.ugks_getDT_noalloc.restype = C.c_int
     L.ugks_getDT_noalloc.argtypes = [C.POINTER(BlockDesc), vp, vp, vp, f64, vp, vp]
     L.ugks_version.restype = C.c_char_p

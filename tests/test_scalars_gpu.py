@@ -39,3 +39,22 @@ def test_reciprocal(cuda, low):
         y = reciprocals(x)
         err = np.abs(y.astype(np.longdouble) - np.longdouble(1.0) / x.astype(np.longdouble))
         assert np.max(err / np.abs(np.spacing(y))) <= 0.5 + 2.0 ** -10
+
+
+@pytest.mark.parametrize("omega", [0.5, 0.66, 0.81, 1.0])
+@pytest.mark.parametrize("low,high", [(0.8, 1.3), (1e-6, 1e6)])
+def test_relax_rate(cuda, omega, low, high):
+    """1 / tau of density 1 is lambda^(omega - 1): pow is within 2 ulp over its range
+    (CUDA's table), the products are by 1, and the reciprocal adds half an ulp; an ulp
+    is at most 2^-52 of its value, and the host's power is good to 2^-60."""
+    rng = np.random.default_rng(11)
+    lam = np.exp(rng.uniform(np.log(low), np.log(high), 1 << 20))
+    d = _lib.BlockDesc()
+    d.relax_type, d.Kn_eff, d.omega, d.PI = 2, 1.0, omega, np.pi
+    t = torch.from_numpy(lam).cuda()
+    out = torch.empty_like(t)
+    _lib.check(_lib.lib().ugks_check_relax_rate(C.byref(d), t.data_ptr(), len(lam), out.data_ptr(), stream()),
+               "ugks_check_relax_rate")
+    want = np.power(lam.astype(np.longdouble), -np.longdouble(1.0 - omega))
+    err = np.abs(out.cpu().numpy().astype(np.longdouble) - want) / want
+    assert np.max(err) <= 2.5 * 2.0 ** -52 + 2.0 ** -60
