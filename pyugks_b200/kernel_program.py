@@ -65,11 +65,18 @@ class KernelProgram:
         return call
 
 
+# the current device's current stream, without the Stream object that
+# torch.cuda.current_stream() makes (13 us of a 26 us call); names of torch's own
+# that not every version has to have
+_get_device = getattr(torch._C, "_cuda_getDevice", None)
+_get_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(queue):
     if queue is None:
-        # the current device's current stream, without the Stream object that
-        # torch.cuda.current_stream() makes (13 us of a 26 us call)
-        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        if _get_device is None or _get_raw_stream is None:
+            return torch.cuda.current_stream().cuda_stream
+        return _get_raw_stream(_get_device())
     if isinstance(queue, int):
         return queue
     return queue.cuda_stream
