@@ -256,8 +256,9 @@ int ugks_adsorbingWallCL_P2(const ugks_block_desc *d, size_t g0, size_t g1, cons
  * *_mixed: they are FP32 *deviations* from a reference Maxwellian M of the
  * solve (ugks_fused_block.ref): f = M + df and
  * flux = dt len (u . n) M + dflux, in a velocity-pair layout
- * [Ni][Nj][(Nv + 1) / 2] x (h_2p, h_2p+1, b_2p, b_2p+1); an odd Nv pads the
- * last pair with a velocity whose entries stay 0.  The tensor velocity grid
+ * [Ni][Nj][ceil(u_num / 2) * v_num] x (h, h', b, b'): pair a v_num + jv holds
+ * velocities (2a, jv) and (2a + 1, jv); an odd u_num pads the last pair row with
+ * velocities whose entries stay 0.  The tensor velocity grid
  * (u_num * v_num == Nv) is required.  Moments, the conserved update, the
  * relaxation, dt and the residual stay FP64 in both.
  * --------------------------------------------------------------------- */
@@ -309,7 +310,9 @@ typedef struct ugks_fused_block {
   double *wall_prop;           /* [max(ni,nj)][4] x 4                       */
   double *wall_cover;          /* [max(ni,nj)][4] x 4                       */
   double *wall_fluxes;         /* [max(ni,nj)][4] x 8                       */
-  double *wall_dist;           /* [max(ni,nj)][Nv] x 2                      */
+  double *wall_dist;           /* [max(ni,nj)][Nv] x 2: the reflected distribution
+                                  of the adsorbing wall that comes last in the order
+                                  N, S, E, W on the row                     */
   double *cell_mom;            /* [Ni][Nj] x 4: sum over v of f (1, u, v,
                                   (u^2+v^2)/2 | 1/2) per cell, global frame;
                                   written by the init, cell and ghost passes,
@@ -337,7 +340,7 @@ typedef struct ugks_solve_state {
   double delta_dt;             /* dt growth limit (ugks_sim.py:306)         */
   double max_dt;               /* CFL / max frequency of the last dt update */
   unsigned long long max_freq; /* bits of the running max CFL frequency (atomicMax) */
-  int32_t retry;               /* 1 while this step's flux pass is redone   */
+  int32_t retry;               /* unused, 0 (the step derives it from dt)   */
   int32_t status;              /* 0 ok, 1 NaN in f, 4 isotherm, 6 bad block
                                   connection (clError.c codes otherwise), 8 a bulk
                                   copy of the face pass outlived its wait bound */
@@ -371,23 +374,24 @@ typedef struct ugks_fused_sizes {
   int32_t n_faces;        /* face work items (2 per cell corner of every block) */
   int32_t n_cells;        /* interior cells                                    */
   int32_t n_ghost;        /* ghost cells of the four strips of every block     */
-  int32_t max_nv;         /* largest Nv (sizes the face pass's shared memory)  */
+  int32_t max_nv;         /* largest Nv (sizes the mixed wall faces' shared memory) */
   int32_t face_begin[4];  /* first face work item of the blocks of flux_method k */
   int32_t face_count[4];  /* their number (0 when no block uses method k)      */
   int32_t max_axes;       /* largest u_num + v_num, up to 512, of a tensor velocity grid */
   /* face-pass launches: runs of consecutive blocks with one flux method and
      one Nv (merged within a method when there are more than
-     UGKS_MAX_FACE_SEGMENTS), each launched with shared memory for its own Nv */
+     UGKS_MAX_FACE_SEGMENTS), each launched with shared memory for its own axes */
   int32_t n_segments;
   int32_t seg_begin[UGKS_MAX_FACE_SEGMENTS];
   int32_t seg_count[UGKS_MAX_FACE_SEGMENTS];
   int32_t seg_method[UGKS_MAX_FACE_SEGMENTS];
   int32_t seg_max_nv[UGKS_MAX_FACE_SEGMENTS];
   int32_t seg_max_axes[UGKS_MAX_FACE_SEGMENTS];  /* largest u_num + v_num, of any size */
-  /* launch shape per face-pass segment (0 by velocity count; 1..4 force one
-     of the compiled shapes, ugks_fused.cu FaceShape) and of the cell pass
-     (0 default; 2 or 3 CTAs of 8 warps per SM); ugks_fused_layout sets 0, a
-     caller (the autotuner) may change them before stepping.  The shape
+  /* launch shape per face-pass segment (0 the default, shape 1; 1..4 one of the
+     compiled shapes, ugks_fused.cu FaceShape and MomentsShape) and of the cell
+     pass (0 default; 2 or 3: registers for 2 or 3 times 8 warps per SM);
+     ugks_fused_layout sets 0, a caller (the autotuner) may change them before
+     stepping.  The shape
      changes the order of the per-face sums, not the arithmetic: results agree
      to round-off across shapes and are reproducible for a fixed shape. */
   int32_t seg_variant[UGKS_MAX_FACE_SEGMENTS];

@@ -1,7 +1,8 @@
-// ugks_fused.cu -- the whole UGKS time step in four launches, for every block
-// of every solve of a device-resident block table.
+// ugks_fused.cu -- the whole UGKS time step in a few launches (FP64 four for one
+// limiter and velocity grid; mixed seven, ugks_delta.cuh), for every block of every
+// solve of a device-resident block table.
 //
-// Per step (UGKSim.one_step, ugks_sim.py:407-501):
+// Per FP64 step (UGKSim.one_step, ugks_sim.py:407-501):
 //   face pass   a face per warp, in either direction: reconstruction (iFace),
 //               face moments (getFaceCons/getAL/getAR), slopes (getPLR),
 //               initMacroFlux, calcFaceQ, macroFlux and distFlux fused; wall
@@ -463,14 +464,13 @@ __device__ __forceinline__ void reconstruct_f(const float2 (&xs)[FM == 1 ? 5 : 3
   fb = fmaf(sb, ds, Sb[MID]);
 }
 
-// scale * exp(-lambda (x - c)^2) over the nodes of one velocity axis
+// exp(-lambda (x - c)^2) over the nodes of one velocity axis
 template <typename R>
 __device__ __forceinline__ void axis_exp(R *out, const double *quad, int n, int stride,
-                                         int comp, double c, double lambda, int t, int nt,
-                                         double scale = 1.0) {
+                                         int comp, double c, double lambda, int t, int nt) {
   for (int i = t; i < n; i += nt) {
     const double x = quad[2 * (size_t)i * stride + comp] - c;
-    out[i] = (R)(scale * exp(-lambda * (x * x)));
+    out[i] = (R)exp(-lambda * (x * x));
   }
 }
 
@@ -819,13 +819,13 @@ __device__ __forceinline__ bool face_work(const ugks_fused_block *__restrict__ B
 // Any velocity grid and any face normal; no barrier, no shared memory per
 // velocity: 16 faces are in flight on an SM whatever the velocity grid, each at
 // its own phase, and the serial middle part of one hides behind the sweeps of
-// the others.  On the 2x2-block cavity (Nv 1089, WENO5) 0.976 -> 0.730 ms, on a
-// 96x96 cavity with Nv 2401 (vanLeer) 1.154 -> 0.869 ms, against a CTA per face
+// the others.  On the 2x2-block cavity (Nv 1089, WENO5) 0.976 -> 0.716 ms, on a
+// 96x96 cavity with Nv 2401 (vanLeer) 1.154 -> 0.868 ms, against a CTA per face
 // that kept face values and slopes in shared memory over three velocity sweeps
 // (six, at Nv 2401 two, faces per SM, with barriers around its serial part).
-// Bound by the L1 / shared data pipe (73%: the stencil rows pass it once as
-// cp.async and once as loads) and FP64 issue (49%) at 16 warps per SM.  Measured
-// and not kept (0.730 ms here): no face values stored, the reconstruction run
+// Bound by the L1 / shared data pipe (71%: the stencil rows pass it once as
+// cp.async and once as loads) and FP64 issue (50%) at 16 warps per SM.  Measured
+// and not kept (against 0.730 ms then): no face values stored, the reconstruction run
 // again in sweep 2, 0.917; stencil rows by plain loads a trip ahead, 0.840;
 // rings of 3 or 4 stages, 0.750-0.790; 20 and 24 warps per SM at 96 and 80
 // registers, 0.775 and 1.016 (the rows in flight outgrow L2); two velocities
@@ -915,8 +915,8 @@ constexpr int face_ring_elems() { return FACE_RING * FaceRows<FM>::L * 32; }
 // The per-face coefficients, by the face's warp: `rec` holds the moments and
 // receives the record.  Even lanes compute the side before the face, odd lanes
 // the side after it (the same instructions with one sign flipped).  Not
-// inlined: it runs once per face, and its registers (about 130) would weigh on
-// the sweeps, which run at 96.
+// inlined: it runs once per face, and its registers would weigh on the sweeps (128
+// in the default shape, 96 and 168 in shapes 2 and 4).
 __device__ __noinline__ void face_coefficients(const ugks_fused_block &blk, double dt, const FaceWork fwk,
                                                double *rec) {
   const ugks_block_desc &d = blk.d;
@@ -2036,8 +2036,10 @@ cudaError_t set_step_attributes() {
   return cudaSuccess;
 }
 
-// the largest velocity grid a step accepts, as bytes against 200 KB: per
-// velocity a face's values and slopes (FP64) or a wall face's values (mixed)
+// The largest velocity grid a step accepts, as bytes against 200 KB.  Mixed: a wall
+// face's values, which its CTA holds in shared memory.  FP64: the bound (6400
+// velocities) of a face pass that held a face's values and slopes there; nothing of
+// that size is left in shared memory, and grids above it stay refused as before.
 template <typename T>
 inline size_t face_limit_bytes(int max_nv, int max_axes) {
   if (std::is_same<T, float>::value) return delta_wall_smem(max_nv);
@@ -2143,10 +2145,13 @@ struct NvtxRange {
 // well.  Mixed: by work, faces times velocities.  FP64: up to as many cells as the
 // cell pass holds in one wave of the 3 CTAs an SM has with that split (4 with its
 // own).  Step in us without and with programmatic launches, square cavities (cells
-// a side, velocities): mixed 24, 17^2 (0.4 M) 55.6 and 42.9; 56, 25^2 (4.1 M) 126
-// and 113; 80, 25^2 (8.2 M) 193 and 184; 62, 33^2 (8.6 M) 190 and 182; 88, 33^2
-// (17 M) 339 and 355.  FP64 24, 17^2 45.4 and 41.3; 40, 25^2 91.1 and 83.6; 36,
-// 41^2 203 and 200; 44, 33^2 157 and 183; 63, 33^2 293 and 310.
+// a side, velocities), vanLeer: mixed 24, 17^2 (0.4 M) 52.5 and 42.5; 56, 25^2 (4.1 M)
+// 117 and 104; 80, 25^2 (8.2 M) 193 and 184; 62, 33^2 (8.6 M) 183 and 180; 88, 33^2
+// (17 M) 304 and 315.  FP64 24, 17^2 46.3 and 38.1; 40, 25^2 93 and 86; 36, 41^2 196
+// and 193; 44, 33^2 149 and 173; 63, 33^2 279 and 301.  Tables of small cavities (17^2
+// velocities, two limiters): mixed 8 of 24 (2.9 M) 133 and 131, 16 of 24 (5.8 M) 245
+// and 252, 64 of 12 (6.3 M) 304 and 311; FP64 4 of 12 54 and 47, 4 of 24 91.7 and
+// 92.2, 64 of 12 387 and 399.
 template <typename T>
 inline StepStream step_stream(cudaStream_t st, const ugks_fused_sizes *z) {
   if (std::is_same<T, float>::value) return {st, (double)z->n_faces * z->max_nv <= 1e7 ? 70 : 0};

@@ -5,9 +5,10 @@ more solves (a solve = one pyUGKS simulation, possibly multi-block) and
 advances them with the fused entry points of libugks_b200.so:
 
 * ``ugks_step_fp64`` / ``ugks_step_mixed``: one ``UGKSim.one_step`` of every
-  active solve in four kernel launches (mixed: eight), with dt
-  control, the reference's single flux retry, and the ghost update done on
-  the device (no host synchronisation inside a step);
+  active solve in four kernel launches (mixed: seven; more for several
+  limiters or velocity grids, ``launches_per_step``), with dt control, the
+  reference's single flux retry, and the ghost update done on the device (no
+  host synchronisation inside a step);
 * ``ugks_residual``: the reference residual on demand.
 
 ``precision="fp64"`` stores f and the face fluxes as double (the plain
@@ -316,9 +317,10 @@ class FusedSolver:
     # ---------------------------------------------------------------- stepping
     def launches_per_step(self) -> int:
         """Kernel launches of one ugks_step_* call (ugks_step_launches): one
-        face pass per (limiter, Nv) segment, one retry pass per limiter
-        present, the cell pass and the ghost pass; mixed precision adds the
-        face pass's wall, coefficient and flux launches."""
+        face pass per (limiter, Nv) segment, one retry pass (FP64: per limiter
+        present), the cell pass and the ghost pass; mixed precision adds the
+        face pass's wall, coefficient and flux launches, FP64 one for
+        Cercignani-Lampis walls of more than 1100 velocities."""
         return self.lib.ugks_step_launches(C.byref(self.sizes), 0 if self.precision == "fp64" else 1)
 
     def step(self, n: int = 1):
