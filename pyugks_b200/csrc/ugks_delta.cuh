@@ -250,15 +250,16 @@ __device__ __forceinline__ void wall_item_delta(const ugks_fused_block *__restri
 
 // a wall work item (2 (ni + nj) per block), when that side of the block is a wall
 constexpr int WALL_NT = 128;
+template <int NT>
 __device__ __forceinline__ void wall_work_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                 ugks_solve_state *__restrict__ solves, int w, int retry_pass) {
   const ugks_fused_block &blk = B[find_block<3>(B, nb, w)];
   UGKS_CHECK_ITEM(3, blk, w, solves);
   const int fw = wall_to_face(blk, w);
   switch (blk.d.flux_method) {
-    case 0: wall_item_delta<0, WALL_NT>(B, nb, solves, fw, retry_pass); break;
-    case 1: wall_item_delta<1, WALL_NT>(B, nb, solves, fw, retry_pass); break;
-    case 3: wall_item_delta<3, WALL_NT>(B, nb, solves, fw, retry_pass); break;
+    case 0: wall_item_delta<0, NT>(B, nb, solves, fw, retry_pass); break;
+    case 1: wall_item_delta<1, NT>(B, nb, solves, fw, retry_pass); break;
+    case 3: wall_item_delta<3, NT>(B, nb, solves, fw, retry_pass); break;
     default: break;
   }
 }
@@ -266,10 +267,13 @@ __device__ __forceinline__ void wall_work_delta(const ugks_fused_block *__restri
 __global__ void __launch_bounds__(WALL_NT) wall_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                            ugks_solve_state *__restrict__ solves) {
   pdl_begin();
-  wall_work_delta(B, nb, solves, (int)blockIdx.x, 0);
+  wall_work_delta<WALL_NT>(B, nb, solves, (int)blockIdx.x, 0);
 }
-// and redone after a dt change
-__global__ void __launch_bounds__(WALL_NT) wall_retry_delta(const ugks_fused_block *__restrict__ B, int nb,
+// and redone after a dt change (WIDE_NT threads in tables with Cercignani-Lampis
+// walls of wide grids: a step that redoes 32 such faces of 2401 velocities took 39 ms
+// with WALL_NT threads, 26 so)
+template <int NT>
+__global__ void __launch_bounds__(NT) wall_retry_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                             ugks_solve_state *__restrict__ solves, int ns) {
   pdl_begin();
   int walls = 0;  // items of the solves before
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(WALL_NT) wall_retry_delta(const ugks_fused_blo
         const ugks_fused_block &b = B[x.first_block], &e = B[x.first_block + x.nblocks - 1];
         const int n = e.wall_begin + 2 * (e.d.ni + e.d.nj) - b.wall_begin;
         for (int w = first_item(blockIdx.x, walls, gridDim.x); w < n; w += gridDim.x) {
-          wall_work_delta(B, nb, solves, b.wall_begin + w, 1);
+          wall_work_delta<NT>(B, nb, solves, b.wall_begin + w, 1);
           __syncthreads();  // the next item reuses the shared tables
         }
         walls += n;

@@ -1948,9 +1948,10 @@ cudaError_t set_wall_attributes() {
       if (e != cudaSuccess) return e;
   }
   if constexpr (std::is_same<T, float>::value) {
-    const cudaError_t e = allow_smem(wall_pass_delta);
-    if (e != cudaSuccess) return e;
-    return allow_smem(wall_retry_delta);
+    cudaError_t r[3] = {allow_smem(wall_pass_delta), allow_smem(wall_retry_delta<WALL_NT>),
+                        allow_smem(wall_retry_delta<WIDE_NT>)};
+    for (cudaError_t e : r)
+      if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -2100,7 +2101,10 @@ void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, 
   const unsigned rg = retry_grid(ns);
   if constexpr (std::is_same<T, float>::value) {
     // only the wall faces have anything to redo
-    if (z->n_wall) launch(wall_retry_delta, rg, WALL_NT, delta_wall_smem(z->max_nv), st, B, nb, solves, ns);
+    const int nt = has_cl_walls(z) ? WIDE_NT : WALL_NT;
+    if (z->n_wall)
+      launch(nt == WIDE_NT ? wall_retry_delta<WIDE_NT> : wall_retry_delta<WALL_NT>, rg, nt, delta_wall_smem(z->max_nv), st,
+             B, nb, solves, ns);
   } else {
     if (has_cl_walls(z)) launch_retry_shape<WIDE_NT / 32, 1>(B, nb, z, solves, ns, st);
     else launch_retry_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, z, solves, ns, st);
