@@ -443,7 +443,7 @@ int ugks_step_mixed(const ugks_fused_block *blocks_dev, int nblocks, const ugks_
 
 /* The same step with cudaEventRecord of events[0..7] (cudaEvent_t) on the
    stream around the phases: [0] start, [1] and [2] after the face
-   pass, [3] and [4] after the retry face pass (mixed: its coefficient and flux
+   pass, [3] and [4] after the retry pass of the walls (mixed: coefficient and flux
    launches are part of the face pass, [1]..[4] follow them), [5] and [6] after
    the cell pass, [7] after the ghost pass, which ends the step (dt update).
    mixed != 0 selects FP32 storage.  A null entry records nothing (each

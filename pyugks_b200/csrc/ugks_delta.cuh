@@ -249,7 +249,6 @@ __device__ __forceinline__ void wall_item_delta(const ugks_fused_block *__restri
 }
 
 // a wall work item (2 (ni + nj) per block), when that side of the block is a wall
-constexpr int WALL_NT = 128;
 template <int NT>
 __device__ __forceinline__ void wall_work_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                 ugks_solve_state *__restrict__ solves, int w, int retry_pass) {
@@ -263,8 +262,10 @@ __device__ __forceinline__ void wall_work_delta(const ugks_fused_block *__restri
     default: break;
   }
 }
-// wall faces of the main pass: a CTA per wall work item
-__global__ void __launch_bounds__(WALL_NT) wall_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
+// wall faces of the main pass: a CTA per wall work item, at 128 registers, so that it
+// takes little from the moments sweep beside it (at 142 a step of the 2x2-block cavity
+// 672 us against 655)
+__global__ void __launch_bounds__(WALL_NT, 4) wall_pass_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                            ugks_solve_state *__restrict__ solves) {
   pdl_begin();
   wall_work_delta<WALL_NT>(B, nb, solves, (int)blockIdx.x, 0);
@@ -276,19 +277,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT) wall_retry_delta(const ugks_fused_block *__restrict__ B, int nb,
                                                             ugks_solve_state *__restrict__ solves, int ns) {
   pdl_begin();
-  int walls = 0;  // items of the solves before
-  each_solve(
-      ns, [&](int s) { return retries(solves[s]); },
-      [&](int s) {
-        const ugks_solve_state &x = solves[s];
-        const ugks_fused_block &b = B[x.first_block], &e = B[x.first_block + x.nblocks - 1];
-        const int n = e.wall_begin + 2 * (e.d.ni + e.d.nj) - b.wall_begin;
-        for (int w = first_item(blockIdx.x, walls, gridDim.x); w < n; w += gridDim.x) {
-          wall_work_delta<NT>(B, nb, solves, b.wall_begin + w, 1);
-          __syncthreads();  // the next item reuses the shared tables
-        }
-        walls += n;
-      });
+  redo_walls(B, solves, ns, [&](int w) { wall_work_delta<NT>(B, nb, solves, w, 1); });
 }
 
 // 2. coefficients: the chain of face_coefficients, an interior face on two

@@ -8,8 +8,9 @@
 //               initMacroFlux, calcFaceQ, macroFlux and distFlux fused; wall
 //               faces a CTA each: accommodatingWallDist | adsorbingWall_P1 + P2,
 //               then wallFlux and wallMassEnergyFluxes.
-//   face pass   again, only for solves whose dt changed (updateTimeStep inside
-//               the dt loop, ugks_sim.py:430-441).
+//   wall faces  again, only for solves whose dt changed (updateTimeStep inside
+//               the dt loop, ugks_sim.py:430-441); an interior face takes the dt of
+//               the last pass at once.
 //   cell pass   a cell per warp: calcQ, updateMacro and UGKS_update fused, plus
 //               the cell's CFL frequency (clFindDT).
 //   ghost pass  one CTA per ghost cell of every block face (updateBC), and the
@@ -1199,7 +1200,7 @@ __device__ __forceinline__ int wall_to_face(const ugks_fused_block &blk, int w) 
 // of WIDE_NT threads, beside which the faces run.  Step in ms with these walls in
 // the face pass's CTAs of 128 threads and so: 32 wall faces of 1681 velocities 11.2
 // and 3.8, 256 of 1369 8.7 and 5.4, 256 of 2401 25.0 and 14.3.
-constexpr int WIDE_NV = 1100, WIDE_NT = 512;
+constexpr int WALL_NT = 128, WIDE_NV = 1100, WIDE_NT = 512;
 __host__ __device__ inline bool wide_cl_wall(const ugks_fused_block &blk, int wall) {
   return blk.d.Nv > WIDE_NV && blk.bc_type[wall] == BC_ADSORBING && blk.d.reflect[wall] == UGKS_REFLECT_CL;
 }
@@ -1256,65 +1257,53 @@ __global__ void __launch_bounds__(WPC * 32, MINB) face_pass_fp64(const ugks_fuse
     wall_work_fp64<WPC * 32>(B, nb, solves, (int)blockIdx.x, 0, kind);
   } else if (item < count && face_work<FM, true>(B, nb, solves, first + item, 0, fwk) && fwk.wall < 0) {
     const ugks_fused_block &blk = B[fwk.bi];
-    face_item_fp64<FM>(blk, solves[blk.solve].dt, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp), fwk);
+    // the dt of the step's final flux pass: the reference's first pass, when it is
+    // redone, leaves nothing of an interior face
+    face_item_fp64<FM>(blk, step_dt(solves[blk.solve]).flux, dyn + warp * wstride, face_ring<FM, WPC>(dyn, wstride, warp),
+                       fwk);
   }
 }
 
-// The flux pass redone after a dt change (ugks_sim.py:432-441), for few solves in
-// few steps.  Every CTA finds the solves that retry, and the whole launch works on
-// each of them: their walls count through as one list, dealt to the CTAs in turn,
-// their faces as another, to the warps.  With CTAs of its own for every solve, one
-// that retries among 16 (48x48 cells, 625 velocities, FP64) had 37 of 592, and its
-// pass took 0.69 ms against 0.08 (a step 2.16 and 1.54 ms); one among 64 of 24x24
-// cells and 289 velocities, a step 1.57 and 1.17 ms.
+// The walls' flux pass redone after a dt change (ugks_sim.py:432-441), for few solves
+// in few steps.  An interior face has nothing to redo, a wall has: its coverage moves
+// in both passes.  Every CTA finds the solves that retry, and their walls count through
+// as one list, dealt to the CTAs in turn.  Against a pass over all faces of these
+// solves, a step whose dt grows by its limit: 64x64 cells of 625 velocities 497 -> 206
+// us, 32x16 of 2401 435 -> 261, 16 solves of 48x48 and 625 2453 -> 1523.
 inline unsigned retry_grid(int ns) { return (unsigned)std::min(592l, 148l * ns); }
-template <typename Need, typename Work>
-__device__ __forceinline__ void each_solve(int ns, Need need, Work work) {
-  if (ns == 1) {  // the usual table, out in 3 us less of a 32x32-cell step than by lanes
-    if (need(0)) work(0);
+__device__ __forceinline__ bool retries(const ugks_solve_state &x) { return x.active && x.nblocks > 0 && step_dt(x).retry; }
+template <typename Work>
+__device__ __forceinline__ void redo_walls(const ugks_fused_block *__restrict__ B,
+                                           const ugks_solve_state *__restrict__ solves, int ns, Work work) {
+  int before = 0;  // walls of the solves before
+  auto solve = [&](int s) {
+    const ugks_solve_state &x = solves[s];
+    const ugks_fused_block &b = B[x.first_block], &e = B[x.first_block + x.nblocks - 1];
+    const int n = e.wall_begin + 2 * (e.d.ni + e.d.nj) - b.wall_begin, ctas = gridDim.x;
+    for (int w = ((int)blockIdx.x + ctas - before % ctas) % ctas; w < n; w += ctas) {
+      work(b.wall_begin + w);
+      __syncthreads();  // the next item reuses the shared tables
+    }
+    before += n;
+  };
+  if (ns == 1) {  // the usual table
+    if (retries(solves[0])) solve(0);
     return;
   }
   // a lane per solve, by every warp for itself: all of a CTA with the same result
   const int lane = threadIdx.x & 31;
   bool any = false;
-  for (int s = lane; s < ns; s += 32) any |= need(s);
+  for (int s = lane; s < ns; s += 32) any |= retries(solves[s]);
   if (!__any_sync(0xffffffffu, any)) return;
   for (int s0 = 0; s0 < ns; s0 += 32)
-    for (unsigned m = __ballot_sync(0xffffffffu, s0 + lane < ns && need(s0 + lane)); m; m &= m - 1) work(s0 + __ffs(m) - 1);
+    for (unsigned m = __ballot_sync(0xffffffffu, s0 + lane < ns && retries(solves[s0 + lane])); m; m &= m - 1)
+      solve(s0 + __ffs(m) - 1);
 }
-__device__ __forceinline__ bool retries(const ugks_solve_state &x) { return x.active && x.nblocks > 0 && step_dt(x).retry; }
-// item of `size` workers' worker k in a list that begins after `before` items
-__device__ __forceinline__ int first_item(int k, int before, int size) { return (k + size - before % size) % size; }
-
-template <int FM, int WPC, int MINB>
-__global__ void __launch_bounds__(WPC * 32, MINB) face_retry_fp64(const ugks_fused_block *__restrict__ B, int nb,
-                                                                  ugks_solve_state *__restrict__ solves, int ns,
-                                                                  int wstride) {
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) wall_retry_fp64(const ugks_fused_block *__restrict__ B, int nb,
+                                                                ugks_solve_state *__restrict__ solves, int ns) {
   pdl_begin();
-  extern __shared__ double dyn[];
-  const int warp = threadIdx.x >> 5, ctas = gridDim.x, warps = ctas * WPC;
-  int walls = 0, faces = 0;  // items of the solves before
-  each_solve(
-      ns, [&](int s) { return retries(solves[s]) && B[solves[s].first_block].d.flux_method == FM; },
-      [&](int s) {
-        const ugks_solve_state &x = solves[s];
-        const ugks_fused_block &b = B[x.first_block], &e = B[x.first_block + x.nblocks - 1];
-        const int nw = e.wall_begin + 2 * (e.d.ni + e.d.nj) - b.wall_begin;
-        for (int w = first_item(blockIdx.x, walls, ctas); w < nw; w += ctas) {
-          wall_work_fp64<WPC * 32>(B, nb, solves, b.wall_begin + w, 1, WALL_ANY);
-          __syncthreads();  // the next item reuses the shared tables
-        }
-        walls += nw;
-        const int nf = e.face_begin + 2 * (e.d.ni + 1) * (e.d.nj + 1) - b.face_begin;
-        for (int w = first_item((int)blockIdx.x * WPC + warp, faces, warps); w < nf; w += warps) {
-          FaceWork fwk;
-          if (!face_work<FM>(B, nb, solves, b.face_begin + w, 1, fwk) || fwk.wall >= 0) continue;
-          const ugks_fused_block &blk = B[fwk.bi];
-          face_item_fp64<FM>(blk, step_dt(solves[blk.solve]).flux, dyn + warp * wstride,
-                             face_ring<FM, WPC>(dyn, wstride, warp), fwk);
-        }
-        faces += nf;
-      });
+  redo_walls(B, solves, ns, [&](int w) { wall_work_fp64<NT>(B, nb, solves, w, 1, WALL_ANY); });
 }
 // ---------------------------------------------------------------------------
 // cell pass: calcQ (clKernel.c:480-543) + updateMacro (clUGKS.c:1158-1187) +
@@ -1931,19 +1920,10 @@ cudaError_t set_face_shape() {
     if (e != cudaSuccess) return e;
   return cudaSuccess;
 }
-template <int W, int M>
-cudaError_t set_retry_shape() {
-  cudaError_t r[3] = {allow_smem(face_retry_fp64<0, W, M>), allow_smem(face_retry_fp64<1, W, M>),
-                      allow_smem(face_retry_fp64<3, W, M>)};
-  for (cudaError_t e : r)
-    if (e != cudaSuccess) return e;
-  return cudaSuccess;
-}
 template <typename T>
 cudaError_t set_wall_attributes() {
   if constexpr (std::is_same<T, double>::value) {
-    cudaError_t r[6] = {set_face_shape<1>(), set_face_shape<2>(), set_face_shape<3>(), set_face_shape<4>(),
-                        set_retry_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(), set_retry_shape<WIDE_NT / 32, 1>()};
+    cudaError_t r[4] = {set_face_shape<1>(), set_face_shape<2>(), set_face_shape<3>(), set_face_shape<4>()};
     for (cudaError_t e : r)
       if (e != cudaSuccess) return e;
   }
@@ -2085,30 +2065,17 @@ inline void launch_faces(int v, const ugks_fused_block *B, int nb, ugks_solve_st
   }
 }
 
-template <int WPC, int MINB>
-void launch_retry_shape(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves, int ns,
-                        StepStream st) {
-  const unsigned g = std::min(retry_grid(ns), 148u * MINB), t = WPC * 32;
-  const int ws = face_stride(z->max_axes);
-  if (z->face_count[0]) launch(face_retry_fp64<0, WPC, MINB>, g, t, face_smem<0, WPC>(ws), st, B, nb, solves, ns, ws);
-  if (z->face_count[1]) launch(face_retry_fp64<1, WPC, MINB>, g, t, face_smem<1, WPC>(ws), st, B, nb, solves, ns, ws);
-  if (z->face_count[3]) launch(face_retry_fp64<3, WPC, MINB>, g, t, face_smem<3, WPC>(ws), st, B, nb, solves, ns, ws);
-}
-// the retry pass of every flux method (rare)
+// the walls redone after a dt change (rare)
 template <typename T>
 void launch_retry(const ugks_fused_block *B, int nb, const ugks_fused_sizes *z, ugks_solve_state *solves, int ns,
                   StepStream st) {
-  const unsigned rg = retry_grid(ns);
-  if constexpr (std::is_same<T, float>::value) {
-    // only the wall faces have anything to redo
-    const int nt = has_cl_walls(z) ? WIDE_NT : WALL_NT;
-    if (z->n_wall)
-      launch(nt == WIDE_NT ? wall_retry_delta<WIDE_NT> : wall_retry_delta<WALL_NT>, rg, nt, delta_wall_smem(z->max_nv), st,
-             B, nb, solves, ns);
-  } else {
-    if (has_cl_walls(z)) launch_retry_shape<WIDE_NT / 32, 1>(B, nb, z, solves, ns, st);
-    else launch_retry_shape<FaceShape<1>::wpc, FaceShape<1>::minb>(B, nb, z, solves, ns, st);
-  }
+  if (!z->n_wall) return;
+  const bool wide = has_cl_walls(z);
+  const unsigned g = retry_grid(ns), nt = wide ? WIDE_NT : WALL_NT;
+  if constexpr (std::is_same<T, float>::value)
+    launch(wide ? wall_retry_delta<WIDE_NT> : wall_retry_delta<WALL_NT>, g, nt, delta_wall_smem(z->max_nv), st, B, nb, solves, ns);
+  else
+    launch(wide ? wall_retry_fp64<WIDE_NT> : wall_retry_fp64<WALL_NT>, g, nt, 0, st, B, nb, solves, ns);
 }
 
 // the mixed moments sweep of one segment, in launch shape v (ugks_fused_sizes.seg_variant)
@@ -2395,8 +2362,7 @@ int ugks_step_launches(const ugks_fused_sizes *z, int mixed) {
   if (mixed && z->n_wall) n += 1;   // and its wall launch
   for (int k = 0; k < z->n_segments && k < UGKS_MAX_FACE_SEGMENTS; ++k)
     n += z->seg_count[k] > 0 && !(mixed && z->seg_method[k] == UGKS_SEG_CL_WALLS) ? 1 : 0;
-  if (mixed) n += z->n_wall ? 1 : 0;  // retry pass (mixed: walls)
-  else for (int m = 0; m < 4; ++m) n += z->face_count[m] > 0 ? 1 : 0;
+  n += z->n_wall ? 1 : 0;  // retry pass
   n += z->n_cells ? 1 : 0;
   n += 1;                                                          // ghost pass (or the dt update alone)
   return n;

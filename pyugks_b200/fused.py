@@ -317,9 +317,9 @@ class FusedSolver:
     # ---------------------------------------------------------------- stepping
     def launches_per_step(self) -> int:
         """Kernel launches of one ugks_step_* call (ugks_step_launches): one
-        face pass per (limiter, Nv) segment, one retry pass (FP64: per limiter
-        present), the cell pass and the ghost pass; mixed precision adds the
-        face pass's wall, coefficient and flux launches, FP64 one for
+        face pass per (limiter, Nv) segment, the walls' retry pass, the cell pass
+        and the ghost pass; mixed precision adds the face pass's wall,
+        coefficient and flux launches, FP64 one for
         Cercignani-Lampis walls of more than 1100 velocities."""
         return self.lib.ugks_step_launches(C.byref(self.sizes), 0 if self.precision == "fp64" else 1)
 

@@ -55,9 +55,9 @@ def test_walls(cuda, reflect, m, redo, precision):
     check(gpu, 0, ora, TOL[precision])
 
 
-@pytest.mark.parametrize("precision,launches", [("fp64", 8), ("mixed", 9)])
+@pytest.mark.parametrize("precision,launches", [("fp64", 7), ("mixed", 9)])
 def test_table_of_both(cuda, precision, launches):
-    """Three segments; FP64: two retry launches and the walls'."""
+    """Three segments; FP64: the walls' launch with them."""
     cases = [channel("CL", 16), channel("S", 36), channel("CL", 36, "WENO5")]
     gpu = FusedSolver(cases, precision=precision)
     assert gpu.launches_per_step() == launches
